@@ -14,7 +14,8 @@ namespace {
 
 constexpr int BM = 128, BK = 32;             // tile rows, K per stage (64 B of bf16)
 constexpr int TILE = BM * BK * 2;            // bytes of one 128 x 32 bf16 slice tile of A
-constexpr int kThreads = 128;
+constexpr int kEpiThreads = 256;             // 8 epilogue warps
+constexpr int kThreads = kEpiThreads + 64;   // and the TMA and the MMA warp
 constexpr unsigned long long kWaitNs = 2000000000ull;  // bound of every wait (2 s)
 
 // Slice pairs (t, u) with t + u <= NS - 1 in order of t + u; pairs of order
@@ -40,11 +41,12 @@ struct Pairs {
 
 struct Args {
   int64_t M, N, rpad_a, rpad_b, ldc, ldfix;
-  int32_t tiles_m, tiles_n, lower, kblocks, chunk_kb, direct, U, alpha_exp, alpha_neg;
+  int32_t tiles_n, lower, kblocks, chunk_kb, block_kb, U;
+  double alpha, beta;
   const int32_t* exa;
   const int32_t* exb;
   double* C;
-  unsigned long long* fix;
+  unsigned long long* fix;  // K split over blocks: fixed-point sums (else null, C is written)
   int* err;
 };
 
@@ -118,29 +120,72 @@ __device__ __forceinline__ void mma_bf16(uint32_t tmem_d, unsigned long long ade
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
-        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]),
-        "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]),
-        "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Eight columns of the calling warp's 32 tensor-memory lanes; the caller
+// waits (tcgen05.wait::ld) before it uses them.
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&v)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(taddr));
 }
 
-// v * 2^E for a fixed-point integer v, rounded once (int64 -> double).
+// v * 2^E for a fixed-point integer v, rounded once (to nearest even).  Built
+// with integer instructions: GB300's 64-bit conversions and float64 adds share
+// the narrow FP64 pipe (1.6 lanes per clock and SM).
 __device__ __forceinline__ double fix_to_double(long long v, int E) {
   if (v == 0) return 0.0;
-  const double d = __ll2double_rn(v);
-  const long long b = __double_as_longlong(d);
-  const int ex = (int)((b >> 52) & 0x7FF) + E;
-  if (ex > 0 && ex < 2047) return __longlong_as_double(b + ((long long)E << 52));
-  return scalbn(d, E);
+  const unsigned long long u = v < 0 ? 0ull - (unsigned long long)v : (unsigned long long)v;
+  const int lz = __clzll((long long)u);
+  const int ex = 1086 - lz + E;
+  if (ex > 0 && ex < 2046) {
+    const unsigned long long norm = u << lz;
+    unsigned long long mant = norm >> 11;
+    const unsigned rem = (unsigned)norm & 0x7FFu;
+    mant += (rem > 0x400u || (rem == 0x400u && (mant & 1ull))) ? 1ull : 0ull;
+    // the implicit bit (and a carry out of the rounding) adds to the exponent
+    const unsigned long long bits = ((unsigned long long)(ex - 1) << 52) + mant;
+    return __longlong_as_double((long long)(bits | ((unsigned long long)v & 0x8000000000000000ull)));
+  }
+  return scalbn(__ll2double_rn(v), E);
+}
+
+// v * 2^U rounded to nearest even for |v * 2^U| < 2^62, with integer
+// instructions (as fix_to_double).
+__device__ __forceinline__ long long float_to_fixed(float v, int U) {
+  const int b = __float_as_int(v);
+  const int field = (b >> 23) & 0xFF;
+  if (field == 0) return 0;  // the accumulators hold no subnormal values above 2^-U / 2
+  const unsigned mant = ((unsigned)b & 0x7FFFFFu) | 0x800000u;
+  const int sh = field - 150 + U;
+  long long r;
+  if (sh >= 0) {
+    r = (long long)((unsigned long long)mant << min(sh, 39));
+  } else if (sh < -25) {
+    r = 0;
+  } else {
+    const unsigned q = mant >> -sh, rem = mant & ((1u << -sh) - 1u), half = 1u << (-sh - 1);
+    r = (long long)(q + ((rem > half || (rem == half && (q & 1u))) ? 1u : 0u));
+  }
+  return b < 0 ? -r : r;
 }
 
 // ---------------------------------------------------------------- the product
+// One BM x BN output tile per thread block and a range of its K chunks
+// (blockIdx.y).  Warp 8 issues the TMA loads, one thread of warp 9 the MMAs;
+// warps 0-7 drain the accumulators of every finished chunk into 64-bit
+// fixed-point sums kept in registers (row = tensor-memory lane, half of the
+// columns per warp) while the TMA loads of the next chunk are in flight, and
+// write C (or, when K is split over blocks, add to the fixed-point workspace)
+// once at the end.
+//
+// What bounds it: for long K the slice tiles' traffic from L2 and the drain
+// between chunks; for the K = 32 updates of the Cholesky factorization the
+// latency of one load, one MMA group and the write-back.  A block per chunk,
+// with 64-bit conversions, an integer atomic per entry and chunk and one load
+// of C at a time, took 2.9 ms for the whole 1999 x 1999 x 5051 lower product
+// (msdp_tc_gemm) against 1.05 ms with this and the slicing below.
 template <int NS, int NG, int BN, int NST>
 __global__ void __launch_bounds__(kThreads, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb, const Args a) {
@@ -148,18 +193,21 @@ __global__ void __launch_bounds__(kThreads, 1)
   constexpr int TILE_B = BN * BK * 2;
   constexpr int STAGE = NS * (TILE + TILE_B);
   constexpr uint32_t TCOLS = NG * BN <= 128 ? 128u : (NG * BN <= 256 ? 256u : 512u);
+  constexpr int HALF = BN / 2;  // columns per epilogue warp
   static_assert(NG * BN <= 512, "tensor memory holds 512 columns");
+  static_assert(HALF % 8 == 0 && TILE_B % 512 == 0, "column segments of 8, swizzle atoms of 512 bytes");
 
   extern __shared__ unsigned char smem_raw[];
+  __shared__ int exb_s[BN];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t sb = (raw + 1023u) & ~1023u;       // 1 KiB aligned stage buffers
   unsigned char* gb = smem_raw + (sb - raw);
-  const uint32_t bar0 = sb + NST * STAGE;           // full[NST], empty[NST], done
-  uint32_t* tslot = (uint32_t*)(gb + NST * STAGE + 8 * (2 * NST + 1));
+  const uint32_t bar0 = sb + NST * STAGE;           // full[NST], empty[NST], done, drained
+  uint32_t* tslot = (uint32_t*)(gb + NST * STAGE + 8 * (2 * NST + 2));
   volatile int* abort_flag = (volatile int*)(tslot + 1);
   auto full = [&](int s) { return bar0 + 8u * s; };
   auto empty = [&](int s) { return bar0 + 8u * (NST + s); };
-  const uint32_t done = bar0 + 8u * (2 * NST);
+  const uint32_t done = bar0 + 8u * (2 * NST), drained = done + 8u;
   auto tileA = [&](int s, int t) { return sb + (uint32_t)(s * STAGE + t * TILE); };
   auto tileB = [&](int s, int u) { return sb + (uint32_t)(s * STAGE + NS * TILE + u * TILE_B); };
 
@@ -167,24 +215,30 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int tm = (int)(blockIdx.x / a.tiles_n), tn = (int)(blockIdx.x % a.tiles_n);
   // lower triangle only: tiles entirely above the diagonal have nothing to do
   if (a.lower && (int64_t)tn * BN > (int64_t)tm * BM + BM - 1) return;
-  const int kb0 = blockIdx.y * a.chunk_kb;
-  const int nkb = min(a.chunk_kb, a.kblocks - kb0);
+  const int kb0 = (int)blockIdx.y * a.block_kb;
+  const int nkb = min(a.block_kb, a.kblocks - kb0);
+  const int nch = (nkb + a.chunk_kb - 1) / a.chunk_kb;
 
-  if (threadIdx.x == 0) {
+  if (threadIdx.x == kEpiThreads) {
     for (int s = 0; s < NST; ++s) {
       mbar_init(full(s), 1);
       mbar_init(empty(s), 1);
     }
     mbar_init(done, 1);
+    mbar_init(drained, kEpiThreads / 32);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 2) {
+  if (warp == kEpiThreads / 32 + 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tslot)),
                  "r"(TCOLS)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  if (threadIdx.x < BN) {
+    const int64_t col = (int64_t)tn * BN + threadIdx.x;
+    exb_s[threadIdx.x] = col < a.N ? a.exb[col] : 0;
   }
   tc_fence_before();
   __syncthreads();
@@ -192,100 +246,156 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t tbase = *tslot;
   const unsigned long long deadline = gtime() + kWaitNs;
 
-  if (warp == 0 && lane == 0) {
-    // TMA producer: every slice of A and B for one 32-wide K block per stage
-    int issued = 0;
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % NST;
-      if (i >= NST && !mbar_wait(empty(s), ((i / NST) & 1) ^ 1, deadline)) {
-        *abort_flag = 1;
-        atomicExch(a.err, 1);
-        break;
+  if (warp == kEpiThreads / 32) {
+    if (lane == 0) {
+      // TMA producer: every slice of A and B for one 32-wide K block per stage
+      int issued = 0;
+      for (int i = 0; i < nkb; ++i) {
+        const int s = i % NST;
+        if (i >= NST && !mbar_wait(empty(s), ((i / NST) & 1) ^ 1, deadline)) {
+          *abort_flag = 1;
+          atomicExch(a.err, 1);
+          break;
+        }
+        if (*abort_flag) break;
+        mbar_expect_tx(full(s), STAGE);
+        const int x = (kb0 + i) * BK;
+#pragma unroll
+        for (int t = 0; t < NS; ++t) {
+          tma_load_2d(&ma, tileA(s, t), x, (int)(t * a.rpad_a + (int64_t)tm * BM), full(s));
+          tma_load_2d(&mb, tileB(s, t), x, (int)(t * a.rpad_b + (int64_t)tn * BN), full(s));
+        }
+        issued = i + 1;
       }
-      if (*abort_flag) break;
-      mbar_expect_tx(full(s), STAGE);
-      const int x = (kb0 + i) * BK;
-#pragma unroll
-      for (int t = 0; t < NS; ++t) tma_load_2d(&ma, tileA(s, t), x, (int)(t * a.rpad_a + (int64_t)tm * BM), full(s));
-#pragma unroll
-      for (int u = 0; u < NS; ++u) tma_load_2d(&mb, tileB(s, u), x, (int)(u * a.rpad_b + (int64_t)tn * BN), full(s));
-      issued = i + 1;
+      if (*abort_flag) {
+        // let the copies already issued land before the block exits
+        const unsigned long long d2 = gtime() + kWaitNs / 4;
+        for (int i = max(0, issued - NST); i < issued; ++i) mbar_wait(full(i % NST), (i / NST) & 1, d2);
+      }
     }
-    if (*abort_flag) {
-      // let the copies already issued land before the block exits
-      const unsigned long long d2 = gtime() + kWaitNs / 4;
-      for (int i = max(0, issued - NST); i < issued; ++i) mbar_wait(full(i % NST), (i / NST) & 1, d2);
+    __syncwarp();
+  } else if (warp == kEpiThreads / 32 + 1) {
+    if (lane == 0) {
+      // MMA issuer: all slice pairs of the stage into their group accumulators
+      bool ok = true;
+      int i = 0;
+      for (int c = 0; c < nch && ok; ++c) {
+        // the accumulators of the chunk before have been read
+        if (c > 0 && (!mbar_wait(drained, (c - 1) & 1, deadline) || *abort_flag)) {
+          *abort_flag = 1;
+          atomicExch(a.err, 4);
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        const int i1 = min(nkb, (c + 1) * a.chunk_kb);
+        for (bool first = true; i < i1; ++i, first = false) {
+          const int s = i % NST;
+          if (!mbar_wait(full(s), (i / NST) & 1, deadline) || *abort_flag) {
+            *abort_flag = 1;
+            atomicExch(a.err, 2);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+#pragma unroll
+          for (int p = 0; p < Pairs<NS, NG>::N; ++p) {
+#pragma unroll
+            for (int kk = 0; kk < BK / 16; ++kk) {
+              const unsigned long long ad = smem_desc(tileA(s, P.t[p]) + kk * 32);
+              const unsigned long long bd = smem_desc(tileB(s, P.u[p]) + kk * 32);
+              mma_bf16<BN>(tbase + (uint32_t)(P.g[p] * BN), ad, bd, (!first || !P.first[p] || kk > 0) ? 1u : 0u);
+            }
+          }
+          mma_commit(empty(s));
+        }
+        if (ok) mma_commit(done);
+      }
     }
-  } else if (warp == 1 && lane == 0) {
-    // MMA issuer: all slice pairs of the stage into their group accumulators
+    __syncwarp();
+  } else {
+    // epilogue: thread = one row of the tile (tensor-memory lane), columns
+    // [c0, c0 + HALF)
+    const int c0 = (warp >> 2) * HALF;
+    const int64_t row = (int64_t)tm * BM + (warp & 3) * 32 + lane;
+    const bool row_ok = row < a.M;
+    const uint32_t tw = tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
+    long long acc[HALF];
+#pragma unroll
+    for (int j = 0; j < HALF; ++j) acc[j] = 0;
     bool ok = true;
-    for (int i = 0; i < nkb; ++i) {
-      const int s = i % NST;
-      if (!mbar_wait(full(s), (i / NST) & 1, deadline) || *abort_flag) {
+    for (int c = 0; c < nch; ++c) {
+      ok = mbar_wait(done, c & 1, deadline) && !*abort_flag;
+      ok = __all_sync(0xffffffffu, ok);
+      if (!ok) {
         *abort_flag = 1;
-        atomicExch(a.err, 2);
-        ok = false;
+        if (lane == 0) atomicExch(a.err, 3);
         break;
       }
       tc_fence_after();
 #pragma unroll
-      for (int p = 0; p < Pairs<NS, NG>::N; ++p) {
+      for (int sg = 0; sg < HALF / 8; ++sg) {
+        uint32_t v[NG][8];
 #pragma unroll
-        for (int kk = 0; kk < BK / 16; ++kk) {
-          const unsigned long long ad = smem_desc(tileA(s, P.t[p]) + kk * 32);
-          const unsigned long long bd = smem_desc(tileB(s, P.u[p]) + kk * 32);
-          mma_bf16<BN>(tbase + (uint32_t)(P.g[p] * BN), ad, bd, (i > 0 || !P.first[p] || kk > 0) ? 1u : 0u);
+        for (int g = 0; g < NG; ++g) tmem_ld8(tw + (uint32_t)(g * BN + sg * 8), v[g]);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int g = 0; g < NG; ++g) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (g < NG - 1) {
+              // an integer below 2^24 times 2^-8g (U >= 24 covers g <= 3)
+              const int q = __float2int_rn(__uint_as_float(v[g][j]) * (float)(1 << (8 * g)));
+              acc[sg * 8 + j] += (long long)q << (a.U - 8 * g);
+            } else {
+              acc[sg * 8 + j] += float_to_fixed(__uint_as_float(v[g][j]), a.U);
+            }
+          }
         }
       }
-      mma_commit(empty(s));
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0 && c + 1 < nch) mbar_arrive(drained);
     }
-    if (ok) mma_commit(done);
-  }
-  __syncwarp();
-
-  // epilogue: thread = one row of the tile (tensor-memory lane)
-  const bool ok = mbar_wait(done, 0, deadline) && !*abort_flag;
-  if (!ok && threadIdx.x == 0) atomicExch(a.err, 3);
-  __syncwarp();
-  tc_fence_after();
-  if (ok) {
-    const int64_t row = (int64_t)tm * BM + warp * 32 + lane;
-    const bool row_ok = row < a.M;
-    const int ea = row_ok ? a.exa[row] : 0;
-    const float scaleU = __int_as_float((127 + a.U) << 23);
-    const uint32_t tw = tbase + ((uint32_t)(warp * 32) << 16);
-#pragma unroll 1
-    for (int cc = 0; cc < BN / 32; ++cc) {
-      long long acc[32];
+    if (ok && row_ok) {
+      const int ea = a.exa[row] - a.U - 14;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) acc[j] = 0;
+      for (int sg = 0; sg < HALF / 8; ++sg) {
+        const int64_t col0 = (int64_t)tn * BN + c0 + sg * 8;
+        if (a.fix) {
 #pragma unroll
-      for (int g = 0; g < NG; ++g) {
-        uint32_t v[32];
-        tmem_ld32(tw + (uint32_t)(g * BN + cc * 32), v);
-#pragma unroll
-        for (int j = 0; j < 32; ++j) acc[j] += __float2ll_rn(__uint_as_float(v[j]) * scaleU);
-      }
-      if (row_ok) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-          const int64_t col = (int64_t)tn * BN + cc * 32 + j;
-          if (col >= a.N || (a.lower && row < col)) continue;
-          if (a.direct) {
-            double d = fix_to_double(acc[j], ea + a.exb[col] - a.U - 14 + a.alpha_exp);
-            d = a.alpha_neg ? -d : d;
-            double* o = a.C + row + col * a.ldc;
-            *o = a.direct == 2 ? *o + d : d;
-          } else {
-            atomicAdd(a.fix + row + col * a.ldfix, (unsigned long long)acc[j]);
+          for (int j = 0; j < 8; ++j) {
+            const int64_t col = col0 + j;
+            if (col < a.N && !(a.lower && row < col))
+              atomicAdd(a.fix + row + col * a.ldfix, (unsigned long long)acc[sg * 8 + j]);
           }
+          continue;
+        }
+        // eight independent loads of C before the first store
+        double old[8];
+        if (a.beta != 0.0) {
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const int64_t col = col0 + j;
+            old[j] = (col < a.N && !(a.lower && row < col)) ? a.C[row + col * a.ldc] : 0.0;
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int64_t col = col0 + j;
+          double d = fix_to_double(acc[sg * 8 + j], ea + exb_s[c0 + sg * 8 + j]);
+          if (a.alpha == -1.0) d = -d;
+          else if (a.alpha != 1.0) d = a.alpha * d;
+          if (a.beta == 1.0) d = old[j] + d;
+          else if (a.beta != 0.0) d = d + a.beta * old[j];
+          if (col < a.N && !(a.lower && row < col)) a.C[row + col * a.ldc] = d;
         }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 2) {
+  if (warp == kEpiThreads / 32 + 1) {
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TCOLS) : "memory");
   }
@@ -307,15 +417,20 @@ __global__ void k_finish(int64_t M, int64_t N, const long long* __restrict__ fix
 }
 
 // ---------------------------------------------------------------- slicing
-__device__ __forceinline__ double src_load(const Source& s, int64_t R, int64_t k) {
+// Start of row R of a source; element k is at p[k * ks] or, with kmap, at
+// p[a * rs + b * ks] for k -> (a, b).
+__device__ __forceinline__ const double* src_row(const Source& s, int64_t R) {
   const uint32_t j = (uint32_t)R / (uint32_t)s.nr;
   const int64_t i = R - (int64_t)j * s.nr;
+  return s.p + (int64_t)j * s.bs + (s.kmap ? 0 : i * s.rs);
+}
+__device__ __forceinline__ double src_at(const Source& s, const double* row, int64_t k) {
   if (s.kmap) {
     const int2 ab = s.kmap[k];
-    const double v = s.p[(int64_t)j * s.bs + ab.x * s.rs + ab.y * s.ks];
+    const double v = row[ab.x * s.rs + ab.y * s.ks];
     return ab.x == ab.y ? v : v * 1.4142135623730951;
   }
-  return s.p[(int64_t)j * s.bs + i * s.rs + k * s.ks];
+  return row[k * s.ks];
 }
 // Row exponents, one warp per row (rows read along k).
 __global__ void k_rowexp_warp(Source s, int64_t Rpad, int32_t* __restrict__ ex) {
@@ -323,43 +438,76 @@ __global__ void k_rowexp_warp(Source s, int64_t Rpad, int32_t* __restrict__ ex) 
   const int lane = threadIdx.x & 31;
   if (R >= Rpad) return;
   int m = 0;
-  if (R < s.rows)
-    for (int64_t k = lane; k < s.K; k += 32) m = max(m, exp_field(src_load(s, R, k)));
+  if (R < s.rows) {
+    const double* row = src_row(s, R);
+#pragma unroll 4
+    for (int64_t k = lane; k < s.K; k += 32) m = max(m, exp_field(src_at(s, row, k)));
+  }
 #pragma unroll
   for (int o = 16; o; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
   if (lane == 0) ex[R] = row_exp(m);
 }
-// Row exponents, one thread per row (rows contiguous in memory).
-__global__ void k_rowexp_thread(Source s, int64_t Rpad, int32_t* __restrict__ ex) {
-  const int64_t R = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (R >= Rpad) return;
+// Row exponents of rows contiguous in memory: 32 rows per block, one per
+// lane (256-byte loads), the 32 warps take every 32nd k.  One thread per row
+// left 2000 rows to 8 SMs: 560 us for 1999 x 5051, against 30 us of copy time.
+__global__ void __launch_bounds__(1024) k_rowexp_lanes(Source s, int64_t Rpad, int32_t* __restrict__ ex) {
+  __shared__ int part[32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int64_t R = (int64_t)blockIdx.x * 32 + lane;
   int m = 0;
-  if (R < s.rows)
-    for (int64_t k = 0; k < s.K; ++k) m = max(m, exp_field(src_load(s, R, k)));
-  ex[R] = row_exp(m);
+  if (R < s.rows) {
+    const double* row = src_row(s, R);
+#pragma unroll 8
+    for (int64_t k = w; k < s.K; k += 32) m = max(m, exp_field(row[k * s.ks]));
+  }
+  part[w][lane] = m;
+  __syncthreads();
+  if (w == 0 && R < Rpad) {
+#pragma unroll
+    for (int q = 1; q < 32; ++q) m = max(m, part[q][lane]);
+    ex[R] = row_exp(m);
+  }
 }
 
-// 32 x 32 tiles: read (through shared memory when rows are the contiguous
-// direction), cut into NS slices, write K-major bf16 (zeros in the padding).
+// Tiles of 32 rows x 64 k: read (through shared memory when rows are the
+// contiguous direction), cut into NS slices, write K-major bf16 pairs (zeros
+// in the padding).  Kpad is a multiple of 32: the second half of the last
+// tile may lie outside.
 template <int NS>
 __global__ void __launch_bounds__(256) k_slice(Source s, int64_t Rpad, int64_t Kpad, const int32_t* __restrict__ ex,
                                               __nv_bfloat16* __restrict__ out) {
-  __shared__ double tile[32][33];
-  const int64_t r0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 32;
+  __shared__ double tile[32][66];
+  const int64_t r0 = (int64_t)blockIdx.x * 32, k0 = (int64_t)blockIdx.y * 64;
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const bool along_k = s.kmap != nullptr || s.ks == 1 || s.rs != 1;
+  if (along_k) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int rr = along_k ? ty + 8 * i : tx, kk = along_k ? tx : ty + 8 * i;
-    const int64_t R = r0 + rr, k = k0 + kk;
-    tile[rr][kk] = (R < s.rows && k < s.K) ? src_load(s, R, k) : 0.0;
+    for (int i = 0; i < 4; ++i) {
+      const int64_t R = r0 + ty + 8 * i;
+      const double* row = R < s.rows ? src_row(s, R) : nullptr;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const int64_t k = k0 + tx + 32 * h;
+        tile[ty + 8 * i][tx + 32 * h] = (row && k < s.K) ? src_at(s, row, k) : 0.0;
+      }
+    }
+  } else {
+    const int64_t R = r0 + tx;
+    const double* row = R < s.rows ? src_row(s, R) : nullptr;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int64_t k = k0 + ty + 8 * i;
+      tile[tx][ty + 8 * i] = (row && k < s.K) ? row[k * s.ks] : 0.0;
+    }
   }
   __syncthreads();
+  if (k0 + 2 * tx >= Kpad) return;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const int rr = ty + 8 * i;
-    const int64_t R = r0 + rr, k = k0 + tx;
-    write_slices<NS>(tile[rr][tx], R < s.rows ? ex[R] : 0, out + R * Kpad + k, Rpad * Kpad);
+    const int64_t R = r0 + ty + 8 * i;
+    const int e = R < s.rows ? ex[R] : 0;
+    const double2 v = *(const double2*)&tile[ty + 8 * i][2 * tx];
+    write_slice_pair<NS>(v.x, v.y, e, (uint32_t*)(out + R * Kpad + k0 + 2 * tx), Rpad * Kpad / 2);
   }
 }
 
@@ -380,11 +528,11 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 
 template <int NS, int BN, int NST>
 constexpr int smem_bytes() {
-  return NST * NS * (TILE + BN * BK * 2) + 1024 + 8 * (2 * NST + 1) + 16;
+  return NST * NS * (TILE + BN * BK * 2) + 1024 + 8 * (2 * NST + 2) + 16;
 }
 
 template <int NS, int NG, int BN, int NST>
-cudaError_t launch(const Sliced& A, const Sliced& B, const Args& a, int64_t ntiles, int nchunks, cudaStream_t st) {
+cudaError_t launch(const Sliced& A, const Sliced& B, const Args& a, int64_t ntiles, int splits, cudaStream_t st) {
   constexpr int smem = smem_bytes<NS, BN, NST>();
   static_assert(smem <= 232448, "shared memory per block");
   static std::once_flag once;
@@ -393,8 +541,8 @@ cudaError_t launch(const Sliced& A, const Sliced& B, const Args& a, int64_t ntil
     attr = cudaFuncSetAttribute(k_tc_gemm<NS, NG, BN, NST>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   });
   if (attr != cudaSuccess) return attr;
-  const CUtensorMap& mb = BN == 64 ? B.map64 : B.map;
-  k_tc_gemm<NS, NG, BN, NST><<<dim3((unsigned)ntiles, (unsigned)nchunks), kThreads, smem, st>>>(A.map, mb, a);
+  const CUtensorMap& mb = BN == 64 ? B.map64 : BN == 96 ? B.map96 : B.map;
+  k_tc_gemm<NS, NG, BN, NST><<<dim3((unsigned)ntiles, (unsigned)splits), kThreads, smem, st>>>(A.map, mb, a);
   return cudaGetLastError();
 }
 
@@ -423,7 +571,7 @@ cudaError_t sliced_init(Sliced* s, void* mem, int64_t rows, int64_t K, int ns, c
   if (!enc) return cudaErrorNotSupported;
   const cuuint64_t dims[2] = {(cuuint64_t)s->Kpad, (cuuint64_t)(ns * s->Rpad)};
   const cuuint64_t strides[1] = {(cuuint64_t)(s->Kpad * 2)};
-  const cuuint32_t box[2] = {BK, BM}, box64[2] = {BK, 64};
+  const cuuint32_t box[2] = {BK, BM}, box64[2] = {BK, 64}, box96[2] = {BK, 96};
   const cuuint32_t es[2] = {1, 1};
   if (ns * s->Rpad >= (int64_t)1 << 31) return cudaErrorInvalidValue;
   CUresult r = enc(&s->map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s->s, dims, strides, box, es,
@@ -431,6 +579,10 @@ cudaError_t sliced_init(Sliced* s, void* mem, int64_t rows, int64_t K, int ns, c
                    CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r == CUDA_SUCCESS)
     r = enc(&s->map64, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s->s, dims, strides, box64, es,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r == CUDA_SUCCESS)
+    r = enc(&s->map96, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, s->s, dims, strides, box96, es,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? cudaSuccess : cudaErrorInvalidValue;
@@ -442,8 +594,8 @@ cudaError_t slice(const Source& src, Sliced* d, cudaStream_t st) {
   if (along_k)
     k_rowexp_warp<<<(unsigned)((d->Rpad + 7) / 8), 256, 0, st>>>(src, d->Rpad, d->ex);
   else
-    k_rowexp_thread<<<(unsigned)((d->Rpad + 255) / 256), 256, 0, st>>>(src, d->Rpad, d->ex);
-  const dim3 grid((unsigned)(d->Rpad / 32), (unsigned)(d->Kpad / 32));
+    k_rowexp_lanes<<<(unsigned)(d->Rpad / 32), 1024, 0, st>>>(src, d->Rpad, d->ex);
+  const dim3 grid((unsigned)(d->Rpad / 32), (unsigned)((d->Kpad + 63) / 64));
   switch (d->ns) {
     case 3: k_slice<3><<<grid, 256, 0, st>>>(src, d->Rpad, d->Kpad, d->ex, d->s); break;
     case 7: k_slice<7><<<grid, 256, 0, st>>>(src, d->Rpad, d->Kpad, d->ex, d->s); break;
@@ -458,24 +610,52 @@ namespace {
 // K per chunk: the order-0 group (1 pair) of the mixed mode is exact up to
 // 1024; the order-3 group (4 pairs) of the FP64 mode up to 256.
 int chunk_kb_of(Mode m) { return m == kMixed ? 32 : 8; }
-int bn_of(Mode m) { return m == kMixed ? 128 : 64; }
-// The epilogue writes C itself (1: C = v, 2: C += v) for one K chunk and
-// alpha = +-2^p with beta 0 or 1; otherwise fixed-point sums and a finish pass.
-int direct_mode(int nchunks, const Out& o, int* aexp) {
-  int e = 0;
-  const double f = std::frexp(std::fabs(o.alpha), &e);
-  *aexp = e - 1;
-  if (nchunks != 1 || f != 0.5) return 0;
-  return o.beta == 0.0 ? 1 : (o.beta == 1.0 ? 2 : 0);
+
+// Column width of the tiles and the number of blocks K is split over.
+struct Plan {
+  int bn = 128, splits = 1;
+};
+int64_t tile_count(int64_t M, int64_t N, int bn, bool lower) {
+  const int64_t tm = (M + BM - 1) / BM, tn = (N + bn - 1) / bn;
+  if (!lower) return tm * tn;
+  int64_t t = 0;
+  for (int64_t i = 0; i < tm; ++i) t += std::min<int64_t>(tn, (i * BM + BM - 1) / bn + 1);
+  return t;
+}
+// The plan with the smallest estimate of rounds of the 152 SMs times the time
+// of a block: its chunks, a fixed part (pipeline fill, write-back), and the
+// memset and finish pass when K is split.  Wider FP64 tiles reread A less
+// but leave fewer blocks.
+Plan plan(const Sliced& A, const Sliced& B, Mode mode, const Out& o) {
+  const int ck = chunk_kb_of(mode);
+  const int kblocks = (int)(A.Kpad / BK), nch = (kblocks + ck - 1) / ck;
+  const double part = std::min(1.0, (double)kblocks / ck);  // a single short chunk
+  Plan best;
+  double best_t = INFINITY;
+  const int widths[2] = {mode == kMixed ? 128 : 64, mode == kMixed ? 128 : 96};
+  for (int w = 0; w < (mode == kMixed ? 1 : 2); ++w) {
+    const int bn = widths[w];
+    const double tc = part * (mode == kMixed ? 11.0 : bn == 64 ? 12.0 : 15.0);
+    const double fixed = mode == kMixed ? 6.0 : bn == 64 ? 6.0 : 7.0;
+    const int64_t tiles = tile_count(A.rows, B.rows, bn, o.lower);
+    for (int sp = 1; sp <= (o.fix ? std::min(nch, 64) : 1); ++sp) {
+      const int per = (nch + sp - 1) / sp;
+      const int used = (nch + per - 1) / per;
+      if (used != sp) continue;  // the same blocks with fewer splits
+      const double rounds = (double)((tiles * sp + 151) / 152);
+      const double t = rounds * (per * tc + fixed) + (sp > 1 ? 6.0 + 4e-6 * (double)(A.rows * B.rows) : 0.0);
+      if (t < 0.97 * best_t) {
+        best_t = t;
+        best.bn = bn;
+        best.splits = sp;
+      }
+    }
+  }
+  return best;
 }
 }  // namespace
 
-bool needs_fix(const Sliced& A, const Sliced&, Mode mode, const Out& o) {
-  const int ck = chunk_kb_of(mode);
-  const int nchunks = (int)((A.Kpad / BK + ck - 1) / ck);
-  int aexp;
-  return direct_mode(nchunks, o, &aexp) == 0;
-}
+bool needs_fix(const Sliced& A, const Sliced& B, Mode mode, const Out& o) { return plan(A, B, mode, o).splits > 1; }
 
 cudaError_t gemm(const Sliced& A, const Sliced& B, Mode mode, const Out& o, cudaStream_t st, int64_t* launches) {
   const int ns = slices_of(mode);
@@ -492,40 +672,38 @@ cudaError_t gemm(const Sliced& A, const Sliced& B, Mode mode, const Out& o, cuda
   a.chunk_kb = chunk_kb_of(mode);
   const int nchunks = (a.kblocks + a.chunk_kb - 1) / a.chunk_kb;
   if (nchunks > 65535) return cudaErrorInvalidValue;
-  int aexp = 0;
-  a.direct = direct_mode(nchunks, o, &aexp);
-  a.alpha_exp = aexp;
-  a.alpha_neg = o.alpha < 0 ? 1 : 0;
-  if (!a.direct && !o.fix) return cudaErrorInvalidValue;
+  const Plan pl = plan(A, B, mode, o);
+  a.block_kb = (nchunks + pl.splits - 1) / pl.splits * a.chunk_kb;
   int lg = 0;
   while (((int64_t)1 << lg) < std::max<int64_t>(A.K, 2)) ++lg;
-  a.U = std::max(16, std::min(46, 47 - lg));
+  a.U = std::max(24, std::min(46, 47 - lg));
   a.exa = A.ex;
   a.exb = B.ex;
   a.C = o.C;
   a.ldc = o.ldc;
-  a.fix = (unsigned long long*)o.fix;
+  a.alpha = o.alpha;
+  a.beta = o.beta;
+  a.fix = pl.splits > 1 ? (unsigned long long*)o.fix : nullptr;
   a.ldfix = o.ldfix;
   a.err = o.err;
   a.lower = o.lower ? 1 : 0;
-  const int BN = bn_of(mode);
-  const int64_t tm = (M + BM - 1) / BM, tn = (N + BN - 1) / BN;
-  a.tiles_m = (int32_t)tm;
+  const int64_t tm = (M + BM - 1) / BM, tn = (N + pl.bn - 1) / pl.bn;
   a.tiles_n = (int32_t)tn;
   const int64_t ntiles = tm * tn;
   if (ntiles >= ((int64_t)1 << 31)) return cudaErrorInvalidValue;
   cudaError_t e = cudaSuccess;
-  if (!a.direct) {
+  if (a.fix) {
     e = cudaMemset2DAsync(o.fix, (size_t)(o.ldfix * 8), 0, (size_t)(M * 8), (size_t)N, st);
     if (e != cudaSuccess) return e;
   }
   // mixed: orders 0 | 1-2 (2 groups, 128-column tiles, 4 stages);
-  // FP64: orders 0 | 1 | 2 | 3 | 4-6 (5 groups, 64-column tiles, 2 stages)
-  e = mode == kMixed ? launch<3, 2, 128, 4>(A, B, a, ntiles, nchunks, st)
-                     : launch<7, 5, 64, 2>(A, B, a, ntiles, nchunks, st);
+  // FP64: orders 0 | 1 | 2 | 3 | 4-6 (5 groups, 64- or 96-column tiles, 2 stages)
+  e = mode == kMixed ? launch<3, 2, 128, 4>(A, B, a, ntiles, pl.splits, st)
+      : pl.bn == 64  ? launch<7, 5, 64, 2>(A, B, a, ntiles, pl.splits, st)
+                     : launch<7, 5, 96, 2>(A, B, a, ntiles, pl.splits, st);
   if (e != cudaSuccess) return e;
   if (launches) *launches += 1;
-  if (!a.direct) {
+  if (a.fix) {
     const int64_t total = M * N;
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 152 * 32);
     k_finish<<<grid, 256, 0, st>>>(M, N, o.fix, o.ldfix, A.ex, B.ex, a.U, o.alpha, o.beta, o.C, o.ldc, a.lower);
@@ -569,11 +747,13 @@ extern "C" int msdp_tc_gemm(int32_t precision, int32_t transa, int32_t transb, i
   sb.p = B; sb.rows = N; sb.K = K; sb.nr = N; sb.bs = 0;
   sb.rs = transb ? 1 : ldb; sb.ks = transb ? ldb : 1;
   if (e == cudaSuccess) e = slice(sa, &SA, st);
-  if (e == cudaSuccess) e = slice(sb, &SB, st);
+  // op(A) op(A)': the rows of both operands are the same elements
+  const bool same = A == B && M == N && sa.rs == sb.rs && sa.ks == sb.ks;
+  if (e == cudaSuccess && !same) e = slice(sb, &SB, st);
   Out o;
   o.C = C; o.ldc = ldc; o.alpha = alpha; o.beta = beta; o.lower = lower != 0;
   o.fix = (long long*)(mem + ba + bb); o.ldfix = M; o.err = err;
-  if (e == cudaSuccess) e = gemm(SA, SB, mode, o, st, nullptr);
+  if (e == cudaSuccess) e = gemm(SA, same ? SA : SB, mode, o, st, nullptr);
   int herr = 0;
   if (e == cudaSuccess) e = cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);

@@ -25,8 +25,9 @@
 //           Schur assembly of the mixed whole-GPU path); 128 x 128 tiles;
 //   kFp64   7 slices, 28 products; orders 0, 1, 2 and 3 exact per chunk of
 //           256, orders 4-6 in one accumulator: relative error about 5e-15
-//           of |A||B| (the FP64 path's products); 128 x 64 tiles, so the
-//           five accumulators fit the 512 columns of tensor memory.
+//           of |A||B| (the FP64 path's products); tiles of 128 x 64 or
+//           128 x 96, so the five accumulators fit the 512 columns of tensor
+//           memory.
 //
 // Operands reach shared memory by TMA (cp.async.bulk.tensor, 64-byte
 // swizzle, one 128 x 32 bf16 box per slice and stage), the MMA is issued by
@@ -65,6 +66,7 @@ struct Sliced {
   int ns = 0;
   CUtensorMap map;    // boxes of 128 rows (A operand, 128-column B tiles)
   CUtensorMap map64;  // boxes of 64 rows (64-column B tiles)
+  CUtensorMap map96;  // boxes of 96 rows (96-column B tiles)
 };
 
 int64_t sliced_bytes(int64_t rows, int64_t K, int ns);
@@ -112,18 +114,59 @@ __device__ __forceinline__ long long to_fixed(double x, int e) {
   return b < 0 ? -v : v;
 }
 
-// Cut x (row exponent e) into NS slices q_t 2^-8t (bf16) and store them
-// at out[t * slice_stride].
+// The NS slices of x (row exponent e): integers q_t with |q_t| <= 128 and
+// x 2^-e = sum q_t 2^-(8t+7) + remainder, each rounded half up from what the
+// ones before left.  The first three come from the high word of the
+// fixed-point value alone, the fourth leaves 31 bits, so only 32-bit
+// instructions are needed.
+template <int NS>
+__device__ __forceinline__ void slice_ints(double x, int e, int (&q)[NS]) {
+  const long long r = to_fixed(x, e);
+  int hi = (int)(r >> 32);
+  const unsigned lo = (unsigned)r;
+#pragma unroll
+  for (int t = 0; t < 3 && t < NS; ++t) {
+    const int sft = 23 - 8 * t;
+    q[t] = (hi + (1 << (sft - 1))) >> sft;
+    hi -= q[t] << sft;
+  }
+  if (NS > 3) {
+    q[3] = ((int)__funnelshift_l(lo, (unsigned)hi, 2) + 1) >> 1;
+    int w = (int)(lo - ((unsigned)q[3] << 31));
+#pragma unroll
+    for (int t = 4; t < NS; ++t) {
+      const int sft = 55 - 8 * t;
+      q[t] = (w + (1 << (sft - 1))) >> sft;
+      w -= q[t] << sft;
+    }
+  }
+}
+// Upper half of the FP32 pattern of q 2^-8t: the bf16 pattern (|q| <= 128 has
+// at most 8 significant bits); 1.5 2^23 + q and back converts without the
+// conversion unit.
+__device__ __forceinline__ uint32_t slice_bits(int q, int t) {
+  const float f = __int_as_float(0x4B400000 + q) - 12582912.0f;
+  return __float_as_uint(f * __int_as_float((127 - 8 * t) << 23));
+}
+
+// Slices of x0 and x1 (neighbours along k) stored as bf16 pairs at
+// out[t * slice_stride].
+template <int NS>
+__device__ __forceinline__ void write_slice_pair(double x0, double x1, int e, uint32_t* out, int64_t slice_stride) {
+  int q0[NS], q1[NS];
+  slice_ints<NS>(x0, e, q0);
+  slice_ints<NS>(x1, e, q1);
+#pragma unroll
+  for (int t = 0; t < NS; ++t)
+    out[t * slice_stride] = __byte_perm(slice_bits(q0[t], t), slice_bits(q1[t], t), 0x7632);
+}
+// Slices of x stored at out[t * slice_stride].
 template <int NS>
 __device__ __forceinline__ void write_slices(double x, int e, __nv_bfloat16* out, int64_t slice_stride) {
-  long long r = to_fixed(x, e);
+  int q[NS];
+  slice_ints<NS>(x, e, q);
 #pragma unroll
-  for (int t = 0; t < NS; ++t) {
-    const int sft = 55 - 8 * t;
-    const long long q = (r + (1ll << (sft - 1))) >> sft;
-    r -= q * (1ll << sft);
-    out[t * slice_stride] = __float2bfloat16_rn((float)q * __int_as_float((127 - 8 * t) << 23));
-  }
+  for (int t = 0; t < NS; ++t) out[t * slice_stride] = __ushort_as_bfloat16((unsigned short)(slice_bits(q[t], t) >> 16));
 }
 
 }  // namespace tcg
