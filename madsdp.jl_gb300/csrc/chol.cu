@@ -2,146 +2,383 @@
 #include "chol.h"
 
 #include <algorithm>
+#include <mutex>
 
 namespace chol {
 namespace {
 
 constexpr int NB = 32;    // block column width (= K of the trailing update)
-constexpr int ROWS = 64;  // panel rows per thread block, one per thread
+constexpr int ROWS = 32;  // panel rows per thread block, one per lane
 
-template <class T>
-__device__ __forceinline__ T sqrt_t(T x);
-template <>
-__device__ __forceinline__ double sqrt_t<double>(double x) { return sqrt(x); }
-template <>
-__device__ __forceinline__ float sqrt_t<float>(float x) { return sqrtf(x); }
+// sqrt(d) and 1/sqrt(d) of a positive finite pivot.  double: an FP32
+// reciprocal square root of the mantissa and one third-order correction
+// (y (1 + e/2 + 3/8 e^2), e = 1 - m y^2), then one Newton correction of the
+// root: about 300 clocks of dependent FP64 instructions where sqrt and a
+// division take about 1000, and the 32 pivots are one serial chain.
+__device__ __forceinline__ void pivot_root(double d, double& root, double& inv) {
+  const long long b = __double_as_longlong(d);
+  const int field = (int)(b >> 52);
+  if (field == 0) {  // subnormal
+    root = sqrt(d);
+    inv = 1.0 / root;
+    return;
+  }
+  const int k = (field - 1023) >> 1, odd = (field - 1023) & 1;
+  const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | ((long long)(1023 + odd) << 52));  // [1, 4)
+  const double y = (double)rsqrtf((float)m);
+  const double e = fma(-m * y, y, 1.0);
+  const double z = fma(y * e, fma(0.375, e, 0.5), y);
+  inv = __longlong_as_double(__double_as_longlong(z) - ((long long)k << 52));
+  const double s = d * inv;
+  root = fma(fma(-s, s, d) * 0.5, inv, s);
+}
+__device__ __forceinline__ void pivot_root(float d, float& root, float& inv) {
+  root = sqrtf(d);
+  inv = 1.0f / root;
+}
 
 // Block column k0: factor the diagonal block, solve the panel rows of this
 // thread block, write both back and the panel's slices for the update.
 // The factored diagonal block goes to `diag` (NB x NB per block column), not
 // to A: other thread blocks of the same launch may still be reading it.
+//
+// Warp 0 factors the diagonal block (row per lane, in registers; every block
+// does so, none waits on another) and publishes its columns in shared memory;
+// warp 1 eliminates the same columns from 32 panel rows, four columns behind
+// (one named barrier per four columns); all four warps then cut the rows into
+// slices.  Bound by the chain of 32 pivots and by warp 0's 500 FP64
+// instructions on its quarter of the SM: 57 us (ncu).  A block-wide factor
+// with three barriers, a square root and a division per column, and 64 rows
+// per block, took 99-123 us.
 template <class T, int NS>
-__global__ void __launch_bounds__(ROWS) k_panel(int n, int k0, double* __restrict__ A, int64_t lda,
-                                               int* __restrict__ info, __nv_bfloat16* __restrict__ sl,
-                                               int32_t* __restrict__ ex, int64_t Rpad, double* __restrict__ diag) {
-  __shared__ T L[NB][NB + 1];
+__global__ void __launch_bounds__(128) k_panel(int n, int k0, double* __restrict__ A, int64_t lda,
+                                              int* __restrict__ info, __nv_bfloat16* __restrict__ sl,
+                                              int32_t* __restrict__ ex, int64_t Rpad, double* __restrict__ diag) {
+  __shared__ T col[NB][NB];       // col[j][r] = L(r, j)
   __shared__ T rdiag[NB];
-  __shared__ int bad;
+  __shared__ double xs[ROWS][NB + 1];
+  __shared__ int exs[ROWS];
+  __shared__ int bad_s;
   if (*(volatile int*)info != 0) return;  // an earlier block column failed
   const int kb = min(NB, n - k0);
-  const int tid = threadIdx.x;
-  for (int idx = tid; idx < NB * NB; idx += ROWS) {
-    const int r = idx % NB, c = idx / NB;
-    T v = (T)0;
-    if (r < kb && c < kb) {
-      if (r >= c) v = (T)A[(k0 + r) + (int64_t)(k0 + c) * lda];
-    } else if (r == c) {
-      v = (T)1;
-    }
-    L[r][c] = v;
-  }
-  if (tid == 0) bad = 0;
-  __syncthreads();
-  for (int j = 0; j < kb; ++j) {
-    if (tid == 0) {
-      const T d = L[j][j];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // panel rows exist only below a full diagonal block (k0 + NB < n)
+  const int64_t R = (int64_t)blockIdx.x * ROWS + lane, i = (int64_t)k0 + NB + R;
+  const bool own = kb == NB && i < n;
+  T x[NB];
+  if (warp == 0) {
+#pragma unroll
+    for (int c = 0; c < NB; ++c)
+      x[c] = (lane < kb && c <= lane) ? (T)A[(k0 + lane) + (int64_t)(k0 + c) * lda] : (lane == c ? (T)1 : (T)0);
+    int bad = 0;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      T d = __shfl_sync(0xffffffffu, x[j], j);
       if (!(d > (T)0) || !isfinite(d)) {
-        bad = k0 + j + 1;
-      } else {
-        const T sq = sqrt_t<T>(d);
-        L[j][j] = sq;
-        rdiag[j] = (T)1 / sq;
+        if (!bad) bad = k0 + j + 1;
+        d = (T)1;  // the factor is not used
       }
+      T root, inv;
+      pivot_root(d, root, inv);
+      const T l = lane == j ? root : x[j] * inv;
+      x[j] = l;
+      col[j][lane] = l;
+      if (lane == j) rdiag[j] = inv;
+      __syncwarp();
+      if ((j & 3) == 3) asm volatile("bar.arrive %0, 64;" ::"r"(1 + (j >> 2)) : "memory");
+#pragma unroll
+      for (int c = j + 1; c < NB; ++c) x[c] -= l * col[j][c];
     }
-    __syncthreads();
-    if (bad) break;
-    if (tid > j && tid < kb) L[tid][j] *= rdiag[j];
-    __syncthreads();
-    if (tid > j && tid < kb) {
-      const T lij = L[tid][j];
-      for (int c = j + 1; c <= tid; ++c) L[tid][c] -= lij * L[c][j];
+    if (lane == 0) bad_s = bad;
+  } else if (warp == 1) {
+#pragma unroll
+    for (int c = 0; c < NB; ++c) x[c] = own ? (T)A[i + (int64_t)(k0 + c) * lda] : (T)0;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) {
+      if ((j & 3) == 0) asm volatile("bar.sync %0, 64;" ::"r"(1 + (j >> 2)) : "memory");
+      x[j] *= rdiag[j];
+#pragma unroll
+      for (int c = j + 1; c < NB; ++c) x[c] -= x[j] * col[j][c];
     }
-    __syncthreads();
+    int mx = 0;
+#pragma unroll
+    for (int c = 0; c < NB; ++c) {
+      xs[lane][c] = (double)x[c];
+      mx = max(mx, tcg::exp_field((double)x[c]));
+    }
+    exs[lane] = tcg::row_exp(mx);
   }
-  if (bad) {
-    if (blockIdx.x == 0 && tid == 0) atomicCAS(info, 0, bad);
+  __syncthreads();
+  if (bad_s) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(info, 0, bad_s);
     return;
   }
-  if (blockIdx.x == 0)
-    for (int idx = tid; idx < NB * NB; idx += ROWS) diag[(int64_t)k0 * NB + idx] = (double)L[idx % NB][idx / NB];
-  // panel rows exist only below a full diagonal block (k0 + NB < n)
-  const int64_t i = (int64_t)k0 + NB + (int64_t)blockIdx.x * ROWS + tid;
-  if (kb < NB || i >= n) return;
-  T x[NB];
+  if (warp == 0 && blockIdx.x == 0) {
 #pragma unroll
-  for (int c = 0; c < NB; ++c) x[c] = (T)A[i + (int64_t)(k0 + c) * lda];
-  // x <- x L11^-T, column by column (each solved entry updates the later ones)
-#pragma unroll
-  for (int c = 0; c < NB; ++c) {
-    x[c] *= rdiag[c];
-#pragma unroll
-    for (int k = c + 1; k < NB; ++k) x[k] -= x[c] * L[k][c];
+    for (int c = 0; c < NB; ++c) diag[((int64_t)k0 + c) * NB + lane] = lane >= c ? (double)x[c] : 0.0;
   }
-  int mx = 0;
+  if (warp == 1 && own) {
 #pragma unroll
-  for (int c = 0; c < NB; ++c) {
-    const double v = (double)x[c];
-    A[i + (int64_t)(k0 + c) * lda] = v;
-    mx = max(mx, tcg::exp_field(v));
+    for (int c = 0; c < NB; ++c) A[i + (int64_t)(k0 + c) * lda] = (double)x[c];
+    ex[R] = exs[lane];
   }
-  const int e = tcg::row_exp(mx);
-  const int64_t R = i - (k0 + NB);
-  ex[R] = e;
+  // slices: eight columns of one row per thread
+  const int row = threadIdx.x >> 2, seg = (threadIdx.x & 3) * 8;
+  const int64_t Rr = (int64_t)blockIdx.x * ROWS + row;
+  if (kb == NB && k0 + NB + Rr < n) {
+    double v[8];
 #pragma unroll
-  for (int c = 0; c < NB; ++c) tcg::write_slices<NS>((double)x[c], e, sl + R * NB + c, Rpad * NB);
-}
-
-// Lower triangles of the factored diagonal blocks into A (after the last
-// block column; the info check skips a failed factorization).
-__global__ void k_put_diag(int n, double* __restrict__ A, int64_t lda, const double* __restrict__ diag,
-                           const int* __restrict__ info) {
-  if (*info != 0) return;
-  const int64_t total = (int64_t)((n + NB - 1) / NB) * NB * NB;
-  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
-       idx += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t k0 = idx / (NB * NB) * NB;
-    const int q = (int)(idx % (NB * NB)), r = q % NB, c = q / NB;
-    if (r >= c && k0 + r < n) A[(k0 + r) + (k0 + c) * lda] = diag[idx];
+    for (int c = 0; c < 8; ++c) v[c] = xs[row][seg + c];
+    tcg::write_slices8<NS>(v, exs[row], sl + Rr * NB + seg, Rpad * NB);
   }
 }
 
-// Inverse of each factored diagonal block (one thread block of NB warps per
-// block; warp c forms column c row by row with a warp sum).
-__global__ void __launch_bounds__(NB * 32) k_diag_inverse(int n, const double* __restrict__ diag,
-                                                          double* __restrict__ dinv, const int* __restrict__ info) {
+// After the last block column (the info check skips a failed factorization):
+// the lower triangles of the factored diagonal blocks into A and, when dinv
+// is given, their inverses.  One warp per block; lane c solves L x = e_c in
+// registers (528 FP64 instructions, about 6 us).
+__global__ void __launch_bounds__(32) k_diag_finish(int n, double* __restrict__ A, int64_t lda,
+                                                   const double* __restrict__ diag, double* __restrict__ dinv,
+                                                   const int* __restrict__ info) {
   if (*info != 0) return;
-  __shared__ double Ls[NB][NB + 1], inv[NB][NB + 1];
+  __shared__ double Ls[NB][NB];  // Ls[c][r] = L(r, c)
   const int64_t k0 = (int64_t)blockIdx.x * NB;
-  const int kb = (int)min((int64_t)NB, (int64_t)n - k0);
-  const int t = threadIdx.x, lane = t & 31, c = t >> 5;
-  {
-    const int r = t % NB, cc = t / NB;
-    Ls[r][cc] = diag[k0 * NB + t];  // column-major NB x NB block
-    inv[r][cc] = 0.0;
+  const int kb = (int)min((int64_t)NB, (int64_t)n - k0), lane = threadIdx.x;
+#pragma unroll 8
+  for (int c = 0; c < NB; ++c) {
+    const double v = diag[(k0 + c) * NB + lane];
+    Ls[c][lane] = v;
+    if (lane >= c && lane < kb) A[(k0 + lane) + (k0 + c) * lda] = v;
   }
-  __syncthreads();
-  for (int r = 0; r < kb; ++r) {
-    double term = (lane >= c && lane < r) ? Ls[r][lane] * inv[lane][c] : 0.0;
-    for (int o = 16; o; o >>= 1) term += __shfl_xor_sync(0xffffffffu, term, o);
-    if (lane == 0 && c <= r) inv[r][c] = ((r == c ? 1.0 : 0.0) - term) / Ls[r][r];
-    __syncthreads();
+  if (!dinv) return;
+  __syncwarp();
+  const double rd = 1.0 / Ls[lane][lane];  // the padding is the identity
+  double x[NB];
+#pragma unroll
+  for (int r = 0; r < NB; ++r) x[r] = r == lane ? 1.0 : 0.0;
+#pragma unroll
+  for (int k = 0; k < NB; ++k) {
+    x[k] *= __shfl_sync(0xffffffffu, rd, k);
+#pragma unroll
+    for (int r = k + 1; r < NB; ++r) x[r] = fma(-Ls[k][r], x[k], x[r]);
   }
-  {
-    const int r = t % NB, cc = t / NB;
-    dinv[k0 * NB + t] = (r < kb && cc < kb) ? inv[r][cc] : 0.0;
+#pragma unroll
+  for (int r = 0; r < NB; ++r) dinv[(k0 + lane) * NB + r] = (r < kb && lane < kb) ? x[r] : 0.0;
+}
+
+// ---------------------------------------------------------------- triangular solves
+__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, int rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ unsigned long long gtime() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+// Bounded wait for a phase of a barrier that a block of the cluster completes.
+__device__ __forceinline__ bool cluster_wait(uint32_t bar, uint32_t parity, unsigned long long deadline) {
+  for (uint32_t it = 0;; ++it) {
+    uint32_t ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, "
+        "p;\n}"
+        : "=r"(ok)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((it & 255u) == 255u && gtime() > deadline) return false;
   }
 }
 
-// x <- L^-T L^-1 x with the factor in L (lower) and the inverses of its
-// diagonal blocks; one thread block, block row by block row.  The sums over
+constexpr int kSolveThreads = 512;
+constexpr int kSolveSmemMax = 220 * 1024;
+constexpr unsigned long long kSolveWaitNs = 2000000000ull;
+
+// Shared memory of a block: x (padded), partial sums of its blocks, two
+// exchange buffers per warp group, one barrier per block row.
+__host__ __device__ inline int64_t solve_smem(int nbk, int cs) {
+  const int own = (nbk + cs - 1) / cs;
+  return 8 * ((int64_t)nbk * NB + (int64_t)own * NB * NB + 4 * 2 * 4 * NB + nbk);
+}
+
+// x <- L^-T L^-1 x in one cluster.  Block rows of 32 go round the cluster's
+// blocks.  Forward: as soon as y_b is known its owner writes it to every
+// block's shared memory and signals barrier b there; every block subtracts
+// L(B, b) y_b from its own later block rows B (a group of four warps per
+// block row, eight columns a warp), the owner of b + 1 first.  Backward: the
+// same with L(b, B)' (lanes along the rows of L, so that its columns are
+// read in order; the sum over the lanes is taken when B's turn comes).  Bound
+// by the FP64 pipes of the cluster's SMs (n^2 multiply-adds at 1.6 per clock
+// and SM) and, per block row, by one exchange and two 32 x 32 products:
+// 385 us at n = 2000 and 25 us at n = 100 (ncu).  One block of 1024 threads
+// alone took 1706 and 46 us.
+// Every wait is bounded; a wait that runs out sets *err and the block goes on
+// to the closing cluster barrier.
+__global__ void __launch_bounds__(kSolveThreads) k_chol_solve(int n, const double* __restrict__ L, int64_t ld,
+                                                             const double* __restrict__ dinv, double* __restrict__ x,
+                                                             const int* __restrict__ info, int* __restrict__ err) {
+  if (*info != 0) return;  // the same for every block of the cluster
+  extern __shared__ double sm[];
+  int cs, rank;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cs));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int nbk = (n + NB - 1) / NB, own = (nbk + cs - 1) / cs;
+  double* xv = sm;                                 // [nbk * NB]
+  double* accs = xv + (int64_t)nbk * NB;           // [own][NB][NB]
+  double* exch = accs + (int64_t)own * NB * NB;    // [4 groups][2][4][NB]
+  unsigned long long* bars = (unsigned long long*)(exch + 4 * 2 * 4 * NB);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int cg = warp & 3, grp = warp >> 2;        // eight columns; the group's block rows q = grp, grp + 4, ...
+  double* ea = exch + grp * 2 * 4 * NB;
+  double* eb = ea + 4 * NB;
+  for (int t = threadIdx.x; t < nbk * NB; t += kSolveThreads) xv[t] = t < n ? x[t] : 0.0;
+  for (int t = threadIdx.x; t < own * NB * NB; t += kSolveThreads) accs[t] = 0.0;
+  for (int t = threadIdx.x; t < nbk; t += kSolveThreads)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(bars + t)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  const unsigned long long deadline = gtime() + kSolveWaitNs;
+  bool ok = true;
+  auto group_sync = [&] { asm volatile("bar.sync %0, 128;" ::"r"(1 + grp) : "memory"); };
+  // v (the right-hand side of block row b, in every warp of the group), then
+  // x_b = D v (or D' v) to every block of the cluster, and its barrier
+  auto finish = [&](int b, const double (&dreg)[8], double v) {
+    double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+    for (int c = 0; c < 8; c += 2) {
+      s0 = fma(dreg[c], __shfl_sync(0xffffffffu, v, cg * 8 + c), s0);
+      s1 = fma(dreg[c + 1], __shfl_sync(0xffffffffu, v, cg * 8 + c + 1), s1);
+    }
+    eb[cg * NB + lane] = s0 + s1;
+    group_sync();
+    const double y = (eb[lane] + eb[NB + lane]) + (eb[2 * NB + lane] + eb[3 * NB + lane]);
+    const uint32_t dst = smem_u32(xv + (int64_t)b * NB + lane), bar = smem_u32(bars + b);
+    for (int r = cg; r < cs; r += 4)
+      asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(cluster_addr(dst, r)), "d"(y) : "memory");
+    asm volatile("fence.acq_rel.cluster;" ::: "memory");
+    __syncwarp();
+    if (lane == 0)
+      for (int r = cg; r < cs; r += 4)
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr(bar, r))
+                     : "memory");
+  };
+  // ---- forward: L y = x
+  for (int b = -1; b < nbk - 1; ++b) {
+    // the group's part of the next block row, before y_b is there
+    const int nxt = b + 1, q0 = nxt / cs;
+    const bool critical = nxt % cs == rank && (q0 & 3) == grp;
+    double dreg[8], lreg[8];
+    if (critical) {
+      const bool rok = nxt * NB + lane < n;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        dreg[c] = dinv[((int64_t)nxt * NB + cg * 8 + c) * NB + lane];
+        lreg[c] = (b >= 0 && rok) ? L[(int64_t)nxt * NB + lane + ((int64_t)b * NB + cg * 8 + c) * ld] : 0.0;
+      }
+    }
+    if (b >= 0) ok = ok && cluster_wait(smem_u32(bars + b), 0, deadline);
+    const double* yb = xv + (int64_t)(b < 0 ? 0 : b) * NB + cg * 8;
+    if (critical) {
+      double s0 = accs[(q0 * 4 + cg) * NB + lane], s1 = 0.0;
+#pragma unroll
+      for (int c = 0; c < 8; c += 2) {
+        s0 = fma(lreg[c], yb[c], s0);
+        s1 = fma(lreg[c + 1], yb[c + 1], s1);
+      }
+      ea[cg * NB + lane] = s0 + s1;
+      group_sync();
+      const double sum = (ea[lane] + ea[NB + lane]) + (ea[2 * NB + lane] + ea[3 * NB + lane]);
+      finish(nxt, dreg, xv[(int64_t)nxt * NB + lane] - sum);
+      accs[(q0 * 4 + cg) * NB + lane] = 0.0;
+    }
+    if (b >= 0) {
+      for (int q = grp; q < own; q += 4) {
+        const int Bq = q * cs + rank;
+        if (Bq <= b + 1 || Bq >= nbk) continue;
+        const int64_t row = (int64_t)Bq * NB + lane;
+        if (row < n) {
+          const double* Lr = L + row + ((int64_t)b * NB + cg * 8) * ld;
+          double s0 = accs[(q * 4 + cg) * NB + lane], s1 = 0.0;
+#pragma unroll
+          for (int c = 0; c < 8; c += 2) {
+            s0 = fma(Lr[c * ld], yb[c], s0);
+            s1 = fma(Lr[(c + 1) * ld], yb[c + 1], s1);
+          }
+          accs[(q * 4 + cg) * NB + lane] = s0 + s1;
+        }
+      }
+    }
+  }
+  ok = ok && cluster_wait(smem_u32(bars + nbk - 1), 0, deadline);
+  // every y has arrived everywhere before any z overwrites it
+  __syncthreads();
+  for (int t = threadIdx.x; t < own * NB * NB; t += kSolveThreads) accs[t] = 0.0;
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  // ---- backward: L' z = y
+  for (int b = nbk; b > 0; --b) {
+    const int nxt = b - 1, q0 = nxt / cs;
+    const bool critical = nxt % cs == rank && (q0 & 3) == grp;
+    double dreg[8], lreg[8];
+    if (critical) {
+      const bool rok = b < nbk && b * NB + lane < n;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        dreg[c] = dinv[((int64_t)nxt * NB + lane) * NB + cg * 8 + c];
+        lreg[c] = rok ? L[(int64_t)b * NB + lane + ((int64_t)nxt * NB + cg * 8 + c) * ld] : 0.0;
+      }
+    }
+    if (b < nbk) ok = ok && cluster_wait(smem_u32(bars + b), 1, deadline);
+    const double zb = b < nbk ? xv[(int64_t)b * NB + lane] : 0.0;
+    if (critical) {
+      // the eight columns' sums over the lanes: written out, then column
+      // `lane` added up, eight lanes' terms per warp
+      double* ac = accs + ((int64_t)q0 * NB + cg * 8) * NB;
+#pragma unroll
+      for (int c = 0; c < 8; ++c) ac[c * NB + lane] = fma(lreg[c], zb, ac[c * NB + lane]);
+      group_sync();
+      const double* col = accs + ((int64_t)q0 * NB + lane) * NB;
+      double s0 = 0.0, s1 = 0.0;
+#pragma unroll
+      for (int t = 0; t < 8; t += 2) {
+        // rotated by the column so that the lanes read different banks
+        s0 += col[cg * 8 + ((t + lane) & 7)];
+        s1 += col[cg * 8 + ((t + 1 + lane) & 7)];
+      }
+      ea[cg * NB + lane] = s0 + s1;
+      group_sync();
+      const double sum = (ea[lane] + ea[NB + lane]) + (ea[2 * NB + lane] + ea[3 * NB + lane]);
+      finish(nxt, dreg, xv[(int64_t)nxt * NB + lane] - sum);
+    }
+    if (b < nbk) {
+      const bool rok = b * NB + lane < n;
+      for (int q = grp; q < own; q += 4) {
+        const int Bq = q * cs + rank;
+        if (Bq >= b - 1) continue;
+        if (rok) {
+          const double* Lc = L + (int64_t)b * NB + lane + ((int64_t)Bq * NB + cg * 8) * ld;
+          double* ac = accs + ((int64_t)q * NB + cg * 8) * NB;
+#pragma unroll
+          for (int c = 0; c < 8; ++c) ac[c * NB + lane] = fma(Lc[c * ld], zb, ac[c * NB + lane]);
+        }
+      }
+    }
+  }
+  ok = ok && cluster_wait(smem_u32(bars), 1, deadline);
+  if (!ok) atomicExch(err, 5);
+  __syncthreads();
+  for (int t = rank * kSolveThreads + threadIdx.x; t < n; t += cs * kSolveThreads) x[t] = ok ? xv[t] : nan("");
+  // no block leaves while another may still write to its shared memory
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The same in one thread block of 1024 threads, for orders (above 8500) whose
+// vectors do not fit the cluster's shared memory: block row by block row, the sums over
 // the solved part read NB consecutive entries per column (coalesced), four
 // independent accumulators per thread.
-__global__ void __launch_bounds__(1024) k_chol_solve(int n, const double* __restrict__ L, int64_t ld,
+__global__ void __launch_bounds__(1024) k_chol_solve_block(int n, const double* __restrict__ L, int64_t ld,
                                                      const double* __restrict__ dinv, double* x,
                                                      const int* __restrict__ info) {
   if (*info != 0) return;
@@ -215,8 +452,9 @@ int64_t work_bytes(int64_t nmax) {
   return panel_bytes(nmax) + 2 * (nmax + NB) * NB * 8;
 }
 
-cudaError_t init(Work* w, void* mem, int64_t nmax, int* err, cudaStream_t st) {
+cudaError_t init(Work* w, void* mem, int64_t nmax, int* err, cudaStream_t st, bool solves) {
   w->mem = mem;
+  w->solves = solves;
   w->nmax = std::max<int64_t>(nmax, 1);
   w->err = err;
   w->diag = (double*)((char*)mem + panel_bytes(w->nmax));
@@ -227,10 +465,40 @@ cudaError_t init(Work* w, void* mem, int64_t nmax, int* err, cudaStream_t st) {
 cudaError_t solve(const Work& w, int n, const double* L, int64_t ld, double* x, const int* info, cudaStream_t st,
                   int64_t* launches) {
   if (n <= 0) return cudaSuccess;
-  if (n > w.nmax) return cudaErrorInvalidValue;
-  k_chol_solve<<<1, 1024, 0, st>>>(n, L, ld, w.dinv, x, info);
+  if (n > w.nmax || !w.solves) return cudaErrorInvalidValue;
+  // 16 blocks (more than the portable 8) from 9 block rows on: the work is
+  // FP64-pipe bound, n^2 multiply-adds at 1.6 per clock and SM
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  static bool wide = false;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(k_chol_solve, cudaFuncAttributeMaxDynamicSharedMemorySize, kSolveSmemMax);
+    wide = cudaFuncSetAttribute(k_chol_solve, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    cudaGetLastError();
+  });
+  if (attr != cudaSuccess) return attr;
+  const int nbk = (n + NB - 1) / NB;
+  int cs = 1;
+  while (cs < nbk && cs < (wide ? 16 : 8)) cs *= 2;
+  if (solve_smem(nbk, cs) > kSolveSmemMax) {
+    k_chol_solve_block<<<1, 1024, 0, st>>>(n, L, ld, w.dinv, x, info);
+    if (launches) *launches += 1;
+    return cudaGetLastError();
+  }
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)cs);
+  cfg.blockDim = dim3(kSolveThreads);
+  cfg.dynamicSmemBytes = (size_t)solve_smem(nbk, cs);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cs;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, k_chol_solve, n, L, ld, (const double*)w.dinv, x, info, w.err);
   if (launches) *launches += 1;
-  return cudaGetLastError();
+  return e != cudaSuccess ? e : cudaGetLastError();
 }
 
 cudaError_t potrf(Work& w, int n, double* A, int64_t lda, int* info, tcg::Mode mode, cudaStream_t st,
@@ -249,9 +517,9 @@ cudaError_t potrf(Work& w, int n, double* A, int64_t lda, int* info, tcg::Mode m
     const int64_t nr = n - k0 - kb;
     const unsigned grid = (unsigned)std::max<int64_t>(1, (nr + ROWS - 1) / ROWS);
     if (mode == tcg::kMixed)
-      k_panel<float, 3><<<grid, ROWS, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
+      k_panel<float, 3><<<grid, 128, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
     else
-      k_panel<double, 7><<<grid, ROWS, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
+      k_panel<double, 7><<<grid, 128, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;
@@ -269,10 +537,8 @@ cudaError_t potrf(Work& w, int n, double* A, int64_t lda, int* info, tcg::Mode m
     }
   }
   if (n > 0) {
-    const int64_t total = (int64_t)((n + NB - 1) / NB) * NB * NB;
-    k_put_diag<<<(unsigned)std::min<int64_t>((total + 255) / 256, 1024), 256, 0, st>>>(n, A, lda, w.diag, info);
-    k_diag_inverse<<<(unsigned)((n + NB - 1) / NB), NB * 32, 0, st>>>(n, w.diag, w.dinv, info);
-    if (launches) *launches += 2;
+    k_diag_finish<<<(unsigned)((n + NB - 1) / NB), 32, 0, st>>>(n, A, lda, w.diag, w.solves ? w.dinv : nullptr, info);
+    if (launches) *launches += 1;
     e = cudaGetLastError();
   }
   return e;
@@ -299,7 +565,7 @@ extern "C" int msdp_dense_cholesky(int32_t precision, int32_t n, double* A, int6
   int* derr = dinfo + 1;
   chol::Work w;
   cudaError_t e = cudaMemsetAsync(derr, 0, sizeof(int), st);
-  if (e == cudaSuccess) e = chol::init(&w, mem, n, derr, st);
+  if (e == cudaSuccess) e = chol::init(&w, mem, n, derr, st, false);
   if (e == cudaSuccess)
     e = chol::potrf(w, n, A, lda, dinfo, precision == MSDP_MIXED ? tcg::kMixed : tcg::kFp64, st, nullptr);
   int h[2] = {0, 0};

@@ -4,9 +4,10 @@
 // block factorizations (src/blocks.jl:94-113, src/directions.jl:46).
 //
 // One launch per 32-wide block column: every thread block factors the
-// 32 x 32 diagonal block in shared memory (redundantly, so no block waits on
-// another), then solves its rows of the panel below against it
-// (L21 = A21 L11^-T) and writes them back together with their bf16 slices;
+// 32 x 32 diagonal block in one warp's registers (redundantly, so no block
+// waits on another) while a second warp solves 32 rows of the panel below
+// against it (L21 = A21 L11^-T), and writes them back together with their
+// bf16 slices;
 // a second launch applies the trailing update A22 -= L21 L21' on the tensor
 // cores (tcgemm.h, lower triangle only).  kFp64: FP64 diagonal blocks and
 // FP64-accurate updates; kMixed: FP32 diagonal blocks and split-precision
@@ -26,12 +27,14 @@ struct Work {
   double* diag = nullptr;  // factored diagonal blocks (NB x NB per block column)
   double* dinv = nullptr;  // their inverses (the triangular solves)
   int64_t nmax = 0;
+  bool solves = true;    // potrf also forms dinv
   int* err = nullptr;    // tensor-core error flag (device)
 };
 
 int64_t work_bytes(int64_t nmax);
-// Bind to device memory of work_bytes(nmax) bytes.
-cudaError_t init(Work* w, void* mem, int64_t nmax, int* err, cudaStream_t st);
+// Bind to device memory of work_bytes(nmax) bytes; `solves` = false for a
+// workspace whose factors are never passed to solve().
+cudaError_t init(Work* w, void* mem, int64_t nmax, int* err, cudaStream_t st, bool solves = true);
 // Lower Cholesky factor of A (n x n, leading dimension lda) in place; the
 // strict upper triangle is not touched.  *info (device) becomes k + 1 for the
 // first pivot k that is not positive and finite, else 0 (LAPACK potrf).

@@ -2001,7 +2001,7 @@ int tc_setup(S* s, bool mixed) {
   void* cwh = tcalloc(chol::work_bytes(std::max(m, 1)));
   s->hinfo_dev = (int*)tcalloc(sizeof(int));
   if (!s->tAm || !s->tBm || !s->tfix || !s->terr || !cwm || !cwh || !s->hinfo_dev) return 1;
-  CU(s, chol::init(&s->cw, cwm, nmax, s->terr, s->st));
+  CU(s, chol::init(&s->cw, cwm, nmax, s->terr, s->st, false));
   CU(s, chol::init(&s->cwH, cwh, std::max(m, 1), s->terr, s->st));
   CU(s, cudaMemsetAsync(s->hinfo_dev, 0, sizeof(int), s->st));
   CU(s, cudaMemsetAsync(s->terr, 0, sizeof(int), s->st));

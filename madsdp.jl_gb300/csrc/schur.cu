@@ -39,13 +39,27 @@ constexpr int kThreads = 256;
 constexpr int kRedBlocks = 128;
 
 // y = Hsym x with Hsym(i, j) = H(max(i, j), min(i, j)) (lower triangle):
-// the j <= i part by rows (coalesced over i), then the j > i part by columns.
-__global__ void k_symv_lower_rows(int m, const double* __restrict__ H, const double* __restrict__ x,
-                                  double* __restrict__ y) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
-    double s = 0.0;
-    for (int j = 0; j <= i; ++j) s = fma(H[i + (int64_t)j * m], x[j], s);
-    y[i] = s;
+// the j <= i part by rows, then the j > i part by columns.  Rows: 32 per
+// block, one per lane (coalesced), the 32 warps take every 32nd column; a
+// thread per row left m = 717 to three blocks (165 us).
+__global__ void __launch_bounds__(1024) k_symv_lower_rows(int m, const double* __restrict__ H,
+                                                         const double* __restrict__ x, double* __restrict__ y) {
+  __shared__ double part[32][33];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i0 = blockIdx.x * 32, i = i0 + lane, jn = min(m, i0 + 32);
+  double s = 0.0;
+  if (i < m) {
+#pragma unroll 4
+    for (int j = w; j < jn; j += 32)
+      if (j <= i) s = fma(H[i + (int64_t)j * m], x[j], s);
+  }
+  part[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && i < m) {
+    double t = 0.0;
+#pragma unroll
+    for (int q = 0; q < 32; ++q) t += part[q][lane];
+    y[i] = t;
   }
 }
 __global__ void k_symv_lower_cols(int m, const double* __restrict__ H, const double* __restrict__ x,
@@ -117,8 +131,7 @@ int factor(msdp_schur* ws, tcg::Mode mode, int32_t* success) {
 // ws->r = b - H x; the largest |r| and |b| through the pinned partials
 bool residual(msdp_schur* ws, double* rn, double* bn) {
   const int m = ws->m;
-  const unsigned g = (unsigned)std::min((m + kThreads - 1) / kThreads, 152 * 8);
-  k_symv_lower_rows<<<g, kThreads, 0, ws->st>>>(m, ws->H, ws->x, ws->r);
+  k_symv_lower_rows<<<(unsigned)((m + 31) / 32), 1024, 0, ws->st>>>(m, ws->H, ws->x, ws->r);
   k_symv_lower_cols<<<(unsigned)std::min(m, 152 * 8), kThreads, 0, ws->st>>>(m, ws->H, ws->x, ws->r);
   k_residual<<<kRedBlocks, kThreads, 0, ws->st>>>(m, ws->b, ws->r, ws->red);
   if (cudaMemcpyAsync(ws->hmax, ws->red, sizeof(double) * 2 * kRedBlocks, cudaMemcpyDeviceToHost, ws->st) !=

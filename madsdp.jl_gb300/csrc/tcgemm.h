@@ -14,7 +14,7 @@
 //     applies (on GB300 it truncates: a sum that is not exact drifts by up
 //     to one unit in the last place per MMA); each chunk's order sums are
 //     converted to a 64-bit fixed-point integer, so chunks add exactly
-//     (integer atomics for split K) and the result does not depend on the
+//     (in registers; integer atomics where K is split over blocks) and the result does not depend on the
 //     order of the chunks;
 //   - the highest orders share one inexact FP32 accumulator whose magnitude
 //     is small enough that its truncation stays below the target accuracy.
@@ -160,13 +160,21 @@ __device__ __forceinline__ void write_slice_pair(double x0, double x1, int e, ui
   for (int t = 0; t < NS; ++t)
     out[t * slice_stride] = __byte_perm(slice_bits(q0[t], t), slice_bits(q1[t], t), 0x7632);
 }
-// Slices of x stored at out[t * slice_stride].
+// Slices of x[0..8) (neighbours along k) stored as 16 bytes per slice at
+// out[t * slice_stride], which is 16-byte aligned.
 template <int NS>
-__device__ __forceinline__ void write_slices(double x, int e, __nv_bfloat16* out, int64_t slice_stride) {
-  int q[NS];
-  slice_ints<NS>(x, e, q);
+__device__ __forceinline__ void write_slices8(const double (&x)[8], int e, __nv_bfloat16* out, int64_t slice_stride) {
+  uint32_t w[NS][4];
 #pragma unroll
-  for (int t = 0; t < NS; ++t) out[t * slice_stride] = __ushort_as_bfloat16((unsigned short)(slice_bits(q[t], t) >> 16));
+  for (int h = 0; h < 4; ++h) {
+    int q0[NS], q1[NS];
+    slice_ints<NS>(x[2 * h], e, q0);
+    slice_ints<NS>(x[2 * h + 1], e, q1);
+#pragma unroll
+    for (int t = 0; t < NS; ++t) w[t][h] = __byte_perm(slice_bits(q0[t], t), slice_bits(q1[t], t), 0x7632);
+  }
+#pragma unroll
+  for (int t = 0; t < NS; ++t) *(uint4*)(out + t * slice_stride) = make_uint4(w[t][0], w[t][1], w[t][2], w[t][3]);
 }
 
 }  // namespace tcg
