@@ -4,33 +4,23 @@
 #include <algorithm>
 #include <mutex>
 
+#include "tridiag.cuh"
+
 namespace chol {
 namespace {
 
 constexpr int NB = 32;    // block column width (= K of the trailing update)
 constexpr int ROWS = 32;  // panel rows per thread block, one per lane
 
-// sqrt(d) and 1/sqrt(d) of a positive finite pivot.  double: an FP32
-// reciprocal square root of the mantissa and one third-order correction
-// (y (1 + e/2 + 3/8 e^2), e = 1 - m y^2), then one Newton correction of the
-// root: about 300 clocks of dependent FP64 instructions where sqrt and a
-// division take about 1000, and the 32 pivots are one serial chain.
+// sqrt(d) and 1/sqrt(d) of a positive finite pivot; in double by the short
+// chain of tridiag.cuh, because the 32 pivots are one serial chain.
 __device__ __forceinline__ void pivot_root(double d, double& root, double& inv) {
-  const long long b = __double_as_longlong(d);
-  const int field = (int)(b >> 52);
-  if (field == 0) {  // subnormal
+  if (__double2hiint(d) < 0x00100000) {  // subnormal
     root = sqrt(d);
     inv = 1.0 / root;
     return;
   }
-  const int k = (field - 1023) >> 1, odd = (field - 1023) & 1;
-  const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | ((long long)(1023 + odd) << 52));  // [1, 4)
-  const double y = (double)rsqrtf((float)m);
-  const double e = fma(-m * y, y, 1.0);
-  const double z = fma(y * e, fma(0.375, e, 0.5), y);
-  inv = __longlong_as_double(__double_as_longlong(z) - ((long long)k << 52));
-  const double s = d * inv;
-  root = fma(fma(-s, s, d) * 0.5, inv, s);
+  fast_root(d, root, inv);
 }
 __device__ __forceinline__ void pivot_root(float d, float& root, float& inv) {
   root = sqrtf(d);

@@ -32,7 +32,7 @@
 #include "../../include/madsdp_gpu.h"
 #include "chol.h"
 #include "eigref.h"
-#include "la.cuh"
+#include "lanczos.h"
 #include "tcgemm.h"
 #include "tridiag.h"
 
@@ -384,116 +384,6 @@ __global__ void k_aff_lin(int ns, double a, double b, const double* x, const dou
     out[i] = (x[i] + a * dx[i]) * (z[i] + b * dz[i]);
 }
 
-// svec of m symmetric n x n matrices (column-major upper triangle,
-// off-diagonal entries times sqrt 2): <B_j, B_k> = svec(B_j) . svec(B_k)
-// One eigenproblem of a step-length evaluation (n x n basis, 4 (n + 1)
-// work entries, result slot).
-struct LanczosJob {
-  int n;
-  const double* Z;
-  double* Q;   // n x n basis
-  double* ws;  // 4 (n + 1)
-  double* out;
-};
-
-// lambda_min of formed symmetric Z (n <= 256), one thread block of 256
-// threads per matrix: row i of each Lanczos vector on thread i, the basis in
-// global memory, full reorthogonalization twice (warp w forms the
-// coefficients of basis vectors w, w + 8, ...), and the stopping rule of the
-// one-warp routine of la.cuh: the smallest Ritz value of the tridiagonal
-// every 4 steps, stop once it moves by at most 64 eps max(1, |theta|) or the
-// Krylov space is exhausted.
-constexpr int kLanczosCta = 256;
-__device__ __forceinline__ double cta_sum256(double x, double* red) {
-  x = warp_sum(x);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = x;
-  __syncthreads();
-  double t = 0.0;
-#pragma unroll
-  for (int w = 0; w < kLanczosCta / 32; ++w) t += red[w];
-  __syncthreads();
-  return t;
-}
-__global__ void __launch_bounds__(kLanczosCta) k_lanczos_cta(const LanczosJob* __restrict__ jobs) {
-  const LanczosJob J = jobs[blockIdx.x];
-  const int n = J.n, i = threadIdx.x, lane = i & 31, wid = i >> 5;
-  __shared__ double qs[kLanczosCta], ws[kLanczosCta], coef[kLanczosCta + 1], red[kLanczosCta / 32];
-  __shared__ double theta_s;
-  double* a = J.ws;
-  double* bb = a + (n + 1);
-  double* Q = J.Q;
-  const bool own = i < n;
-  double v = 0.0;
-  if (own) {
-    uint32_t h = (uint32_t)(i + 1) * 2654435761u;
-    h ^= h >> 15; h *= 2246822519u; h ^= h >> 13;
-    v = (double)(h & 0xffffff) / 16777216.0 - 0.5 + 0.01;
-  }
-  const double nrm = sqrt(cta_sum256(v * v, red));
-  if (own) {
-    v /= nrm;
-    Q[i] = v;
-    qs[i] = v;
-  }
-  if (i == 0) bb[0] = 0.0;
-  __syncthreads();
-  double theta = 0.0, theta_prev = INFINITY, znorm = 0.0;
-  for (int j = 0; j < n; ++j) {
-    double w = 0.0, w1 = 0.0;
-    if (own) {
-      int r = 0;
-      for (; r + 1 < n; r += 2) {
-        w = fma(J.Z[i + (int64_t)r * n], qs[r], w);
-        w1 = fma(J.Z[i + (int64_t)(r + 1) * n], qs[r + 1], w1);
-      }
-      if (r < n) w = fma(J.Z[i + (int64_t)r * n], qs[r], w);
-      w += w1;
-    }
-    const double aj = cta_sum256(own ? qs[i] * w : 0.0, red);
-    const double bj = j > 0 ? bb[j] : 0.0;
-    if (own) w -= aj * qs[i] + (j > 0 ? bj * Q[i + (int64_t)(j - 1) * n] : 0.0);
-    if (i == 0) a[j] = aj;
-    for (int pass = 0; pass < 2; ++pass) {
-      if (own) ws[i] = w;
-      __syncthreads();
-      for (int l = wid; l <= j; l += kLanczosCta / 32) {
-        const double* ql = Q + (int64_t)l * n;
-        double t = 0.0;
-        for (int r = lane; r < n; r += 32) t = fma(ql[r], ws[r], t);
-        t = warp_sum(t);
-        if (lane == 0) coef[l] = t;
-      }
-      __syncthreads();
-      if (own)
-        for (int l = 0; l <= j; ++l) w = fma(-coef[l], Q[i + (int64_t)l * n], w);
-    }
-    const double bn = sqrt(cta_sum256(own ? w * w : 0.0, red));
-    const int k = j + 1;
-    znorm = fmax(znorm, fabs(aj) + bn + fabs(bj));
-    if (i == 0) bb[j + 1] = bn;
-    const bool exhausted = (k == n) || !(bn > 2.220446049250313e-16 * znorm * 4.0);
-    if (exhausted || (k >= 4 && (k % 4) == 0)) {
-      __syncthreads();
-      if (wid == 0) {
-        const double th = warp_tridiag_eigmin<double>(k, a, bb);
-        if (lane == 0) theta_s = th;
-      }
-      __syncthreads();
-      theta = theta_s;
-      const double tolr = 2.220446049250313e-16 * 64.0 * fmax(1.0, fabs(theta));
-      if (exhausted || fabs(theta - theta_prev) <= tolr) break;
-      theta_prev = theta;
-    }
-    if (own) {
-      const double q = w / bn;
-      Q[i + (int64_t)(j + 1) * n] = q;
-      qs[i] = q;
-    }
-    __syncthreads();
-  }
-  if (i == 0) *J.out = theta;
-}
-
 // ---- coordinate-list constraints of one block
 // out[j] (+)= sum_{e in j} v_e X[r_e, c_e]
 __global__ void k_jprod(int m, const int64_t* __restrict__ conptr, const int32_t* __restrict__ row,
@@ -732,8 +622,7 @@ struct msdp_solver {
   int64_t lanczos_calls = 0, lanczos_steps = 0, eigmin_dense = 0;  // lambda_min of blocks above 256
   double *lq = nullptr, *lh = nullptr;  // Lanczos basis (n x (kLanczosMax + 1)) and projections
   double* lzp = nullptr;                 // per-block partial sums of the fused Lanczos step
-  double *lq2 = nullptr, *lw2 = nullptr;  // bases and work of the batched device Lanczos
-  void* ljobs = nullptr;
+  lanczos::Job* ljobs = nullptr;         // eigenproblems of one step length (orders up to 256)
   int* dinfo = nullptr;
   double *partial = nullptr, *slots = nullptr;
   double* hslots = nullptr;
@@ -1555,16 +1444,15 @@ void correction(S* s) {
 }
 
 // ---- Lanczos for lambda_min of a formed symmetric Z (blocks above
-// kLanczosWarpMax, 256).  Full reorthogonalization (twice); the step's scalars
+// lanczos::kMaxOrder, 256).  Full reorthogonalization (twice); the step's scalars
 // stay on the device and the host reads them every kLanczosBatch steps to
 // apply the stopping rule at each step in order: the smallest Ritz value of
 // the first step whose Ritz residual |beta_k s_k| is below 1e-12 ||Z||, or
 // of step n.  Gives up at kLanczosMax (the caller then uses the dense
 // eigensolver).
-constexpr int kLanczosMin = 257;
+constexpr int kLanczosMin = lanczos::kMaxOrder + 1;
 constexpr int kLanczosMax = 320;
 constexpr int kLanczosBatch = 8;
-constexpr int kLanczosWarpMax = kLanczosCta;  // batched one-block device Lanczos up to this size
 
 bool lanczos_eigmin(S* s, int n, const double* Z, double* out) {
   double* Q = s->lq;
@@ -1643,8 +1531,8 @@ void form_congruence(S* s, int n, const double* L, const double* D, double* Z) {
   LAUNCH(s, k_sym, (int64_t)n * n, n, Z);
 }
 
-// slot of lambda_min(Z) for n > kLanczosWarpMax: host-driven Lanczos from
-// kLanczosMin on, else (or when it does not converge) the dense eigensolver
+// slot of lambda_min(Z) for n > lanczos::kMaxOrder: host-driven Lanczos or,
+// when it does not converge, the dense eigensolver
 int eigmin_large(S* s, Blk& b, double* Z) {
   const int n = b.n;
   if (n >= kLanczosMin) {
@@ -1703,8 +1591,8 @@ bool step_lengths(S* s, double* a_out, double* b_out) {
     return backtrack(s, true, a_out) && backtrack(s, false, b_out);
   reset_slots(s);
   std::vector<int> lx, ls;
-  std::vector<LanczosJob> jobs;
-  int64_t qoff = 0, woff = 0;
+  std::vector<lanczos::Job> jobs;
+  int njmax = 0;
   for (auto& b : s->B) {
     const int n = b.n;
     // Z_X ~ Lx^-1 dX Lx^-T in T1, Z_S ~ Ls^-1 dS Ls^-T in T2: NT by the
@@ -1720,12 +1608,11 @@ bool step_lengths(S* s, double* a_out, double* b_out) {
       form_congruence(s, n, b.Lx, b.dX, b.T1);
       form_congruence(s, n, b.Ls, b.dS, b.T2);
     }
-    if (n <= kLanczosWarpMax) {
+    if (n <= lanczos::kMaxOrder) {
+      njmax = std::max(njmax, n);
       for (int side = 0; side < 2; ++side) {
         const int slot = next_slot(s);
-        jobs.push_back(LanczosJob{n, side ? b.T2 : b.T1, s->lq2 + qoff, s->lw2 + woff, s->slots + slot});
-        qoff += (int64_t)n * n;
-        woff += 4 * (int64_t)(n + 1);
+        jobs.push_back(lanczos::Job{n, side ? b.T2 : b.T1, s->slots + slot});
         (side ? ls : lx).push_back(slot);
       }
     } else {
@@ -1734,8 +1621,8 @@ bool step_lengths(S* s, double* a_out, double* b_out) {
     }
   }
   if (!jobs.empty()) {
-    CU(s, cudaMemcpyAsync(s->ljobs, jobs.data(), sizeof(LanczosJob) * jobs.size(), cudaMemcpyHostToDevice, s->st));
-    k_lanczos_cta<<<(unsigned)jobs.size(), kLanczosCta, 0, s->st>>>((const LanczosJob*)s->ljobs);
+    CU(s, cudaMemcpyAsync(s->ljobs, jobs.data(), sizeof(lanczos::Job) * jobs.size(), cudaMemcpyHostToDevice, s->st));
+    CU(s, lanczos::eigmin(s->ljobs, (int)jobs.size(), njmax, s->st));
     s->launches += 1;
   }
   const int rx = s->ns ? reduce(s, RED_MINRATIO, s->ns, s->x, s->dx) : -1;
@@ -2455,17 +2342,9 @@ int msdp_solver_create(msdp_context* ctx, const msdp_problem_desc* d, const msdp
     if (!s->lzp) return bail(MSDP_ERR_OUT_OF_MEMORY);
     if (!s->lq || !s->lh) return bail(MSDP_ERR_OUT_OF_MEMORY);
   }
-  {
-    // batched device Lanczos: two bases (X and S side) per small block
-    int64_t q = 0, w = 0, nj = 0;
-    for (auto& b : s->B)
-      if (b.n <= kLanczosWarpMax) { q += 2 * (int64_t)b.n * b.n; w += 8 * (int64_t)(b.n + 1); nj += 2; }
-    if (nj) {
-      s->lq2 = vec(q);
-      s->lw2 = vec(w);
-      s->ljobs = dalloc<unsigned char>(s, (int64_t)sizeof(LanczosJob) * nj);
-      if (!s->lq2 || !s->lw2 || !s->ljobs) return bail(MSDP_ERR_OUT_OF_MEMORY);
-    }
+  if (s->nb) {
+    s->ljobs = dalloc<lanczos::Job>(s, 2 * s->nb);
+    if (!s->ljobs) return bail(MSDP_ERR_OUT_OF_MEMORY);
   }
   double bn = 0.0, dn = 0.0;
   for (int j = 0; j < m; ++j) bn = std::max(bn, std::fabs(d->b[j]));
@@ -2623,12 +2502,12 @@ int msdp_solver_step_eig(msdp_solver* s, int32_t block, const double* L, const d
   CU(s, cudaMemcpyAsync(b.T2, D, 8 * nn, cudaMemcpyHostToDevice, s->st));
   form_congruence(s, n, b.T3, b.T2, b.T1);
   int slot;
-  LanczosJob job{};  // the copy's source: alive until fetch() below has synchronized
-  if (n <= kLanczosWarpMax) {
+  lanczos::Job job{};  // the copy's source: alive until fetch() below has synchronized
+  if (n <= lanczos::kMaxOrder) {
     slot = next_slot(s);
-    job = LanczosJob{n, b.T1, s->lq2, s->lw2, s->slots + slot};
+    job = lanczos::Job{n, b.T1, s->slots + slot};
     CU(s, cudaMemcpyAsync(s->ljobs, &job, sizeof(job), cudaMemcpyHostToDevice, s->st));
-    k_lanczos_cta<<<1, kLanczosCta, 0, s->st>>>((const LanczosJob*)s->ljobs);
+    CU(s, lanczos::eigmin(s->ljobs, 1, n, s->st));
     s->launches += 1;
   } else {
     slot = eigmin_large(s, b, b.T1);
