@@ -12,8 +12,32 @@ namespace {
 constexpr int NB = 32;    // block column width (= K of the trailing update)
 constexpr int ROWS = 32;  // panel rows per thread block, one per lane
 
-// sqrt(d) and 1/sqrt(d) of a positive finite pivot; in double by the short
-// chain of tridiag.cuh, because the 32 pivots are one serial chain.
+// 1/d of a positive finite pivot.  In double: the reciprocal of d's mantissa
+// in FP32 (both conversions by integer instructions) and one third-order
+// correction y (1 + e + e^2), e = 1 - m y: four dependent FP64 instructions,
+// because the 32 pivots are one serial chain.
+__device__ __forceinline__ double pivot_inv(double d) {
+  const long long b = __double_as_longlong(d);
+  const int field = (int)(b >> 52);
+  if (field < 2 || field > 2044) return 1.0 / d;
+  const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll);  // [1, 2)
+  const float f = __frcp_rn(__int_as_float(0x3F800000 | (int)((b >> 29) & 0x7FFFFF)));    // (0.5, 1]
+  const int fb = __float_as_int(f);
+  const double y = __hiloint2double(((fb >> 3) & 0x0FFFFFFF) + 0x38000000, fb << 29);
+  const double e = fma(-m, y, 1.0);
+  const double z = fma(y, fma(e, e, e), y);
+  return __longlong_as_double(__double_as_longlong(z) - ((long long)(field - 1023) << 52));
+}
+__device__ __forceinline__ float pivot_inv(float d) { return 1.0f / d; }
+// positive and finite
+__device__ __forceinline__ bool pivot_ok(double d) {
+  const long long b = __double_as_longlong(d);
+  return b > 0 && b < 0x7FF0000000000000ll;
+}
+__device__ __forceinline__ bool pivot_ok(float d) {
+  const int b = __float_as_int(d);
+  return b > 0 && b < 0x7F800000;
+}
 __device__ __forceinline__ void pivot_root(double d, double& root, double& inv) {
   if (__double2hiint(d) < 0x00100000) {  // subnormal
     root = sqrt(d);
@@ -32,94 +56,160 @@ __device__ __forceinline__ void pivot_root(float d, float& root, float& inv) {
 // The factored diagonal block goes to `diag` (NB x NB per block column), not
 // to A: other thread blocks of the same launch may still be reading it.
 //
-// Warp 0 factors the diagonal block (row per lane, in registers; every block
-// does so, none waits on another) and publishes its columns in shared memory;
-// warp 1 eliminates the same columns from 32 panel rows, four columns behind
-// (one named barrier per four columns); all four warps then cut the rows into
-// slices.  Bound by the chain of 32 pivots and by warp 0's 500 FP64
-// instructions on its quarter of the SM: 57 us (ncu).  A block-wide factor
-// with three barriers, a square root and a division per column, and 64 rows
-// per block, took 99-123 us.
+// Warps 0-3 eliminate the diagonal block (every thread block does so, none
+// waits on another), warps 4-7 the same columns from 32 panel rows, one step
+// behind; row per lane, column c in warp c % 4 of the group, so each group
+// uses all four quarters of the SM: a FP64 instruction holds its quarter for
+// about 64 clocks.  Column j of the diagonal block is published unscaled (x)
+// and divided by the pivot (x / d): x_c -= x_j (x_cj / d_j) needs the
+// reciprocal but no root, and the whole factor is scaled by 1/sqrt(d) at the
+// end, all pivots at once.  In each step the owner of the next column updates
+// it and publishes its pivot before the rest of the step's work; the warps
+// wait for columns by flags in shared memory (bounded), not for each other.
+// No FP64 comparisons: they cost as much as a multiply-add.
+// Bound by 32 times that chain and the 300 instructions per quarter: 24 us
+// (in stream order).  With the diagonal block in one warp and a root in every
+// step the kernel took 40 us, with four warps and block barriers 29 us; with
+// block-wide steps, roots and divisions and 64 rows per block 99-123 us (ncu).
 template <class T, int NS>
-__global__ void __launch_bounds__(128) k_panel(int n, int k0, double* __restrict__ A, int64_t lda,
+__global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict__ A, int64_t lda,
                                               int* __restrict__ info, __nv_bfloat16* __restrict__ sl,
                                               int32_t* __restrict__ ex, int64_t Rpad, double* __restrict__ diag) {
-  __shared__ T col[NB][NB];       // col[j][r] = L(r, j)
-  __shared__ T rdiag[NB];
+  __shared__ T colx[NB][NB], coll[NB][NB];  // column j: x and x / d, by row
+  __shared__ T yv[NB][ROWS];                // column j of the panel, unscaled
+  __shared__ T piv[NB], rinv[NB], root[NB];
   __shared__ double xs[ROWS][NB + 1];
-  __shared__ int exs[ROWS];
-  __shared__ int bad_s;
+  __shared__ int bad_s, stuck_s;
+  __shared__ volatile int ready_d[NB], ready_y[NB];  // columns published
   if (*(volatile int*)info != 0) return;  // an earlier block column failed
   const int kb = min(NB, n - k0);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = warp & 3;
+  const bool dg = warp < 4;
   // panel rows exist only below a full diagonal block (k0 + NB < n)
   const int64_t R = (int64_t)blockIdx.x * ROWS + lane, i = (int64_t)k0 + NB + R;
   const bool own = kb == NB && i < n;
-  T x[NB];
-  if (warp == 0) {
+  constexpr int Q = NB / 4;
+  T x[Q];  // columns 4 q + w
 #pragma unroll
-    for (int c = 0; c < NB; ++c)
-      x[c] = (lane < kb && c <= lane) ? (T)A[(k0 + lane) + (int64_t)(k0 + c) * lda] : (lane == c ? (T)1 : (T)0);
-    int bad = 0;
-#pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      T d = __shfl_sync(0xffffffffu, x[j], j);
-      if (!(d > (T)0) || !isfinite(d)) {
-        if (!bad) bad = k0 + j + 1;
-        d = (T)1;  // the factor is not used
+  for (int q = 0; q < Q; ++q) {
+    const int c = 4 * q + w;
+    if (dg)
+      x[q] = (lane < kb && c <= lane) ? (T)A[(k0 + lane) + (int64_t)(k0 + c) * lda] : (lane == c ? (T)1 : (T)0);
+    else
+      x[q] = own ? (T)A[i + (int64_t)(k0 + c) * lda] : (T)0;
+  }
+  if (threadIdx.x == 0) bad_s = stuck_s = 0;
+  if (threadIdx.x < NB) ready_d[threadIdx.x] = ready_y[threadIdx.x] = 0;
+  // a flag of a warp of this block (all are resident); the limit is far above
+  // any wait
+  auto wait_for = [&](volatile int* flag) {
+    for (int it = 0; it < (1 << 22); ++it)
+      if (*flag) {
+        __threadfence_block();
+        __syncwarp();
+        return;
       }
-      T root, inv;
-      pivot_root(d, root, inv);
-      const T l = lane == j ? root : x[j] * inv;
-      x[j] = l;
-      col[j][lane] = l;
-      if (lane == j) rdiag[j] = inv;
-      __syncwarp();
-      if ((j & 3) == 3) asm volatile("bar.arrive %0, 64;" ::"r"(1 + (j >> 2)) : "memory");
-#pragma unroll
-      for (int c = j + 1; c < NB; ++c) x[c] -= l * col[j][c];
+    stuck_s = 1;
+  };
+  auto raise = [&](volatile int* flag) {
+    __threadfence_block();
+    __syncwarp();
+    if (lane == 0) *flag = 1;
+  };
+  auto publish = [&](int j, T xj) {
+    colx[j][lane] = xj;
+    T d = __shfl_sync(0xffffffffu, xj, j);
+    if (!pivot_ok(d)) {
+      if (lane == 0 && bad_s == 0) bad_s = k0 + j + 1;  // columns come in order
+      d = (T)1;  // the factor is not used
     }
-    if (lane == 0) bad_s = bad;
-  } else if (warp == 1) {
+    coll[j][lane] = xj * pivot_inv(d);
+    if (lane == 0) piv[j] = d;
+    raise(&ready_d[j]);
+  };
+  __syncthreads();
+  if (dg) {
+    if (w == 0) publish(0, x[0]);
 #pragma unroll
-    for (int c = 0; c < NB; ++c) x[c] = own ? (T)A[i + (int64_t)(k0 + c) * lda] : (T)0;
+    for (int j = 0; j < NB - 1; ++j) {
+      if (w != (j & 3)) wait_for(&ready_d[j]);
+      const T xr = colx[j][lane];
+      const int qn = (j + 1) >> 2;
+      if (w == ((j + 1) & 3)) {
+        x[qn] -= xr * coll[j][j + 1];
+        publish(j + 1, x[qn]);
+      }
 #pragma unroll
-    for (int j = 0; j < NB; ++j) {
-      if ((j & 3) == 0) asm volatile("bar.sync %0, 64;" ::"r"(1 + (j >> 2)) : "memory");
-      x[j] *= rdiag[j];
-#pragma unroll
-      for (int c = j + 1; c < NB; ++c) x[c] -= x[j] * col[j][c];
+      for (int q = 0; q < Q; ++q)
+        if (4 * q + 3 > j + 1 && 4 * q + w > j + 1) x[q] -= xr * coll[j][4 * q + w];
     }
-    int mx = 0;
+  } else {
 #pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      xs[lane][c] = (double)x[c];
-      mx = max(mx, tcg::exp_field((double)x[c]));
+    for (int p = 0; p < NB; ++p) {
+      T yr = (T)0;
+      if (p > 0) {
+        wait_for(&ready_d[p - 1]);
+        if (w != ((p - 1) & 3)) wait_for(&ready_y[p - 1]);
+        yr = yv[p - 1][lane];
+      }
+      const int qp = p >> 2;
+      if (w == (p & 3)) {
+        if (p > 0) x[qp] -= yr * coll[p - 1][p];
+        yv[p][lane] = x[qp];
+        raise(&ready_y[p]);
+      }
+      if (p > 0) {
+#pragma unroll
+        for (int q = 0; q < Q; ++q)
+          if (4 * q + 3 > p && 4 * q + w > p) x[q] -= yr * coll[p - 1][4 * q + w];
+      }
     }
-    exs[lane] = tcg::row_exp(mx);
   }
   __syncthreads();
-  if (bad_s) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(info, 0, bad_s);
+  if (bad_s || stuck_s) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(info, 0, bad_s ? bad_s : k0 + 1);
     return;
   }
-  if (warp == 0 && blockIdx.x == 0) {
-#pragma unroll
-    for (int c = 0; c < NB; ++c) diag[((int64_t)k0 + c) * NB + lane] = lane >= c ? (double)x[c] : 0.0;
+  if (warp == 0) {
+    T rt, ri;
+    pivot_root(piv[lane], rt, ri);
+    root[lane] = rt;
+    rinv[lane] = ri;
   }
-  if (warp == 1 && own) {
+  __syncthreads();
 #pragma unroll
-    for (int c = 0; c < NB; ++c) A[i + (int64_t)(k0 + c) * lda] = (double)x[c];
-    ex[R] = exs[lane];
+  for (int q = 0; q < Q; ++q) {
+    const int c = 4 * q + w;
+    if (dg) {
+      if (blockIdx.x == 0)
+        diag[((int64_t)k0 + c) * NB + lane] =
+            lane > c ? (double)(colx[c][lane] * rinv[c]) : (lane == c ? (double)root[c] : 0.0);
+    } else {
+      const double v = (double)(x[q] * rinv[c]);
+      xs[lane][c] = v;
+      if (own) A[i + (int64_t)(k0 + c) * lda] = v;
+    }
   }
-  // slices: eight columns of one row per thread
-  const int row = threadIdx.x >> 2, seg = (threadIdx.x & 3) * 8;
-  const int64_t Rr = (int64_t)blockIdx.x * ROWS + row;
-  if (kb == NB && k0 + NB + Rr < n) {
+  __syncthreads();
+  // row exponents, then slices: eight columns of one row per thread (four
+  // neighbouring lanes share a row)
+  if (threadIdx.x < 128) {
+    const int row = threadIdx.x >> 2, seg = (threadIdx.x & 3) * 8;
+    const int64_t Rr = (int64_t)blockIdx.x * ROWS + row;
     double v[8];
+    int mx = 0;
 #pragma unroll
-    for (int c = 0; c < 8; ++c) v[c] = xs[row][seg + c];
-    tcg::write_slices8<NS>(v, exs[row], sl + Rr * NB + seg, Rpad * NB);
+    for (int c = 0; c < 8; ++c) {
+      v[c] = xs[row][seg + c];
+      mx = max(mx, tcg::exp_field(v[c]));
+    }
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 1));
+    mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, 2));
+    if (kb == NB && k0 + NB + Rr < n) {
+      const int e = tcg::row_exp(mx);
+      if (seg == 0) ex[Rr] = e;
+      tcg::write_slices8<NS>(v, e, sl + Rr * NB + seg, Rpad * NB);
+    }
   }
 }
 
@@ -507,9 +597,9 @@ cudaError_t potrf(Work& w, int n, double* A, int64_t lda, int* info, tcg::Mode m
     const int64_t nr = n - k0 - kb;
     const unsigned grid = (unsigned)std::max<int64_t>(1, (nr + ROWS - 1) / ROWS);
     if (mode == tcg::kMixed)
-      k_panel<float, 3><<<grid, 128, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
+      k_panel<float, 3><<<grid, 256, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
     else
-      k_panel<double, 7><<<grid, 128, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
+      k_panel<double, 7><<<grid, 256, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;
