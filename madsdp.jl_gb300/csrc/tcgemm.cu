@@ -42,6 +42,9 @@ struct Pairs {
 struct Args {
   int64_t M, N, rpad_a, rpad_b, ldc, ldfix;
   int32_t tiles_n, lower, kblocks, chunk_kb, block_kb, U;
+  // alpha: 0: 1, 1: -1, 2: other; beta: 0: 0, 1: 1, 2: other.  As integers: a
+  // comparison of doubles holds the FP64 unit as long as a multiply-add
+  int32_t alpha_kind, beta_kind;
   double alpha, beta;
   const int32_t* exa;
   const int32_t* exb;
@@ -185,7 +188,8 @@ __device__ __forceinline__ long long float_to_fixed(float v, int U) {
 // latency of one load, one MMA group and the write-back.  A block per chunk,
 // with 64-bit conversions, an integer atomic per entry and chunk and one load
 // of C at a time, took 2.9 ms for the whole 1999 x 1999 x 5051 lower product
-// (msdp_tc_gemm) against 1.05 ms with this and the slicing below.
+// (msdp_tc_gemm) against 0.94 ms with this and the slicing below; a single
+// 128 x 64 x 32 tile takes 12.9 us.
 template <int NS, int NG, int BN, int NST>
 __global__ void __launch_bounds__(kThreads, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap ma, const __grid_constant__ CUtensorMap mb, const Args a) {
@@ -319,10 +323,21 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int c0 = (warp >> 2) * HALF;
     const int64_t row = (int64_t)tm * BM + (warp & 3) * 32 + lane;
     const bool row_ok = row < a.M;
+    const float scaleU = __int_as_float((127 + a.U) << 23);
     const uint32_t tw = tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
     long long acc[HALF];
 #pragma unroll
     for (int j = 0; j < HALF; ++j) acc[j] = 0;
+    // narrow tiles: the old C is loaded while the MMAs run
+    constexpr bool kEarly = HALF <= 32;
+    double early[kEarly ? HALF : 1];
+    if (kEarly && !a.fix && a.beta_kind) {
+#pragma unroll
+      for (int j = 0; j < (kEarly ? HALF : 0); ++j) {
+        const int64_t col = (int64_t)tn * BN + c0 + j;
+        early[j] = (row_ok && col < a.N && !(a.lower && row < col)) ? a.C[row + col * a.ldc] : 0.0;
+      }
+    }
     bool ok = true;
     for (int c = 0; c < nch; ++c) {
       ok = mbar_wait(done, c & 1, deadline) && !*abort_flag;
@@ -340,16 +355,20 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int g = 0; g < NG; ++g) tmem_ld8(tw + (uint32_t)(g * BN + sg * 8), v[g]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-        for (int g = 0; g < NG; ++g) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            if (g < NG - 1) {
-              // an integer below 2^24 times 2^-8g (U >= 24 covers g <= 3)
-              const int q = __float2int_rn(__uint_as_float(v[g][j]) * (float)(1 << (8 * g)));
-              acc[sg * 8 + j] += (long long)q << (a.U - 8 * g);
-            } else {
-              acc[sg * 8 + j] += float_to_fixed(__uint_as_float(v[g][j]), a.U);
-            }
+        for (int j = 0; j < 8; ++j) {
+          if constexpr (NG == 5) {
+            // orders 0-3: integers below 2^24 times 2^-8g, gathered in units
+            // of 2^-24 by wide multiply-adds; the rest below 2^-7 in units of
+            // 2^-U, U <= 38
+            long long tsum = (long long)__float2int_rn(__uint_as_float(v[0][j])) * (1 << 24);
+            tsum += (long long)__float2int_rn(__uint_as_float(v[1][j]) * 0x1p8f) * (1 << 16);
+            tsum += (long long)__float2int_rn(__uint_as_float(v[2][j]) * 0x1p16f) * (1 << 8);
+            tsum += (long long)__float2int_rn(__uint_as_float(v[3][j]) * 0x1p24f);
+            acc[sg * 8 + j] += (tsum << (a.U - 24)) + (long long)__float2int_rn(__uint_as_float(v[4][j]) * scaleU);
+          } else {
+            // an exact integer and a remainder below 2^18
+            acc[sg * 8 + j] += (long long)__float2int_rn(__uint_as_float(v[0][j])) << a.U;
+            acc[sg * 8 + j] += float_to_fixed(__uint_as_float(v[NG - 1][j]), a.U);
           }
         }
       }
@@ -373,21 +392,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         // eight independent loads of C before the first store
         double old[8];
-        if (a.beta != 0.0) {
+        if (a.beta_kind) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) {
             const int64_t col = col0 + j;
-            old[j] = (col < a.N && !(a.lower && row < col)) ? a.C[row + col * a.ldc] : 0.0;
+            if (kEarly) old[j] = early[kEarly ? sg * 8 + j : 0];
+            else old[j] = (col < a.N && !(a.lower && row < col)) ? a.C[row + col * a.ldc] : 0.0;
           }
         }
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int64_t col = col0 + j;
           double d = fix_to_double(acc[sg * 8 + j], ea + exb_s[c0 + sg * 8 + j]);
-          if (a.alpha == -1.0) d = -d;
-          else if (a.alpha != 1.0) d = a.alpha * d;
-          if (a.beta == 1.0) d = old[j] + d;
-          else if (a.beta != 0.0) d = d + a.beta * old[j];
+          if (a.alpha_kind == 1) d = -d;
+          else if (a.alpha_kind == 2) d = a.alpha * d;
+          if (a.beta_kind == 1) d = old[j] + d;
+          else if (a.beta_kind == 2) d = d + a.beta * old[j];
           if (col < a.N && !(a.lower && row < col)) a.C[row + col * a.ldc] = d;
         }
       }
@@ -403,16 +423,18 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // C = alpha * fix * 2^(ea + eb - U - 14) + beta * C
 __global__ void k_finish(int64_t M, int64_t N, const long long* __restrict__ fix, int64_t ldfix,
-                         const int32_t* __restrict__ exa, const int32_t* __restrict__ exb, int U, double alpha,
-                         double beta, double* C, int64_t ldc, int lower) {
+                         const int32_t* __restrict__ exa, const int32_t* __restrict__ exb, int U, int alpha_kind,
+                         double alpha, int beta_kind, double beta, double* C, int64_t ldc, int lower) {
   const int64_t total = M * N;
   for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
        idx += (int64_t)gridDim.x * blockDim.x) {
     const int64_t c = idx / M, r = idx - c * M;
     if (lower && r < c) continue;
-    const double v = alpha * fix_to_double(fix[r + c * ldfix], exa[r] + exb[c] - U - 14);
+    double v = fix_to_double(fix[r + c * ldfix], exa[r] + exb[c] - U - 14);
+    if (alpha_kind == 1) v = -v;
+    else if (alpha_kind == 2) v = alpha * v;
     double* o = C + r + c * ldc;
-    *o = beta == 0.0 ? v : v + beta * *o;
+    *o = beta_kind == 0 ? v : beta_kind == 1 ? v + *o : v + beta * *o;
   }
 }
 
@@ -676,13 +698,15 @@ cudaError_t gemm(const Sliced& A, const Sliced& B, Mode mode, const Out& o, cuda
   a.block_kb = (nchunks + pl.splits - 1) / pl.splits * a.chunk_kb;
   int lg = 0;
   while (((int64_t)1 << lg) < std::max<int64_t>(A.K, 2)) ++lg;
-  a.U = std::max(24, std::min(46, 47 - lg));
+  a.U = std::max(24, std::min(mode == kMixed ? 46 : 38, 47 - lg));
   a.exa = A.ex;
   a.exb = B.ex;
   a.C = o.C;
   a.ldc = o.ldc;
   a.alpha = o.alpha;
   a.beta = o.beta;
+  a.alpha_kind = o.alpha == 1.0 ? 0 : o.alpha == -1.0 ? 1 : 2;
+  a.beta_kind = o.beta == 0.0 ? 0 : o.beta == 1.0 ? 1 : 2;
   a.fix = pl.splits > 1 ? (unsigned long long*)o.fix : nullptr;
   a.ldfix = o.ldfix;
   a.err = o.err;
@@ -706,7 +730,7 @@ cudaError_t gemm(const Sliced& A, const Sliced& B, Mode mode, const Out& o, cuda
   if (a.fix) {
     const int64_t total = M * N;
     const unsigned grid = (unsigned)std::min<int64_t>((total + 255) / 256, 152 * 32);
-    k_finish<<<grid, 256, 0, st>>>(M, N, o.fix, o.ldfix, A.ex, B.ex, a.U, o.alpha, o.beta, o.C, o.ldc, a.lower);
+    k_finish<<<grid, 256, 0, st>>>(M, N, o.fix, o.ldfix, A.ex, B.ex, a.U, a.alpha_kind, o.alpha, a.beta_kind, o.beta, o.C, o.ldc, a.lower);
     if (launches) *launches += 1;
     e = cudaGetLastError();
   }
