@@ -45,13 +45,14 @@ __device__ __forceinline__ void store_remote(const double* p, int rank, double v
 // every 4 steps, until it moves by at most 64 eps max(1, |theta|) or the
 // Krylov space is exhausted.  The Ritz value is looked at in FP32 first; the
 // FP64 values of this check and of the one before are formed only when the
-// FP32 ones differ by less than 3e-5 of the norm (a move of 64 eps cannot
-// hide behind FP32's error).
+// FP32 ones differ by less than 3e-6 of the norm: they are within 5e-7 of it
+// (the rounding of the tridiagonal and of the Sturm sequence, 4 eps, and the
+// bracket), so a move of 64 eps cannot be missed.
 //
 // One block of 256 threads per matrix with Z and the basis in global memory
 // and divisions in the Sturm counts took 1.41 ms a launch at n = 100 (two
-// matrices, about 28 steps); the max-cut solve of that order went from 76.4 to
-// 53.7 ms, a launch over blocks of 120, 60, 30 and 30 from 4.96 to 1.51 ms.
+// matrices, about 28 steps); this takes 0.39 ms, and 1.08 ms for a launch over
+// blocks of 120, 60, 30 and 30 (4.96 ms before).
 __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jobs) {
   int cs, rank;
   asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cs));
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
   double* xch = (double*)(sbf + n + 2);         // [2][cs][n + 2], clusters of more than one block
   __shared__ TridiagShared tsh;
   __shared__ double red[8];
+  __shared__ int state, stop;
 
   auto cluster_sync = [&] {
     if (cs == 1) __syncthreads();
@@ -111,6 +113,7 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
   if (t == 0) be[0] = 0.0;
   cluster_sync();
 
+  const int U = nr > 64 ? 1 : nr > 32 ? 2 : 4;  // parts of an update: four warps in all
   // parts of a sum split over threads: a power of two, at most 16
   auto parts_of = [](int outputs) {
     int c = 16;
@@ -157,7 +160,6 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
     }
     // ---- two Gram-Schmidt passes against q_0 .. q_j
     const int L = j + 1;
-    double aj = 0.0;
     bool large = false;
     for (int pass = 0; pass < 2; ++pass) {
       const int LL = L + pass;  // the second pass's last output is w'w
@@ -190,13 +192,22 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
       }
       if (t < LL) coef[t] = s;
       __syncthreads();
-      if (pass == 0) aj = coef[j];
-      if (t < nr) {
-        const double* q = Qs + t * ldq;
+      if (t < nr * U) {
+        const int i = t % nr, u = t / nr, la = u * L / U, lb = (u + 1) * L / U;
+        const double* q = Qs + i * ldq;
+        double s1 = 0.0;
 #pragma unroll 4
-        for (int l = 0; l < L; ++l) w = fma(-coef[l], q[l], w);
+        for (int l = la; l < lb; ++l) s1 = fma(-coef[l], q[l], s1);
+        part[t] = s1;
+      }
+      __syncthreads();
+      if (t < nr) {
+        double s1 = part[t];
+        for (int u = 1; u < U; ++u) s1 += part[u * nr + t];
+        w += s1;
         if (pass == 0) ws[t] = w;
       }
+      if (pass == 0 && t == 0) al[j] = coef[j];
       if (pass == 1) {
         // a coefficient above 2^-30 |w'| changes the norm
         const int en = (__double2hiint(coef[L]) >> 20) - 1023;
@@ -204,53 +215,63 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
         large = __syncthreads_or(2 * ec > en - 60);
       }
     }
-    double bn2 = coef[L];
-    // infinite or NaN entries: no eigenvalue
-    if ((__double2hiint(bn2) & 0x7ff00000) == 0x7ff00000 || (__double2hiint(aj) & 0x7ff00000) == 0x7ff00000) {
+    // ---- the norm (the warps that need it), the new basis vector, the state
+    // of the iteration (thread 0)
+    const int k = j + 1;
+    if (warp * 32 < nr || warp == 0) {
+      double bn2 = coef[L];
+      if (large)
+        for (int l = 0; l < L; ++l) bn2 = fma(-coef[l], coef[l], bn2);
+      const int field = __double2hiint(bn2) >> 20;  // 0x7ff: infinite or NaN; below 27: 1e-300 or negative
+      double bn = 0.0, binv = 0.0;
+      if (field > 27 && field < 0x7ff) fast_root(bn2, bn, binv);
+      if (t < nr && k < n) {
+        const double q = w * binv;
+        Qs[t * ldq + k] = q;
+        if (cs == 1) qs[t] = q;
+        else
+          for (int r = 0; r < cs; ++r) store_remote(qs + r0 + t, r, q);
+      }
+      if (t == 0) {
+        const double aj = al[j], bj = j > 0 ? be[j] : 0.0;
+        znorm = fmax(znorm, fabs(aj) + bn + fabs(bj));
+        be[k] = bn;
+        const bool bad = field == 0x7ff || (__double2hiint(aj) & 0x7ff00000) == 0x7ff00000;
+        state = bad ? 2 : !(bn > 4.0 * kEps * znorm) ? 1 : 0;
+      }
+    }
+    cluster_sync();
+    if (state == 2) {  // infinite or NaN entries: no eigenvalue
       theta = nan("");
       break;
     }
-    if (large)
-      for (int l = 0; l < L; ++l) bn2 = fma(-coef[l], coef[l], bn2);
-    double bn = 0.0, binv = 0.0;
-    if (bn2 > 1e-300) fast_root(bn2, bn, binv);
-    const int k = j + 1;
-    const double bj = j > 0 ? be[j] : 0.0;
-    znorm = fmax(znorm, fabs(aj) + bn + fabs(bj));
-    const bool exhausted = k == n || !(bn > 4.0 * kEps * znorm);
-    if (t == 0) {
-      al[j] = aj;
-      be[j + 1] = bn;
-    }
+    const bool exhausted = k == n || state == 1;
     if (exhausted || (k >= 4 && (k & 3) == 0)) {
-      __syncthreads();
       const int e = tridiag_scale(k, al, be, sa, sb, saf, sbf, tsh);
       const float th32 = tridiag_min32(k, saf, sbf, tsh);  // in units of 2^e
       const float here = ldexpf(th32, e);
-      bool stop = exhausted;
       if (exhausted) {
         theta = tridiag_min64(k, sa, sb, th32, e, tsh);
-      } else if (fabsf(here - theta32_prev) <= 3e-5f * ldexpf(1.0f, e)) {
+        break;
+      }
+      if (fabsf(here - theta32_prev) <= 3e-6f * ldexpf(1.0f, e)) {
         theta = tridiag_min64(k, sa, sb, th32, e, tsh);
-        if (!have_prev) theta_prev = tridiag_min64(k - 4, sa, sb, ldexpf(theta32_prev, -e), e, tsh);
-        stop = fabs(theta - theta_prev) <= 64.0 * kEps * fmax(1.0, fabs(theta));
+        if (!have_prev) {
+          const double th = theta;
+          __syncthreads();
+          theta_prev = tridiag_min64(k - 4, sa, sb, ldexpf(theta32_prev, -e), e, tsh);
+          theta = th;
+        }
+        if (t == 0) stop = fabs(theta - theta_prev) <= 64.0 * kEps * fmax(1.0, fabs(theta));
+        __syncthreads();
+        if (stop) break;
         theta_prev = theta;
         have_prev = true;
       } else {
         have_prev = false;
       }
-      if (stop) break;
       theta32_prev = here;
     }
-    // ---- the new basis vector
-    if (t < nr) {
-      const double q = w * binv;
-      Qs[t * ldq + j + 1] = q;
-      if (cs == 1) qs[t] = q;
-      else
-        for (int r = 0; r < cs; ++r) store_remote(qs + r0 + t, r, q);
-    }
-    cluster_sync();
   }
   if (rank == 0 && t == 0) *J.out = theta;
   // no block leaves while another may still reach its shared memory
@@ -268,10 +289,11 @@ cudaError_t eigmin(const Job* jobs, int count, int nmax, cudaStream_t st) {
     attr = cudaFuncSetAttribute(k_lanczos, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
   });
   if (attr != cudaSuccess) return attr;
-  // the smallest cluster whose blocks hold their rows of Z and of a full
-  // basis: one block up to n = 115, 2 up to 160, 4 up to 220, 8 up to 256
+  // 32 rows a block: the FP64 units of one SM are the bound below (at n = 100
+  // a step takes 18000 clocks in one block, most of it their work, and an
+  // exchange in the cluster 1200); a full basis and the rows of Z fit at 256
   int cs = 1;
-  while (cs < 8 && smem_doubles(nmax, cs) * 8 > kSmemMax) cs *= 2;
+  while (cs < 8 && (nmax + cs - 1) / cs > 32) cs *= 2;
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)(count * cs));
   cfg.blockDim = dim3(kThreads);

@@ -78,8 +78,9 @@ __device__ __forceinline__ bool sturm_above32(int k, const float* a, const float
 }
 
 struct TridiagShared {
-  int e, first[4];
-  float lo, hi;
+  double theta;
+  int e, first[2][4];
+  float lo;
 };
 
 // ---- block-wide forms: called by every thread of the block (at least 128)
@@ -136,35 +137,43 @@ __device__ inline float tridiag_min32(int k, const float* saf, const float* sbf,
   return sh.lo;
 }
 
-// The same in FP64 around an FP32 value: rounds of 128 points on four warps
-// (one per quarter of the SM) until the bracket is 2 eps |theta| or a quarter
-// eps of the norm wide; the whole interval when the FP32 value misses.
-// Returns theta 2^e.
+// The same in FP64 around an FP32 value: rounds of 128 points on the first
+// four warps (one per quarter of the SM) until the bracket is 2 eps |theta| or
+// a quarter eps of the norm wide; the whole interval when the FP32 value
+// misses.  Returns theta 2^e.  The other warps only wait: FP64 work on them
+// would hold up the four.
 __device__ inline double tridiag_min64(int k, const double* sa, const double* sb, float th32, int e, TridiagShared& sh) {
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
   const double eps = 2.220446049250313e-16;
-  for (int attempt = 0;; ++attempt) {
-    const double lo0 = attempt ? -1.0 : fmax(-1.0, (double)th32 - 8e-6), hi0 = attempt ? 1.0 : fmin(1.0, (double)th32 + 8e-6);
-    double lo = lo0, hi = hi0;
-    for (int it = 0; it < 16; ++it) {
-      if (hi - lo <= fmax(2.0 * eps * fmax(fabs(lo), fabs(hi)), 0.25 * eps)) break;
-      const double h = (hi - lo) * (1.0 / 129.0);
-      if (warp < 4) {
-        const unsigned above = __ballot_sync(0xffffffffu, sturm_above(k, sa, sb, lo + h * (double)(t + 1)));
-        if (lane == 0) sh.first[warp] = above == 0xffffffffu ? 32 : __ffs(~above) - 1;
-      }
-      __syncthreads();
-      int first = 128;
+  if (warp < 4) {
+    for (int attempt = 0;; ++attempt) {
+      const double lo0 = attempt ? -1.0 : fmax(-1.0, (double)th32 - 8e-6), hi0 = attempt ? 1.0 : fmin(1.0, (double)th32 + 8e-6);
+      double lo = lo0, hi = hi0;
+      bool lo_moved = false, hi_moved = false;
+      for (int it = 0; it < 16; ++it) {
+        if (hi - lo <= fmax(2.0 * eps * fmax(fabs(lo), fabs(hi)), 0.25 * eps)) break;
+        const double h = (hi - lo) * (1.0 / 129.0);
+        const unsigned above = __ballot_sync(0xffffffffu, sturm_above(k, sa, sb, fma(h, (double)(t + 1), lo)));
+        if (lane == 0) sh.first[it & 1][warp] = above == 0xffffffffu ? 32 : __ffs(~above) - 1;
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        int first = 128;
 #pragma unroll
-      for (int w = 3; w >= 0; --w)
-        if (sh.first[w] < 32) first = w * 32 + sh.first[w];
-      __syncthreads();
-      const double l = lo;
-      lo = l + h * (double)first;
-      if (first < 128) hi = l + h * (double)(first + 1);
+        for (int w = 3; w >= 0; --w)
+          if (sh.first[it & 1][w] < 32) first = w * 32 + sh.first[it & 1][w];
+        const double l = lo;
+        lo = fma(h, (double)first, l);
+        lo_moved = lo_moved || first > 0;
+        if (first < 128) {
+          hi = fma(h, (double)(first + 1), l);
+          hi_moved = true;
+        }
+      }
+      // an end that never moved was not tested
+      if (attempt == 0 && ((!lo_moved && lo0 > -1.0) || (!hi_moved && hi0 < 1.0))) continue;
+      if (t == 0) sh.theta = exp_add(0.5 * (lo + hi), e);
+      break;
     }
-    if (attempt == 0 && ((lo == lo0 && lo0 > -1.0) || (hi == hi0 && hi0 < 1.0))) continue;
-    const double mid = 0.5 * (lo + hi);
-    return exp_add(mid, e);
   }
+  __syncthreads();
+  return sh.theta;
 }
