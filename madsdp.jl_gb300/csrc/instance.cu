@@ -803,39 +803,61 @@ tcg::Source op_rows(const double* Mp, int64_t ld, bool trans, int64_t rows, int6
 // (row exponents and slices of both operands, then the product) cost more
 // time than the arithmetic.
 constexpr int kSmallGemm = 128;
-constexpr int kSgTile = 16;
+constexpr int kSgTile = 8;   // output tile
+constexpr int kSgSplit = 4;  // k parts summed by separate threads
+constexpr int kSgK = 32;     // k per stage
 
-// C = alpha op(A) op(B) + beta C on CUDA cores (FP64), 16 x 16 output tiles
-// with both operand tiles staged in shared memory; lower: only i >= j.
-__global__ void __launch_bounds__(kSgTile * kSgTile)
+// C = alpha op(A) op(B) + beta C on CUDA cores (FP64): 8 x 8 output tiles, so
+// that n = 100 gives 169 blocks for the 152 SMs, and within a block four
+// threads per entry, each with every fourth k; lower: only i >= j.  Bound by
+// the FP64 units (64 clocks per warp instruction and SM quarter): 16 x 16
+// tiles kept 49 SMs busy, 12 us at n = 100.
+__global__ void __launch_bounds__(kSgTile * kSgTile * kSgSplit)
     k_dgemm_small(int m, int n, int k, int ta, int tb, double alpha, const double* __restrict__ A, int lda,
                   const double* __restrict__ B, int ldb, double beta, double* C, int ldc, int lower) {
-  __shared__ double As[kSgTile][kSgTile + 1], Bs[kSgTile][kSgTile + 1];
-  const int tx = threadIdx.x, ty = threadIdx.y;
-  const int i = blockIdx.x * kSgTile + tx, j = blockIdx.y * kSgTile + ty;
+  constexpr int kThr = kSgTile * kSgTile * kSgSplit;
+  __shared__ double As[kSgK][kSgTile + 1], Bs[kSgK][kSgTile + 1], part[kSgSplit][kSgTile * kSgTile];
+  const int t = threadIdx.x, e = t & (kSgTile * kSgTile - 1), g = t / (kSgTile * kSgTile);
+  const int tx = e & (kSgTile - 1), ty = e / kSgTile;
+  const int i0 = blockIdx.x * kSgTile, j0 = blockIdx.y * kSgTile;
+  if (lower && j0 > i0 + kSgTile - 1) return;
   double acc = 0.0;
-  for (int k0 = 0; k0 < k; k0 += kSgTile) {
-    // As[r][c] = op(A)(blockrow + r, k0 + c), Bs[r][c] = op(B)(k0 + r, blockcol + c)
+  for (int k0 = 0; k0 < k; k0 += kSgK) {
+    // As[c][r] = op(A)(i0 + r, k0 + c), Bs[c][r] = op(B)(k0 + c, j0 + r);
+    // neighbouring threads along the direction that is contiguous in memory
+    static_assert(kThr == kSgTile * kSgK, "one entry of each operand per thread");
     {
-      const int r = tx, c = ty, gi = blockIdx.x * kSgTile + r, gk = k0 + c;
-      As[r][c] = (gi < m && gk < k) ? (ta ? A[gk + (int64_t)gi * lda] : A[gi + (int64_t)gk * lda]) : 0.0;
-      const int gk2 = k0 + tx, gj = blockIdx.y * kSgTile + ty;
-      Bs[tx][ty] = (gk2 < k && gj < n) ? (tb ? B[gj + (int64_t)gk2 * ldb] : B[gk2 + (int64_t)gj * ldb]) : 0.0;
+      const int r = ta ? t / kSgK : t % kSgTile, c = ta ? t % kSgK : t / kSgTile;
+      const int gi = i0 + r, gk = k0 + c;
+      As[c][r] = (gi < m && gk < k) ? (ta ? A[gk + (int64_t)gi * lda] : A[gi + (int64_t)gk * lda]) : 0.0;
+    }
+    {
+      const int r = tb ? t % kSgTile : t / kSgK, c = tb ? t / kSgTile : t % kSgK;
+      const int gj = j0 + r, gk = k0 + c;
+      Bs[c][r] = (gk < k && gj < n) ? (tb ? B[gj + (int64_t)gk * ldb] : B[gk + (int64_t)gj * ldb]) : 0.0;
     }
     __syncthreads();
 #pragma unroll
-    for (int l = 0; l < kSgTile; ++l) acc = fma(As[tx][l], Bs[l][ty], acc);
+    for (int l = 0; l < kSgK / kSgSplit; ++l) {
+      const int c = l * kSgSplit + g;
+      if (k0 + c < k) acc = fma(As[c][tx], Bs[c][ty], acc);
+    }
     __syncthreads();
   }
-  if (i < m && j < n && (!lower || i >= j)) {
+  part[g][e] = acc;
+  __syncthreads();
+  const int i = i0 + tx, j = j0 + ty;
+  if (g == 0 && i < m && j < n && (!lower || i >= j)) {
+    const double v = (part[0][e] + part[1][e]) + (part[2][e] + part[3][e]);
     double* c = C + i + (int64_t)j * ldc;
-    *c = beta == 0.0 ? alpha * acc : alpha * acc + beta * *c;
+    *c = beta == 0.0 ? alpha * v : alpha * v + beta * *c;
   }
 }
 void small_gemm(S* s, int ta, int tb, int m, int n, int k, double alpha, const double* A, int lda, const double* B,
                 int ldb, double beta, double* C, int ldc, bool lower) {
-  const dim3 block(kSgTile, kSgTile), grid((m + kSgTile - 1) / kSgTile, (n + kSgTile - 1) / kSgTile);
-  k_dgemm_small<<<grid, block, 0, s->st>>>(m, n, k, ta, tb, alpha, A, lda, B, ldb, beta, C, ldc, lower ? 1 : 0);
+  const dim3 grid((m + kSgTile - 1) / kSgTile, (n + kSgTile - 1) / kSgTile);
+  k_dgemm_small<<<grid, kSgTile * kSgTile * kSgSplit, 0, s->st>>>(m, n, k, ta, tb, alpha, A, lda, B, ldb, beta, C, ldc,
+                                                                  lower ? 1 : 0);
   s->launches += 1;
 }
 
