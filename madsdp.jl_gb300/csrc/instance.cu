@@ -219,112 +219,6 @@ __global__ void k_div_rows(int n, double* A, const double* __restrict__ sc) {
     A[idx] /= sc[idx % n];
 }
 
-// ---- Lanczos steps with the scalars kept on the device
-// out[i] -= sum_j A[i + j lda] v[j]: 32 rows per block of 32 x 32 threads,
-// thread (r, g) sums columns g, g + 32, ... (coalesced over r); the 32
-// partial sums of a row are added in a fixed order
-__global__ void __launch_bounds__(1024) k_gemv_sub(int64_t rows, int cols, const double* __restrict__ A, int64_t lda,
-                                                  const double* __restrict__ v, double* __restrict__ out) {
-  __shared__ double part[32][33];
-  const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int64_t i = (int64_t)blockIdx.x * 32 + r;
-  double s = 0.0;
-  if (i < rows)
-    for (int j = g; j < cols; j += 32) s = fma(A[i + j * lda], v[j], s);
-  part[g][r] = s;
-  __syncthreads();
-  if (g == 0 && i < rows) {
-    double t = 0.0;
-    for (int q = 0; q < 32; ++q) t += part[q][r];
-    out[i] -= t;
-  }
-}
-// ---- one Lanczos step in fewer launches: each reduction leaves per-block
-// partial sums, and the kernel that needs the total sums them itself in a
-// fixed order (every block the same way), so results do not depend on
-// timing and no separate reduction launch is needed.
-__device__ __forceinline__ double block_sum256(double v, double* red) {
-  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int w = 0; w < kThreads / 32; ++w) t += red[w];
-  __syncthreads();
-  return t;
-}
-// sum of np partials, identical in every block
-__device__ __forceinline__ double sum_partials(const double* __restrict__ part, int np, double* red) {
-  double v = 0.0;
-  for (int i = threadIdx.x; i < np; i += blockDim.x) v += part[i];
-  return block_sum256(v, red);
-}
-// w = Z q (Z symmetric: column dots, one block per column as k_gemv_t) and
-// part[b] = sum of q_j w_j over the columns of block b
-__global__ void __launch_bounds__(kThreads) k_lz_matvec(int64_t n, const double* __restrict__ Z,
-                                                        const double* __restrict__ q, double* __restrict__ w,
-                                                        double* __restrict__ part) {
-  __shared__ double red[kThreads / 32];
-  double acc = 0.0;
-  for (int64_t j = blockIdx.x; j < n; j += gridDim.x) {
-    const double* a = Z + j * n;
-    double s = 0.0;
-    for (int64_t i = threadIdx.x; i < n; i += blockDim.x) s = fma(a[i], q[i], s);
-    const double t = block_sum256(s, red);
-    if (threadIdx.x == 0) w[j] = t;
-    acc = fma(q[j], t, acc);
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = acc;
-}
-// a = sum of the matvec's partials (stored to *pa by block 0),
-// w -= a q + sqrt(*pbb) p (no p at the first step)
-__global__ void __launch_bounds__(kThreads) k_lz_update(int64_t n, double* __restrict__ w, const double* __restrict__ q,
-                                                        const double* __restrict__ p, const double* __restrict__ part,
-                                                        int np, double* __restrict__ pa,
-                                                        const double* __restrict__ pbb) {
-  __shared__ double red[kThreads / 32];
-  const double a = sum_partials(part, np, red);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *pa = a;
-  const double b = p ? sqrt(*pbb) : 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    w[i] -= a * q[i] + (p ? b * p[i] : 0.0);
-}
-// k_gemv_sub, and part[b] = sum of the updated out_i^2 over the block's rows
-__global__ void __launch_bounds__(1024) k_gemv_sub_dot(int64_t rows, int cols, const double* __restrict__ A,
-                                                      int64_t lda, const double* __restrict__ v,
-                                                      double* __restrict__ out, double* __restrict__ part) {
-  __shared__ double pr[32][33];
-  const int r = threadIdx.x & 31, g = threadIdx.x >> 5;
-  const int64_t i = (int64_t)blockIdx.x * 32 + r;
-  double s = 0.0;
-  if (i < rows)
-    for (int j = g; j < cols; j += 32) s = fma(A[i + j * lda], v[j], s);
-  pr[g][r] = s;
-  __syncthreads();
-  if (g == 0) {
-    double t = 0.0, sq = 0.0;
-    if (i < rows) {
-      for (int q = 0; q < 32; ++q) t += pr[q][r];
-      const double o = out[i] - t;
-      out[i] = o;
-      sq = o * o;
-    }
-    for (int o = 16; o; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-    if (r == 0) part[blockIdx.x] = sq;
-  }
-}
-// bb = sum of the partials (stored to *pbb by block 0), out = w / sqrt(bb)
-__global__ void __launch_bounds__(kThreads) k_lz_normalize(int64_t n, const double* __restrict__ w,
-                                                           const double* __restrict__ part, int np,
-                                                           double* __restrict__ pbb, double* __restrict__ out) {
-  __shared__ double red[kThreads / 32];
-  const double bb = sum_partials(part, np, red);
-  if (blockIdx.x == 0 && threadIdx.x == 0) *pbb = bb;
-  const double inv = 1.0 / sqrt(bb);
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-    out[i] = w[i] * inv;
-}
-int64_t lanczos_partials(int64_t n) { return std::min<int64_t>(n, 152 * 16) + (n + 31) / 32 + 1; }
-
 // 64-bit copy of sytrf's pivot indices (the solve's format)
 __global__ void k_ipiv64(int m, const int* __restrict__ p, int64_t* __restrict__ q) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) q[i] = p[i];
@@ -620,8 +514,11 @@ struct msdp_solver {
   int* eibuf = nullptr;
   int64_t eig_refined = 0, eig_dense = 0, eig_steps = 0;
   int64_t lanczos_calls = 0, lanczos_steps = 0, eigmin_dense = 0;  // lambda_min of blocks above 256
-  double *lq = nullptr, *lh = nullptr;  // Lanczos basis (n x (kLanczosMax + 1)) and projections
-  double* lzp = nullptr;                 // per-block partial sums of the fused Lanczos step
+  // Lanczos above lanczos::kMaxOrder, two matrices at a time: bases, work
+  // vectors, tridiagonals (device and pinned), the second matrix's stream
+  double *lq = nullptr, *lw = nullptr, *lab = nullptr, *hlab = nullptr;
+  cudaStream_t st2 = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
   lanczos::Job* ljobs = nullptr;         // eigenproblems of one step length (orders up to 256)
   int* dinfo = nullptr;
   double *partial = nullptr, *slots = nullptr;
@@ -1465,19 +1362,20 @@ void correction(S* s) {
   if (s->ns) LAUNCH(s, k_corr_lin, s->ns, s->ns, s->dx, s->dz, s->zinv, s->corrlin);
 }
 
-// ---- Lanczos for lambda_min of a formed symmetric Z (blocks above
-// lanczos::kMaxOrder, 256).  Full reorthogonalization (twice); the step's scalars
-// stay on the device and the host reads them every kLanczosBatch steps to
-// apply the stopping rule at each step in order: the smallest Ritz value of
-// the first step whose Ritz residual |beta_k s_k| is below 1e-12 ||Z||, or
-// of step n.  Gives up at kLanczosMax (the caller then uses the dense
+// ---- Lanczos for lambda_min of formed symmetric Z above lanczos::kMaxOrder.
+// The steps of up to two matrices run on two streams (one's 16-block
+// orthogonalization beside the other's matrix-vector product); the host reads
+// the tridiagonals every kLanczosBatch steps.  Stops at the end of the first
+// batch whose Ritz residual |beta_k s_k| is below 1e-12 ||Z|| (later steps
+// change the Ritz value by the residual's square), at a beta below that or at
+// step n.  Gives up at lanczos::kMaxSteps (the caller then uses the dense
 // eigensolver).
-constexpr int kLanczosMin = lanczos::kMaxOrder + 1;
-constexpr int kLanczosMax = 320;
-constexpr int kLanczosBatch = 8;
+constexpr int kLanczosBatch = 16;
 
-bool lanczos_eigmin(S* s, int n, const double* Z, double* out) {
-  double* Q = s->lq;
+// out[q] = lambda_min(Z[q]) and done[q] for q < count (count <= 2); false on a
+// CUDA error
+bool lanczos_large(S* s, int n, const double* const* Z, int count, double* out, bool* done) {
+  using lanczos::kMaxSteps;
   // fixed pseudo-random start vector (xorshift), normalized
   std::vector<double> q0(n);
   uint64_t st = 0x9E3779B97F4A7C15ull ^ (uint64_t)n;
@@ -1489,55 +1387,72 @@ bool lanczos_eigmin(S* s, int n, const double* Z, double* out) {
   }
   nrm = std::sqrt(nrm);
   for (auto& v : q0) v /= nrm;
-  CU(s, cudaMemcpyAsync(Q, q0.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
-  std::vector<double> al, be;
-  std::vector<int> aslot, bslot;
-  const int kmax = std::min(n, kLanczosMax);
-  const int ga = std::min(n, 152 * 16);
-  for (int k0 = 0; k0 < kmax; k0 += kLanczosBatch) {
+  lanczos::Large job[2];
+  cudaStream_t sts[2] = {s->st, s->st2};
+  const int64_t qlen = (int64_t)n * (kMaxSteps + 1);
+  const int ablen = 2 * kMaxSteps;
+  for (int q = 0; q < count; ++q) {
+    job[q].n = n;
+    job[q].Z = Z[q];
+    job[q].Q = s->lq + q * qlen;
+    job[q].w = s->lw + (int64_t)q * n;
+    job[q].ab = s->lab + q * ablen;
+    CU(s, cudaMemcpyAsync(job[q].Q, q0.data(), sizeof(double) * n, cudaMemcpyHostToDevice, s->st));
+    done[q] = false;
+  }
+  // the second stream starts after what the first has been given so far
+  if (count > 1) {
+    CU(s, cudaEventRecord(s->fork, s->st));
+    CU(s, cudaStreamWaitEvent(s->st2, s->fork, 0));
+  }
+  const int kmax = std::min(n, kMaxSteps);
+  bool open[2] = {true, count > 1};
+  for (int k0 = 0; k0 < kmax && !s->fail && (open[0] || open[1]); k0 += kLanczosBatch) {
     const int k1 = std::min(kmax, k0 + kLanczosBatch);
-    for (int k = k0; k < k1; ++k) {
-      const double* q = Q + (int64_t)k * n;
-      double* w = Q + (int64_t)(k + 1) * n;
-      // seven launches per step: matvec with the a partials, update (sums
-      // them), two reorthogonalization passes (the second leaving the w'w
-      // partials), normalization (sums those)
-      double* pa_part = s->lzp;
-      double* pb_part = s->lzp + ga;
-      const int gsub = (n + 31) / 32;
-      const int sa = next_slot(s);
-      const int sb = next_slot(s);
-      aslot.push_back(sa);
-      k_lz_matvec<<<ga, kThreads, 0, s->st>>>((int64_t)n, Z, q, w, pa_part);
-      k_lz_update<<<grid_for(n), kThreads, 0, s->st>>>((int64_t)n, w, q, k ? Q + (int64_t)(k - 1) * n : nullptr,
-                                                        pa_part, ga, s->slots + sa,
-                                                        k ? s->slots + bslot.back() : s->slots + sa);
-      for (int r = 0; r < 2; ++r) {
-        k_gemv_t<<<std::min(k + 1, 152 * 16), kThreads, 0, s->st>>>(n, k + 1, Q, n, w, s->lh, 0);
-        if (r == 0)
-          k_gemv_sub<<<gsub, 1024, 0, s->st>>>((int64_t)n, k + 1, Q, (int64_t)n, s->lh, w);
-        else
-          k_gemv_sub_dot<<<gsub, 1024, 0, s->st>>>((int64_t)n, k + 1, Q, (int64_t)n, s->lh, w, pb_part);
-      }
-      bslot.push_back(sb);
-      k_lz_normalize<<<grid_for(n), kThreads, 0, s->st>>>((int64_t)n, w, pb_part, gsub, s->slots + sb, w);
-      s->launches += 7;
-      CU(s, cudaGetLastError());
+    // interleaved, so that neither stream waits for the host
+    for (int k = k0; k < k1; ++k)
+      for (int q = 0; q < count; ++q)
+        if (open[q]) CU(s, lanczos::large_steps(job[q], k, k + 1, sts[q]));
+    for (int q = 0; q < count; ++q) {
+      if (!open[q]) continue;
+      CU(s, cudaMemcpyAsync(s->hlab + q * ablen, job[q].ab, sizeof(double) * ablen, cudaMemcpyDeviceToHost, sts[q]));
+      s->launches += 2 * (k1 - k0);
+      s->lanczos_steps += k1 - k0;
     }
-    if (!fetch(s)) return false;
-    s->lanczos_steps += k1 - k0;
-    for (int k = k0; k < k1; ++k) {
-      al.push_back(s->hslots[aslot[k]]);
-      const double beta = std::sqrt(std::max(s->hslots[bslot[k]], 0.0));
+    for (int q = 0; q < count; ++q) {
+      if (!open[q]) continue;
+      CU(s, cudaStreamSynchronize(sts[q]));
+      if (s->fail) break;
+      const double* ha = s->hlab + q * ablen;
+      std::vector<double> al(ha, ha + k1), be(k1);
+      int k = k1;
+      double zn = 0.0;
+      for (int i = 0; i < k1; ++i) {
+        be[i] = std::sqrt(std::max(ha[kMaxSteps + i], 0.0));
+        zn = std::max(zn, std::fabs(al[i]) + be[i] + (i ? be[i - 1] : 0.0));
+        if (!(be[i] > 1e-12 * zn)) {  // an invariant subspace (or an entry that is not a number): nothing after it counts
+          k = i + 1;
+          break;
+        }
+      }
       double znorm = 0.0;
-      const double theta = tridiag_min(al, be, k + 1, &znorm);
-      if (k + 1 == n || beta <= 1e-300) { *out = theta; return true; }
-      const double resid = beta * tridiag_last_component(al, be, k + 1, theta, znorm);
-      if (resid <= 1e-12 * std::max(znorm, 1e-300)) { *out = theta; return true; }
-      be.push_back(beta);
+      const double theta = tridiag_min(al, be, k, &znorm);
+      bool stop = k == n || k < k1 || !(be[k - 1] > 1e-12 * zn);
+      if (!stop) stop = be[k - 1] * tridiag_last_component(al, be, k, theta, znorm) <= 1e-12 * std::max(znorm, 1e-300);
+      if (stop) {
+        out[q] = theta;
+        done[q] = true;
+        open[q] = false;
+      }
     }
   }
-  return false;
+  // what follows on the main stream comes after the second one's work (also
+  // where the loop was left by an error)
+  if (count > 1) {
+    CU(s, cudaEventRecord(s->join, s->st2));
+    CU(s, cudaStreamWaitEvent(s->st, s->join, 0));
+  }
+  return !s->fail;
 }
 
 // ---- step lengths (src/step.jl:148-228)
@@ -1553,25 +1468,27 @@ void form_congruence(S* s, int n, const double* L, const double* D, double* Z) {
   LAUNCH(s, k_sym, (int64_t)n * n, n, Z);
 }
 
-// slot of lambda_min(Z) for n > lanczos::kMaxOrder: host-driven Lanczos or,
-// when it does not converge, the dense eigensolver
-int eigmin_large(S* s, Blk& b, double* Z) {
+// slots of lambda_min(Z[q]), q < count <= 2, for n > lanczos::kMaxOrder:
+// Lanczos or, when it does not converge, the dense eigensolver
+void eigmin_large(S* s, Blk& b, double* const* Z, int count, int* slot) {
   const int n = b.n;
-  if (n >= kLanczosMin) {
-    double lam = 0.0;
-    s->lanczos_calls += 1;
-    if (lanczos_eigmin(s, n, Z, &lam)) {
-      const int slot = next_slot(s);
-      k_put_scalar<<<1, 1, 0, s->st>>>(s->slots + slot, lam);
+  double lam[2] = {0.0, 0.0};
+  bool done[2] = {false, false};
+  s->lanczos_calls += count;
+  lanczos_large(s, n, Z, count, lam, done);
+  for (int q = 0; q < count; ++q) {
+    if (done[q]) {
+      slot[q] = next_slot(s);
+      k_put_scalar<<<1, 1, 0, s->st>>>(s->slots + slot[q], lam[q]);
       s->launches += 1;
-      return slot;
+      continue;
     }
+    const int k = next_info(s);
+    CS(s, cusolverDnDsyevd(s->cs, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER, n, Z[q], n, b.w, s->work, s->lwork,
+                           s->dinfo + k));
+    s->eigmin_dense += 1;
+    slot[q] = copy_slot(s, b.w);
   }
-  const int k = next_info(s);
-  CS(s, cusolverDnDsyevd(s->cs, CUSOLVER_EIG_MODE_NOVECTOR, CUBLAS_FILL_MODE_LOWER, n, Z, n, b.w, s->work, s->lwork,
-                         s->dinfo + k));
-  s->eigmin_dense += 1;
-  return copy_slot(s, b.w);
 }
 
 double eigen_step(double lam, double tau) { return lam > -std::sqrt(kEps) ? 1.0 : std::min(1.0, -tau / lam); }
@@ -1638,8 +1555,11 @@ bool step_lengths(S* s, double* a_out, double* b_out) {
         (side ? ls : lx).push_back(slot);
       }
     } else {
-      lx.push_back(eigmin_large(s, b, b.T1));
-      ls.push_back(eigmin_large(s, b, b.T2));
+      double* const Z[2] = {b.T1, b.T2};
+      int slot[2];
+      eigmin_large(s, b, Z, 2, slot);
+      lx.push_back(slot[0]);
+      ls.push_back(slot[1]);
     }
   }
   if (!jobs.empty()) {
@@ -2084,6 +2004,13 @@ bool detect_rank_one(int n, int m, int64_t nnz, const int32_t* con, const int32_
 
 void release(S* s) {
   if (s->st) cudaStreamSynchronize(s->st);
+  if (s->st2) {
+    cudaStreamSynchronize(s->st2);
+    cudaStreamDestroy(s->st2);
+  }
+  if (s->fork) cudaEventDestroy(s->fork);
+  if (s->join) cudaEventDestroy(s->join);
+  if (s->hlab) cudaFreeHost(s->hlab);
   for (auto& e : s->ev)
     if (e) cudaEventDestroy(e);
   for (void* p : s->allocs) cudaFree(p);
@@ -2357,12 +2284,16 @@ int msdp_solver_create(msdp_context* ctx, const msdp_problem_desc* d, const msdp
   }
   int nmax = 0;
   for (auto& b : s->B) nmax = std::max(nmax, b.n);
-  if (nmax >= kLanczosMin) {
-    s->lq = vec((int64_t)nmax * (std::min(nmax, kLanczosMax) + 1));
-    s->lh = vec(kLanczosMax + 1);
-    s->lzp = vec(lanczos_partials(nmax));
-    if (!s->lzp) return bail(MSDP_ERR_OUT_OF_MEMORY);
-    if (!s->lq || !s->lh) return bail(MSDP_ERR_OUT_OF_MEMORY);
+  if (nmax > lanczos::kMaxOrder) {
+    s->lq = vec(2 * (int64_t)nmax * (lanczos::kMaxSteps + 1));
+    s->lw = vec(2 * (int64_t)nmax);
+    s->lab = vec(4 * lanczos::kMaxSteps);
+    if (!s->lq || !s->lw || !s->lab) return bail(MSDP_ERR_OUT_OF_MEMORY);
+    if (cudaMallocHost((void**)&s->hlab, sizeof(double) * 4 * lanczos::kMaxSteps) != cudaSuccess ||
+        cudaStreamCreateWithFlags(&s->st2, cudaStreamNonBlocking) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&s->join, cudaEventDisableTiming) != cudaSuccess)
+      return bail(MSDP_ERR_CUDA);
   }
   if (s->nb) {
     s->ljobs = dalloc<lanczos::Job>(s, 2 * s->nb);
@@ -2532,7 +2463,7 @@ int msdp_solver_step_eig(msdp_solver* s, int32_t block, const double* L, const d
     CU(s, lanczos::eigmin(s->ljobs, 1, n, s->st));
     s->launches += 1;
   } else {
-    slot = eigmin_large(s, b, b.T1);
+    eigmin_large(s, b, &b.T1, 1, &slot);
   }
   if (!fetch(s)) return s->fail ? s->fail : MSDP_ERR_CUDA;
   *lambda_min = s->hslots[slot];

@@ -278,7 +278,165 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
   if (cs > 1) cluster_sync();
 }
 
+// ---------------------------------------------------------------- orders above 256
+// w = Z q, Z symmetric and read by columns: one warp per entry.  Bound by the
+// FP64 units (n^2 multiply-adds at 1.6 per clock and SM: 8 us at n = 2000); a
+// block per entry with a block-wide sum took 24 us.
+constexpr int kMatvecThreads = 128;
+__global__ void __launch_bounds__(kMatvecThreads) k_matvec(int n, const double* __restrict__ Z,
+                                                          const double* __restrict__ q, double* __restrict__ w) {
+  const int lane = threadIdx.x & 31;
+  const int j = blockIdx.x * (kMatvecThreads / 32) + (threadIdx.x >> 5);
+  if (j >= n) return;
+  const double* a = Z + (int64_t)j * n;
+  double s = 0.0;
+#pragma unroll 8
+  for (int i = lane; i < n; i += 32) s = fma(a[i], q[i], s);
+#pragma unroll
+  for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane == 0) w[j] = s;
+}
+
+// Orthogonalization of w against q_0 .. q_j (twice) and the next basis vector,
+// in one cluster: every block holds a slice of the rows, the coefficients'
+// partial sums go to all blocks through distributed shared memory, and all add
+// them in the same order.  The second pass carries w'w, so the new norm
+// needs no exchange of its own (as in k_lanczos).  A warp sums four
+// coefficients at a time, so that their reduction takes six additions, not
+// twenty.  Bound by 4 j n multiply-adds on the FP64 units of 16 SMs, about
+// 12 us at n = 2000, j = 70; five launches over the whole GPU took 25 us and
+// the gaps between them as much again.
+__host__ __device__ inline int64_t large_smem(int n, int cs) {
+  const int nr = (n + cs - 1) / cs;
+  return 8 * ((int64_t)nr + kThreads + 2 * (kMaxSteps + 2) + 2 * (int64_t)cs * (kMaxSteps + 2));
+}
+__global__ void __launch_bounds__(kThreads) k_orthogonalize(int n, int j, double* __restrict__ Q,
+                                                           const double* __restrict__ w, double* __restrict__ ab) {
+  int cs, rank;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(cs));
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const int nrm = (n + cs - 1) / cs, r0 = min(n, rank * nrm), nr = min(n, r0 + nrm) - r0;
+  extern __shared__ double sm[];
+  double* ws = sm;                       // [nrm]
+  double* part = ws + nrm;               // [kThreads]
+  double* mine = part + kThreads;        // [kMaxSteps + 2] partial sums of this block
+  double* coef = mine + kMaxSteps + 2;   // [kMaxSteps + 2]
+  double* xch = coef + kMaxSteps + 2;    // [2][cs][kMaxSteps + 2]
+  auto cluster_sync = [&] {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  };
+  for (int i = t; i < nr; i += kThreads) ws[i] = w[r0 + i];
+  cluster_sync();  // every block has started before its shared memory is written
+  const double* Qr = Q + r0;
+  const int L = j + 1;
+  bool large = false;
+  for (int pass = 0; pass < 2; ++pass) {
+    const int LL = L + pass;  // the second pass's last output is w'w
+    // ---- partial coefficients, four per warp at a time
+    for (int l0 = 4 * warp; l0 < LL; l0 += 4 * (kThreads / 32)) {
+      const double* p[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) p[u] = l0 + u < L ? Qr + (int64_t)(l0 + u) * n : ws;  // the last: w itself
+      double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
+      for (int i = lane; i < nr; i += 32) {
+        const double x = ws[i];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = fma(p[u][i], x, v[u]);
+      }
+      const bool hi = lane & 16, mid = lane & 8;
+      const double s0 = (hi ? v[2] : v[0]) + __shfl_xor_sync(0xffffffffu, hi ? v[0] : v[2], 16);
+      const double s1 = (hi ? v[3] : v[1]) + __shfl_xor_sync(0xffffffffu, hi ? v[1] : v[3], 16);
+      double s = (mid ? s1 : s0) + __shfl_xor_sync(0xffffffffu, mid ? s0 : s1, 8);
+#pragma unroll
+      for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      const int l = l0 + (lane >> 3);
+      if ((lane & 7) == 0 && l < LL) mine[l] = s;
+    }
+    __syncthreads();
+    double* x = xch + (int64_t)pass * cs * (kMaxSteps + 2);
+    for (int idx = t; idx < LL * cs; idx += kThreads)
+      store_remote(x + (int64_t)rank * (kMaxSteps + 2) + idx % LL, idx / LL, mine[idx % LL]);
+    cluster_sync();
+    for (int l = t; l < LL; l += kThreads) {
+      double s = 0.0;
+      for (int r = 0; r < cs; ++r) s += x[(int64_t)r * (kMaxSteps + 2) + l];
+      coef[l] = s;
+    }
+    __syncthreads();
+    if (pass == 0 && rank == 0 && t == 0) ab[j] = coef[j];
+    // ---- w -= Q coef: rows in groups of 128, four parts of the sum each
+    for (int i0 = 0; i0 < nr; i0 += 128) {
+      const int i = i0 + (t & 127), u = t >> 7;
+      double s = 0.0;
+      if (i < nr) {
+        const double* q = Qr + i;
+#pragma unroll 4
+        for (int l = u * L / 4; l < (u + 1) * L / 4; ++l) s = fma(-coef[l], q[(int64_t)l * n], s);
+      }
+      part[t] = s;
+      __syncthreads();
+      if (t < 128 && i < nr) ws[i] += (part[t] + part[t + 128]) + (part[t + 256] + part[t + 384]);
+      __syncthreads();
+    }
+    if (pass == 1) {
+      // a coefficient above 2^-30 |w'| changes the norm
+      const int en = (__double2hiint(coef[L]) >> 20) - 1023;
+      int ec = -2000;
+      for (int l = t; l < L; l += kThreads) ec = max(ec, ((__double2hiint(coef[l]) >> 20) & 0x7ff) - 1023);
+      large = __syncthreads_or(2 * ec > en - 60);
+    }
+  }
+  if (t < 128) {
+    double bn2 = coef[L];
+    if (large)
+      for (int l = 0; l < L; ++l) bn2 = fma(-coef[l], coef[l], bn2);
+    const int field = __double2hiint(bn2) >> 20;
+    double bn = 0.0, binv = 0.0;
+    if (field > 27 && field < 0x7ff) fast_root(bn2, bn, binv);  // above 1e-300
+    else bn2 = field == 0x7ff ? bn2 : 0.0;
+    for (int i = t; i < nr; i += 128) Q[(int64_t)(j + 1) * n + r0 + i] = ws[i] * binv;
+    if (rank == 0 && t == 0) ab[kMaxSteps + j] = bn2;
+  }
+  cluster_sync();
+}
+
 }  // namespace
+
+cudaError_t large_steps(const Large& a, int k0, int k1, cudaStream_t st) {
+  if (k1 > kMaxSteps || a.n <= 0) return cudaErrorInvalidValue;
+  static std::once_flag once;
+  static cudaError_t attr = cudaSuccess;
+  static bool wide = false;
+  std::call_once(once, [] {
+    attr = cudaFuncSetAttribute(k_orthogonalize, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemMax);
+    wide = cudaFuncSetAttribute(k_orthogonalize, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    cudaGetLastError();
+  });
+  if (attr != cudaSuccess) return attr;
+  const int cs = wide ? 16 : 8;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)cs);
+  cfg.blockDim = dim3(kThreads);
+  cfg.dynamicSmemBytes = (size_t)large_smem(a.n, cs);
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)cs;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cfg.dynamicSmemBytes > (size_t)kSmemMax) return cudaErrorInvalidValue;
+  cudaError_t e = cudaSuccess;
+  const unsigned grid = (unsigned)((a.n + kMatvecThreads / 32 - 1) / (kMatvecThreads / 32));
+  for (int k = k0; k < k1 && e == cudaSuccess; ++k) {
+    k_matvec<<<grid, kMatvecThreads, 0, st>>>(a.n, a.Z, a.Q + (int64_t)k * a.n, a.w);
+    e = cudaLaunchKernelEx(&cfg, k_orthogonalize, a.n, k, a.Q, (const double*)a.w, a.ab);
+    if (e == cudaSuccess) e = cudaGetLastError();
+  }
+  return e;
+}
 
 cudaError_t eigmin(const Job* jobs, int count, int nmax, cudaStream_t st) {
   if (count <= 0) return cudaSuccess;

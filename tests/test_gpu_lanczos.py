@@ -1,10 +1,11 @@
-"""The cluster Lanczos behind EigenStep (blocks up to 256) through
-msdp_solver_step_eig with L = I, against numpy's symmetric eigenvalues, at
-the orders where the number of blocks of a cluster changes (115/116,
-160/161, 220/221) and at the smallest ones.  The iteration stops when the
+"""The Lanczos iterations behind EigenStep through msdp_solver_step_eig with
+L = I, against numpy's symmetric eigenvalues: the cluster kernel (up to 256)
+at the orders where the number of blocks of a cluster changes (32/33, 64/65,
+128/129) and at the smallest ones, the two-launch steps above.  The iteration stops when the
 smallest Ritz value moved by at most 64 eps max(1, |theta|) in four steps;
 with a convergence factor of at most 0.99 per four steps the rest is below
-64 eps * 99 = 1.4e-12, relative to the larger of 1 and the norm."""
+64 eps * 99 = 1.4e-12, relative to the larger of 1 and the norm; above 256 it
+stops at a Ritz residual of 1e-12 of the norm, which bounds the error."""
 import numpy as np
 import pytest
 
@@ -14,7 +15,7 @@ from madsdp_gpu.solver import InstanceSolver
 
 pytestmark = pytest.mark.gpu
 
-ORDERS = [2, 3, 4, 5, 8, 31, 33, 64, 100, 115, 116, 129, 160, 161, 220, 221, 256]
+ORDERS = [2, 3, 4, 5, 8, 31, 32, 33, 64, 65, 100, 128, 129, 255, 256, 257, 300, 320, 321, 517]
 
 
 @pytest.fixture(scope="module")
