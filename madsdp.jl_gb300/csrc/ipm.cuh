@@ -34,6 +34,7 @@ struct SharedState {
   int erd64;     // FP32 phase: E(Rd) in float64 formed for this iteration
   int pad2;
   double bc[8];  // broadcast scalars
+  LanczosShared lz;
   uint64_t t0;   // launch start on this CTA (globaltimer)
 };
 
@@ -369,15 +370,6 @@ __device__ T lanczos_eigmin(int n, const T* Z, T* Q, T* a, T* bb, T* w, T* coef,
   return theta;
 }
 
-// (j, k) with j >= k of the idx-th entry of a packed lower triangle (row major).
-__device__ __forceinline__ void tri_index(int64_t idx, int& j, int& k) {
-  int r = (int)((sqrt(8.0 * (double)idx + 1.0) - 1.0) * 0.5);
-  while ((int64_t)(r + 1) * (r + 2) / 2 <= idx) ++r;
-  while ((int64_t)r * (r + 1) / 2 > idx) --r;
-  j = r;
-  k = (int)(idx - (int64_t)r * (r + 1) / 2);
-}
-
 // ------------------------------------------------------------------ algorithm
 template <class T>
 struct Algo {
@@ -478,25 +470,21 @@ struct Algo {
     bool conv;
     int sweeps = 0;
     PROF_BEGIN(j);
-    const bool f32ws = prm.precision == MSDP_MIXED;  // an FP32 workspace exists
-    const bool smem32 = (2 * nn + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES;
-    if (sizeof(T) == 8 && (f32ws || smem32)) {
+    if (sizeof(T) == 8) {
       // float64 NT scaling (the FP64 path and the FP64 phase of the mixed
       // path): eigenvectors by FP32 Jacobi, then M V and Lx V in FP64 and
       // FP64 polishing sweeps to float64 convergence (quadratic from the
-      // FP32 basis).  Operands live in shared memory when they fit, else in
-      // the (idle) FP32 workspace of a mixed batch and FP64 scratch.
-      float *sMf, *sVf, *Df;
-      if (smem32) {
-        sMf = (float*)smem;
-        sVf = sMf + nn;
-        Df = sVf + nn;
-      } else {
-        const Blk<float> bf = make_blk<float>(B, P, blk_index(b));
-        sMf = bf.W(W_T1);
-        sVf = bf.W(W_T2);
-        Df = bf.V(WV_D);
-      }
+      // FP32 basis).  FP32 operands live in shared memory when both fit (up to
+      // n = 95), else the vectors (and from n = 136 on M too) in the FP64
+      // scratch, and the basis is made orthonormal to FP64 by two Newton-Schulz
+      // steps V (3 I - V'V) / 2 (the defect of 1e-6 is squared twice).  FP64
+      // sweeps from the identity at these sizes took 130 million clocks a call
+      // at n = 128.
+      float* scratch = (float*)b.W(W_T3);
+      const bool both = (2 * nn + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES;
+      float* sMf = nn * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES ? (float*)smem : scratch;
+      float* sVf = both ? sMf + nn : scratch + nn;
+      float* Df = both ? sVf + nn : (float*)b.V(WV_EIG);
       for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
         sMf[k] = (float)M[k];
         sVf[k] = ((k % n) == (k / n)) ? 1.0f : 0.0f;
@@ -507,6 +495,21 @@ struct Algo {
       T* V64 = b.W(W_T2);
       for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) V64[k] = (T)sVf[k];
       __syncthreads();
+      for (int step = 0; !both && step < 2; ++step) {
+        T* K = b.W(W_T3);
+        T* src = step ? GV : V64;
+        T* dst = step ? V64 : GV;
+        cta_gemm<T>(n, 1, 0, 0, 0, (T)1, src, src, (T)0, K, scr(), 1);
+        for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
+          const int r = (int)k % n, c = (int)k / n;
+          if (r < c) continue;
+          const T v = r == c ? (T)1.5 - (T)0.5 * K[k] : (T)-0.5 * K[k];
+          K[k] = v;
+          K[c + (int64_t)r * n] = v;
+        }
+        __syncthreads();
+        cta_gemm<T>(n, 0, 0, 0, 0, (T)1, src, K, (T)0, dst, scr());
+      }
       const bool smem64 = 2 * nn * (int64_t)sizeof(T) <= MSDP_SMEM_BYTES;
       T* sM = smem64 ? (T*)smem : b.W(W_T3);
       T* sB = smem64 ? sM + nn : GV;
@@ -539,21 +542,39 @@ struct Algo {
     PROF_COUNT(SC_N_JACOBI_SWEEPS, sweeps);
     PROF_COUNT(SC_N_JACOBI_CALLS, 1);
     PROF_BEGIN(np);
-    if (threadIdx.x == 0) {
-      int bad = conv ? 0 : 1;
-      for (int k = 0; k < n; ++k)
-        if (!(D[k] > (T)0) || !Num<T>::finite(D[k])) bad = 1;
-      sh.flag = bad;
-    }
-    __syncthreads();
-    if (sh.flag) return false;
+    int bad = conv ? 0 : 1;
+    for (int k = threadIdx.x; k < n; k += NTHREADS)
+      if (!pivot_ok(D[k])) bad = 1;  // positive and finite
+    if (__syncthreads_or(bad)) return false;
     T* G = GV;
     T* t2 = b.W(W_T2);
-    for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
-      const int j = (int)(k / n);
-      const T sq = Num<T>::sqrt_(D[j]);
-      G[k] = G[k] / sq;                 // G = Lx V D^-1/2
-      M[k] = M[k] / (D[j] * sq);        // (M V) D^-3/2
+    // double: the columns' factors once, in shared memory (a root and two
+    // divisions per entry took most of this phase)
+    T* f = (T*)smem;  // D^-1/2, D^-3/2, D^-1
+    if constexpr (sizeof(T) == 8) {
+      for (int k = threadIdx.x; k < n; k += NTHREADS) {
+        double root, inv;
+        chol_pivot<double>(D[k], root, inv);
+        const double rec = fast_recip(D[k]);
+        f[k] = inv;
+        f[n + k] = inv * rec;
+        f[2 * n + k] = rec;
+      }
+      __syncthreads();
+      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
+        const int j = (int)k / n;
+        const T g = G[k] * f[j];
+        G[k] = g;                         // G = Lx V D^-1/2
+        M[k] *= f[n + j];                 // (M V) D^-3/2
+        t2[k] = g * f[2 * n + j];         // G D^-1
+      }
+    } else {
+      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
+        const int j = (int)(k / n);
+        const T sq = Num<T>::sqrt_(D[j]);
+        G[k] = G[k] / sq;                 // G = Lx V D^-1/2
+        M[k] = M[k] / (D[j] * sq);        // (M V) D^-3/2
+      }
     }
     __syncthreads();
     // Gi = ((M V) D^-3/2)' Ls'
@@ -561,8 +582,10 @@ struct Algo {
     cta_gemm<T>(n, 0, 1, 0, 0, (T)1, G, G, (T)0, b.W(W_W), scr(), 1);
     cta_lower_to_full<T>(n, b.W(W_W));
     // S^-1 = G D^-1 G'
-    for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) t2[k] = G[k] / D[k / n];
-    __syncthreads();
+    if constexpr (sizeof(T) != 8) {
+      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) t2[k] = G[k] / D[k / n];
+      __syncthreads();
+    }
     cta_gemm<T>(n, 0, 1, 0, 0, (T)1, t2, G, (T)0, b.W(W_SI), scr(), 1);
     cta_lower_to_full<T>(n, b.W(W_SI));
     PROF_END(np, SC_T_NTPROD);
@@ -1070,7 +1093,7 @@ struct Algo {
         cta_gemm<T>(n, 0, 0, 0, 0, (T)1, t2, b.W(W_G), (T)0, t3, scr());
         for (int64_t k = threadIdx.x; k < b.nn; k += NTHREADS) {
           const int p = (int)(k % n), q = (int)(k / n);
-          RNT[k] = -(t3[k] + t3[q + (int64_t)p * n]) / (D[p] + D[q]);
+          RNT[k] = neg_div(t3[k] + t3[q + (int64_t)p * n], D[p] + D[q]);
         }
         __syncthreads();
         // G RNT G' with RNT symmetric: lower triangle only
@@ -1168,10 +1191,25 @@ struct Algo {
       cta_gemm<T>(n, 1, 0, 0, 0, (T)1, b.W(W_G), dst, (T)0, t1, scr());
       cta_gemm<T>(n, 0, 0, 0, 0, (T)1, t1, b.W(W_G), (T)0, ZS, scr());
       const T* D = b.V(WV_D);
-      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
-        const T sc = Num<T>::rsqrt_(D[k % n]) * Num<T>::rsqrt_(D[k / n]);
-        ZX[k] *= sc;
-        ZS[k] *= sc;
+      if constexpr (sizeof(T) == 8) {
+        T* f = (T*)smem;  // D^-1/2, one root per column instead of two per entry
+        for (int k = threadIdx.x; k < n; k += NTHREADS) {
+          double root, inv;
+          chol_pivot<double>(D[k], root, inv);
+          f[k] = inv;
+        }
+        __syncthreads();
+        for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
+          const T sc = f[(int)k % n] * f[(int)k / n];
+          ZX[k] *= sc;
+          ZS[k] *= sc;
+        }
+      } else {
+        for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
+          const T sc = Num<T>::rsqrt_(D[k % n]) * Num<T>::rsqrt_(D[k / n]);
+          ZX[k] *= sc;
+          ZS[k] *= sc;
+        }
       }
       __syncthreads();
     } else {
@@ -1201,7 +1239,16 @@ struct Algo {
     }
     if (f32) {
     } else if (n <= 256) {
-      lanczos_pair<T>(n, ZX, ZS, b.W(W_Q), b.W(W_RNT), b.V(WV_LA), b.V(WV_LA2), steps);
+      if constexpr (sizeof(T) == 8) {
+        int s1 = 0, s2 = 0;
+        const double lx = cta_lanczos_min(n, ZX, b.W(W_Q), smem, MSDP_SMEM_BYTES, sh.lz, &s1);
+        const double ls = cta_lanczos_min(n, ZS, b.W(W_RNT), smem, MSDP_SMEM_BYTES, sh.lz, &s2);
+        if (threadIdx.x == 0) { sh.bc[2] = lx; sh.bc[3] = ls; }
+        __syncthreads();
+        steps = s1 + s2;
+      } else {
+        lanczos_pair<T>(n, ZX, ZS, b.W(W_Q), b.W(W_RNT), b.V(WV_LA), b.V(WV_LA2), steps);
+      }
     } else {
       const T* zx = ZX;
       const T* zs = ZS;

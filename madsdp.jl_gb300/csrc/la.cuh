@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tridiag.cuh"
+
 #ifndef NTHREADS
 #define NTHREADS 128
 #endif
@@ -124,6 +126,36 @@ template <class T> __device__ void cta_set_identity(int n, T* A, T diag) {
   __syncthreads();
 }
 
+// (j, k) with j >= k of the idx-th entry of a packed lower triangle (row
+// major); the root only has to be near, the loops make it exact.
+__device__ __forceinline__ void tri_index(int64_t idx, int& j, int& k) {
+  int r = (int)((sqrtf(8.0f * (float)idx + 1.0f) - 1.0f) * 0.5f);
+  while ((int64_t)(r + 1) * (r + 2) / 2 <= idx) ++r;
+  while ((int64_t)r * (r + 1) / 2 > idx) --r;
+  j = r;
+  k = (int)(idx - (int64_t)r * (r + 1) / 2);
+}
+
+// 1/d of a normal d by an FP32 reciprocal of the mantissa and one third-order
+// correction (four dependent FP64 instructions, against about 700 clocks for a
+// division); within an ulp.
+__device__ __forceinline__ double fast_recip(double d) {
+  const long long b = __double_as_longlong(d);
+  const int field = (int)(b >> 52) & 0x7FF;
+  if (field < 2 || field > 2044) return 1.0 / d;
+  const double m = __longlong_as_double((b & 0x800FFFFFFFFFFFFFll) | 0x3FF0000000000000ll);  // +-[1, 2)
+  const float f = __frcp_rn(__int_as_float(0x3F800000 | (int)((b >> 29) & 0x7FFFFF)));       // (0.5, 1]
+  const int fb = __float_as_int(f);
+  const double y = __hiloint2double((((fb >> 3) & 0x0FFFFFFF) + 0x38000000) | ((int)(b >> 32) & 0x80000000), fb << 29);
+  const double e = fma(-m, y, 1.0);
+  const double z = fma(y, fma(e, e, e), y);
+  return __longlong_as_double(__double_as_longlong(z) - ((long long)(field - 1023) << 52));
+}
+
+// -s / d; in double by the reciprocal above (within two ulps)
+__device__ __forceinline__ double neg_div(double s, double d) { return -s * fast_recip(d); }
+__device__ __forceinline__ float neg_div(float s, float d) { return -s / d; }
+
 // ---------------------------------------------------------------- GEMM
 // C = alpha * op(A) * op(B) + beta * C for n x n matrices.  ta/tb: 0 = as
 // stored, 1 = transposed.  loA/loB: the stored operand is lower triangular
@@ -133,10 +165,17 @@ template <class T, int R>
 __device__ void cta_gemm_r(int n, int ta, int tb, int loA, int loB, T alpha, const T* __restrict__ A,
                            const T* __restrict__ B, T beta, T* __restrict__ C, int loC = 0) {
   const int nb = (n + R - 1) / R;
-  const int tiles = nb * nb;
+  const int tiles = loC ? nb * (nb + 1) / 2 : nb * nb;
+  const bool unit = alpha == (T)1, zero = beta == (T)0;
   for (int t = threadIdx.x; t < tiles; t += NTHREADS) {
-    const int i0 = (t % nb) * R, j0 = (t / nb) * R;
-    if (loC && j0 > i0 + R - 1) continue;  // only tiles touching the lower triangle
+    int ti, tj;
+    if (loC) {
+      tri_index(t, ti, tj);  // only tiles touching the lower triangle
+    } else {
+      tj = t / nb;
+      ti = t - tj * nb;
+    }
+    const int i0 = ti * R, j0 = tj * R;
     int klo = 0, khi = n;  // k in [klo, khi)
     if (loA) {
       if (!ta) khi = min(khi, i0 + R);  // A(i,k) != 0 -> k <= i
@@ -175,17 +214,22 @@ __device__ void cta_gemm_r(int n, int ta, int tb, int loA, int loB, T alpha, con
         const int i = i0 + r, j = j0 + c;
         if (i < n && j < n) {
           const int64_t o = i + (int64_t)j * n;
-          C[o] = (beta == (T)0) ? alpha * acc[r][c] : fma(alpha, acc[r][c], beta * C[o]);
+          const T v = unit ? acc[r][c] : alpha * acc[r][c];
+          C[o] = zero ? v : fma(alpha, acc[r][c], beta * C[o]);
         }
       }
   }
   __syncthreads();
 }
 
+// Tile sizes.  float: 4 x 4 above n = 24 (shared-memory reads bound it).
+// double: 2 x 2, because a FP64 multiply-add holds its quarter of the SM for
+// 64 clocks and the last round of 4 x 4 tiles leaves many lanes idle (n = 50:
+// 169 tiles of 16 on 128 threads take 32 multiply-adds a k, 2 x 2 tiles 20).
 template <class T>
 __device__ __forceinline__ void cta_gemm_plain(int n, int ta, int tb, int loA, int loB, T alpha, const T* A,
                                                const T* B, T beta, T* C, int loC = 0) {
-  if (n <= 24) cta_gemm_r<T, 2>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC);
+  if (sizeof(T) == 8 || n <= 24) cta_gemm_r<T, 2>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC);
   else cta_gemm_r<T, 4>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC);
 }
 
@@ -224,30 +268,123 @@ __device__ void cta_gemm(int n, int ta, int tb, int loA, int loB, T alpha, const
 // only the lower triangle is read.  Returns false (on every thread) if a
 // pivot is not positive and finite, as LAPACK potrf (src/blocks.jl:94-100,
 // src/schur_solvers.jl:15-19).  `flag` is a shared int.
+//
+// Eight columns at a time: warp 0 factors the 8 x 8 diagonal block in
+// registers, a thread per row solves the panel below, then 4 x 4 (float) or
+// 2 x 2 (double) tiles of the trailing triangle take all eight columns'
+// update.  Every entry sees the same operations in the same order as column
+// by column (multiply-adds by ascending column, then the multiplication by
+// the reciprocal pivot).  Three barriers per eight columns instead of 24, and
+// no index divisions over the whole square: the double Schur factorizations
+// of a three-iteration slice took 11 million clocks at m = 127, now 2.7.
+template <class T> __device__ __forceinline__ void chol_pivot(T d, T& root, T& inv);
+template <> __device__ __forceinline__ void chol_pivot<float>(float d, float& root, float& inv) {
+  root = sqrtf(d);
+  inv = 1.0f / root;
+}
+template <> __device__ __forceinline__ void chol_pivot<double>(double d, double& root, double& inv) {
+  if (__double2hiint(d) < 0x00100000) {  // subnormal
+    root = sqrt(d);
+    inv = 1.0 / root;
+    return;
+  }
+  // root and reciprocal as sqrt and a division round them, by one residual
+  // correction each (Markstein 1990): about 700 clocks instead of 1500
+  fast_root(d, root, inv);
+  inv = fma(fma(-root, inv, 1.0), inv, inv);
+}
+__device__ __forceinline__ bool pivot_ok(double d) {
+  const long long b = __double_as_longlong(d);
+  return b > 0 && b < 0x7FF0000000000000ll;
+}
+__device__ __forceinline__ bool pivot_ok(float d) {
+  const int b = __float_as_int(d);
+  return b > 0 && b < 0x7F800000;
+}
 template <class T>
 __device__ bool cta_potrf(int n, T* a, int lda, int* flag) {
+  constexpr int KB = 8, R = sizeof(T) == 8 ? 2 : 4;
+  __shared__ T L11[KB][KB], rinv[KB];  // L11[k][c] = L(c, k)
   if (threadIdx.x == 0) *flag = 0;
   __syncthreads();
-  for (int k = 0; k < n; ++k) {
-    T* colk = a + (int64_t)k * lda;
-    if (threadIdx.x == 0) {
-      T d = colk[k];
-      if (!(d > (T)0) || !Num<T>::finite(d)) *flag = 1;
-      else colk[k] = Num<T>::sqrt_(d);
+  for (int k0 = 0; k0 < n; k0 += KB) {
+    const int kb = min(KB, n - k0);
+    if (threadIdx.x < 32) {
+      const int r = threadIdx.x;
+      T x[KB];
+#pragma unroll
+      for (int c = 0; c < KB; ++c)
+        x[c] = (r < kb && c <= r) ? a[(k0 + r) + (int64_t)(k0 + c) * lda] : (r == c ? (T)1 : (T)0);
+      bool bad = false;
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        T d = __shfl_sync(0xffffffffu, x[k], k);
+        if (!pivot_ok(d)) {
+          bad = true;
+          d = (T)1;
+        }
+        T root, inv;
+        chol_pivot<T>(d, root, inv);
+        const T l = r == k ? root : x[k] * inv;
+        x[k] = l;
+        if (r < KB) L11[k][r] = l;
+        if (r == k) rinv[k] = inv;
+#pragma unroll
+        for (int c = k + 1; c < KB; ++c) x[c] = fma(-l, __shfl_sync(0xffffffffu, l, c), x[c]);
+      }
+      if (bad) *flag = 1;
+#pragma unroll
+      for (int c = 0; c < KB; ++c)
+        if (r < kb && c <= r) a[(k0 + r) + (int64_t)(k0 + c) * lda] = x[c];
     }
     __syncthreads();
     if (*flag) return false;
-    const T inv = (T)1 / colk[k];
-    for (int i = k + 1 + threadIdx.x; i < n; i += NTHREADS) colk[i] *= inv;
-    __syncthreads();
-    const int m = n - k - 1;
-    const int mm = m * m;
-    for (int idx = threadIdx.x; idx < mm; idx += NTHREADS) {
-      const int ii = idx % m, jj = idx / m;
-      if (ii >= jj) {
-        const int i = k + 1 + ii, j = k + 1 + jj;
-        a[i + (int64_t)j * lda] = fma(-colk[i], colk[j], a[i + (int64_t)j * lda]);
+    const int m0 = k0 + kb, m = n - m0;
+    if (m <= 0) break;
+    for (int i = m0 + threadIdx.x; i < n; i += NTHREADS) {
+      T x[KB];
+#pragma unroll
+      for (int c = 0; c < KB; ++c) x[c] = a[i + (int64_t)(k0 + c) * lda];
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        x[k] *= rinv[k];
+#pragma unroll
+        for (int c = k + 1; c < KB; ++c) x[c] = fma(-x[k], L11[k][c], x[c]);
       }
+#pragma unroll
+      for (int c = 0; c < KB; ++c) a[i + (int64_t)(k0 + c) * lda] = x[c];
+    }
+    __syncthreads();
+    const int nb = (m + R - 1) / R, tiles = nb * (nb + 1) / 2;
+    const T* P = a + m0 + (int64_t)k0 * lda;  // panel rows
+    for (int t = threadIdx.x; t < tiles; t += NTHREADS) {
+      int ti, tj;
+      tri_index(t, ti, tj);
+      const int i0 = ti * R, j0 = tj * R;
+      T acc[R][R];
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < R; ++c)
+          acc[r][c] = (i0 + r < m && j0 + c <= i0 + r) ? a[(m0 + i0 + r) + (int64_t)(m0 + j0 + c) * lda] : (T)0;
+#pragma unroll
+      for (int k = 0; k < KB; ++k) {
+        T li[R], lj[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          li[r] = i0 + r < m ? P[i0 + r + (int64_t)k * lda] : (T)0;
+          lj[r] = j0 + r < m ? P[j0 + r + (int64_t)k * lda] : (T)0;
+        }
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+#pragma unroll
+          for (int c = 0; c < R; ++c) acc[r][c] = fma(-li[r], lj[c], acc[r][c]);
+      }
+#pragma unroll
+      for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int c = 0; c < R; ++c)
+          if (i0 + r < m && j0 + c <= i0 + r) a[(m0 + i0 + r) + (int64_t)(m0 + j0 + c) * lda] = acc[r][c];
     }
     __syncthreads();
   }
@@ -419,8 +556,121 @@ __device__ bool cta_jacobi_svd_g(int n, T* M, T* B, T* sigma, int max_sweeps, in
   return converged;
 }
 
+// The double version: eight lanes per column pair at every order, and only
+// what needs FP64 in FP64.  A FP64 instruction holds its quarter of the SM for
+// 64 clocks whatever the lanes do, so four pairs share a warp's instructions;
+// the rotation test and the angle are formed in FP32 (from the FP64 sums, by
+// their bits), and c comes from the angle by a series (|t| < 1e-4, where the
+// polishing sweeps are) or a corrected FP32 reciprocal root.  About 26 FP64
+// instructions a pair at n = 64 where the generic version has 90, among them
+// two square roots, two divisions and a reciprocal root: 48 million clocks of
+// a three-iteration slice before (FP32 start included), 24 now.
+// Rounds to FP32 by truncation, scaled by 2^-e.
+__device__ __forceinline__ float bits_to_float(double v, int e) {
+  const long long b = __double_as_longlong(v);
+  const int field = ((int)(b >> 52) & 0x7FF) - 1023 - e + 127;
+  if (field <= 0) return 0.0f;
+  const int mag = field >= 255 ? 0x7F7FFFFF : (field << 23) | ((int)(b >> 29) & 0x7FFFFF);
+  return __int_as_float(mag | ((int)(b >> 32) & 0x80000000));
+}
+template <int DUMMY = 0>
+__device__ bool cta_jacobi_svd_f64(int n, double* M, double* B, double* sigma, int max_sweeps, int* counter,
+                                   int* sweeps_out) {
+  constexpr int G = 8, NG = NTHREADS / G;
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), group = threadIdx.x / G;
+  const int N = (n % 2 == 0) ? n : n + 1;
+  const float tol = sqrtf((float)n) * 2.220446e-16f, big_tol = sqrtf(tol);
+  bool converged = (n <= 1);
+  int sweep = 0;
+  for (; sweep < max_sweeps && !converged; ++sweep) {
+    int rotated = 0, big = 0;
+    const int slots = (N / 2 + NG - 1) / NG;  // the same for every group: shuffles stay uniform
+    for (int r = 0; r < N - 1; ++r) {
+      for (int sidx = 0; sidx < slots; ++sidx) {
+        const int k = group + sidx * NG;
+        int p = -1, q = -1;
+        if (k < N / 2) {
+          if (k == 0) { p = N - 1; q = r; }
+          else { p = (r + k) % (N - 1); q = (r - k + (N - 1)) % (N - 1); }
+          if (p >= n || q >= n) p = q = -1;
+        }
+        double* mp = M + (int64_t)(p < 0 ? 0 : p) * n;
+        double* mq = M + (int64_t)(p < 0 ? 0 : q) * n;
+        double app = 0.0, aqq = 0.0, apq = 0.0;
+        if (p >= 0) {
+#pragma unroll 4
+          for (int i = gl; i < n; i += G) {
+            const double x = mp[i], y = mq[i];
+            app = fma(x, x, app); aqq = fma(y, y, aqq); apq = fma(x, y, apq);
+          }
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) {
+          app += __shfl_xor_sync(0xffffffffu, app, o);
+          aqq += __shfl_xor_sync(0xffffffffu, aqq, o);
+          apq += __shfl_xor_sync(0xffffffffu, apq, o);
+        }
+        // scaled by the larger of the two norms' exponents
+        const int e = max((__double2hiint(app) >> 20) & 0x7FF, (__double2hiint(aqq) >> 20) & 0x7FF) - 1023;
+        const float fp = bits_to_float(app, e), fq = bits_to_float(aqq, e), fpq = bits_to_float(apq, e);
+        const float scale = sqrtf(fp) * sqrtf(fq);
+        if (p >= 0 && e < 1024 && fabsf(fpq) > tol * scale) {  // e = 1024: infinite or NaN
+          if (fabsf(fpq) > big_tol * scale) big = 1;
+          // the angle only needs float accuracy (the next sweep removes what
+          // is left); c and s are formed in FP64 so the rotation is orthogonal
+          // to its rounding
+          const float zf = bits_to_float(aqq - app, e) / (2.0f * fpq);
+          const float tf = (zf >= 0.0f ? 1.0f : -1.0f) / (fabsf(zf) + sqrtf(1.0f + zf * zf));
+          const double t = (double)tf, t2 = t * t;
+          double c;
+          if (fabsf(tf) < 1e-4f) {
+            c = fma(t2, fma(t2, 0.375, -0.5), 1.0);
+          } else {
+            const double x = 1.0 + t2, y = (double)rsqrtf((float)x), d = fma(-x * y, y, 1.0);
+            c = fma(y * d, fma(0.375, d, 0.5), y);
+          }
+          const double sn = c * t;
+          double* bp = B + (int64_t)p * n;
+          double* bq = B + (int64_t)q * n;
+#pragma unroll 2
+          for (int i = gl; i < n; i += G) {
+            const double x = mp[i], y = mq[i], u = bp[i], v = bq[i];
+            mp[i] = fma(c, x, -(sn * y));
+            mq[i] = fma(sn, x, c * y);
+            bp[i] = fma(c, u, -(sn * v));
+            bq[i] = fma(sn, u, c * v);
+          }
+          rotated = 1;
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+    }
+    rotated = __syncthreads_or(rotated);
+    big = __syncthreads_or(big);
+    // quadratic convergence, as in the generic version
+    converged = !rotated || !big;
+  }
+  *sweeps_out = sweep;
+  const int nslots = (n + NG - 1) / NG;
+  for (int sidx = 0; sidx < nslots; ++sidx) {
+    const int k = group + sidx * NG;
+    double s = 0.0;
+    if (k < n) {
+      const double* mk = M + (int64_t)k * n;
+      for (int i = gl; i < n; i += G) s = fma(mk[i], mk[i], s);
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (k < n && gl == 0) sigma[k] = sqrt(s);
+  }
+  __syncthreads();
+  return converged;
+}
+
 template <class T>
 __device__ bool cta_jacobi_svd(int n, T* M, T* B, T* sigma, int max_sweeps, int* counter, int* sweeps_out) {
+  if constexpr (sizeof(T) == 8) return cta_jacobi_svd_f64(n, M, B, sigma, max_sweeps, counter, sweeps_out);
   if (n <= 16) return cta_jacobi_svd_g<T, 8>(n, M, B, sigma, max_sweeps, counter, sweeps_out);
   if (n <= 48) return cta_jacobi_svd_g<T, 16>(n, M, B, sigma, max_sweeps, counter, sweeps_out);
   return cta_jacobi_svd_g<T, 32>(n, M, B, sigma, max_sweeps, counter, sweeps_out);
@@ -673,6 +923,216 @@ __device__ T warp_lanczos_eigmin(int n, const T* Z, T* Qs, int kq, T* Qg, T* a, 
     }
     __syncwarp();
   }
+  *steps = k;
+  return theta;
+}
+
+// Shared state of cta_lanczos_min.
+struct LanczosShared {
+  TridiagShared tri;
+  double red[NWARPS];
+  int state, stop;
+};
+
+// Smallest eigenvalue of the symmetric Z (n x n, n <= 256) in float64 by
+// Lanczos with full reorthogonalization, run by the whole CTA: the iteration
+// of warp_lanczos_eigmin (start vector, two passes against the whole basis,
+// Ritz value every 4 steps until it moves by at most 64 eps) with the sums
+// split over all threads as (output, part) pairs, the norm taken from the
+// second pass's w'w, and the Ritz value looked at in FP32 before the FP64 one
+// is formed (tridiag.cuh).  Z, the basis and the vectors live in shared memory
+// as far as they fit (all of it up to n = 64); the rest of the basis in Qg.
+// One warp per matrix kept one quarter of the SM busy and spent a division per
+// row of every Sturm count: 34 million clocks of a three-iteration slice at
+// n = 64 (three CTAs an SM), 8 million with this.
+__device__ inline double cta_lanczos_min(int n, const double* Zg, double* Qg, unsigned char* smem, int64_t smem_bytes,
+                                         LanczosShared& sh, int* steps) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  double* qs = (double*)smem;      // [n]
+  double* ws = qs + n;             // [n]
+  double* part = ws + n;           // [NTHREADS]
+  double* coef = part + NTHREADS;  // [n + 2] each
+  double* al = coef + n + 2;
+  double* be = al + n + 2;
+  double* sa = be + n + 2;
+  double* sb = sa + n + 2;
+  float* saf = (float*)(sb + n + 2);
+  float* sbf = saf + n + 2;
+  double* rest = (double*)(sbf + n + 2);
+  int64_t room = smem_bytes / 8 - (rest - qs);
+  const double* Z = Zg;
+  if ((int64_t)n * n <= room) {
+    for (int k = t; k < n * n; k += NTHREADS) rest[k] = Zg[k];
+    Z = rest;
+    rest += (int64_t)n * n;
+    room -= (int64_t)n * n;
+  }
+  const int kq = (int)(room > 0 ? room / n : 0);
+  auto Qc = [&](int l) -> double* { return l < kq ? rest + (int64_t)l * n : Qg + (int64_t)l * n; };
+  // start vector
+  double nrm2 = 0.0;
+  for (int i = t; i < n; i += NTHREADS) {
+    uint32_t h = (uint32_t)(i + 1) * 2654435761u;
+    h ^= h >> 15; h *= 2246822519u; h ^= h >> 13;
+    const double v = (double)(h & 0xffffff) / 16777216.0 - 0.5 + 0.01;
+    qs[i] = v;
+    nrm2 = fma(v, v, nrm2);
+  }
+  nrm2 = warp_sum(nrm2);
+  if (lane == 0) sh.red[warp] = nrm2;
+  if (t == 0) be[0] = 0.0;
+  __syncthreads();
+  {
+    double s = 0.0;
+#pragma unroll
+    for (int w = 0; w < NWARPS; ++w) s += sh.red[w];
+    double root, inv;
+    fast_root(s, root, inv);
+    for (int i = t; i < n; i += NTHREADS) {
+      const double v = qs[i] * inv;
+      qs[i] = v;
+      Qc(0)[i] = v;
+    }
+  }
+  __syncthreads();
+  const int U = n <= 32 ? 4 : n <= 64 ? 2 : 1;  // parts of a row's sum
+  double theta = 0.0, theta_prev = INFINITY, znorm = 0.0;
+  float theta32_prev = INFINITY;
+  bool have_prev = false;
+  int k = 0;
+  for (int j = 0; j < n; ++j) {
+    // ---- w = Z q
+    if (U > 1) {
+      const int i = t % n, u = t / n;
+      if (u < U) {
+        double s = 0.0;
+#pragma unroll 4
+        for (int r = u * n / U; r < (u + 1) * n / U; ++r) s = fma(Z[(int64_t)r * n + i], qs[r], s);
+        part[t] = s;
+      }
+      __syncthreads();
+      if (t < n) {
+        double s = part[t];
+        for (int v = 1; v < U; ++v) s += part[v * n + t];
+        ws[t] = s;
+      }
+    } else {
+      for (int i = t; i < n; i += NTHREADS) {
+        double s = 0.0;
+#pragma unroll 8
+        for (int r = 0; r < n; ++r) s = fma(Z[(int64_t)r * n + i], qs[r], s);
+        ws[i] = s;
+      }
+    }
+    __syncthreads();
+    // ---- two passes against q_0 .. q_j; the second one's last output is w'w
+    const int L = j + 1;
+    bool large = false;
+    for (int pass = 0; pass < 2; ++pass) {
+      const int LL = L + pass;
+      int C = 16;  // neighbouring lanes of one coefficient
+      while (C > 1 && C * LL > NTHREADS) C >>= 1;
+      for (int l0 = 0; l0 < LL; l0 += NTHREADS / C) {
+        const int l = l0 + t / C, c = t & (C - 1);
+        double s = 0.0;
+        if (l < LL) {
+          const double* q = l < L ? Qc(l) : ws;
+#pragma unroll 4
+          for (int i = c; i < n; i += C) s = fma(q[i], ws[i], s);
+        }
+        for (int o = C >> 1; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (c == 0 && l < LL) coef[l] = s;
+      }
+      __syncthreads();
+      if (pass == 0 && t == 0) al[j] = coef[j];
+      if (U > 1) {
+        const int i = t % n, u = t / n;
+        if (u < U) {
+          double s = 0.0;
+#pragma unroll 4
+          for (int l = u * L / U; l < (u + 1) * L / U; ++l) s = fma(-coef[l], Qc(l)[i], s);
+          part[t] = s;
+        }
+        __syncthreads();
+        if (t < n) {
+          double s = part[t];
+          for (int v = 1; v < U; ++v) s += part[v * n + t];
+          ws[t] += s;
+        }
+      } else {
+        for (int i = t; i < n; i += NTHREADS) {
+          double s = ws[i];
+#pragma unroll 4
+          for (int l = 0; l < L; ++l) s = fma(-coef[l], Qc(l)[i], s);
+          ws[i] = s;
+        }
+      }
+      if (pass == 1) {
+        // a coefficient above 2^-30 |w'| changes the norm
+        const int en = (__double2hiint(coef[L]) >> 20) - 1023;
+        int ec = -2000;
+        for (int l = t; l < L; l += NTHREADS) ec = max(ec, ((__double2hiint(coef[l]) >> 20) & 0x7ff) - 1023);
+        large = __syncthreads_or(2 * ec > en - 60);
+      } else {
+        __syncthreads();
+      }
+    }
+    k = L;
+    double bn2 = coef[L];
+    if (large)
+      for (int l = 0; l < L; ++l) bn2 = fma(-coef[l], coef[l], bn2);
+    const int field = __double2hiint(bn2) >> 20;  // 0x7ff: infinite or NaN; below 27: 1e-300 or negative
+    double bn = 0.0, binv = 0.0;
+    if (field > 27 && field < 0x7ff) fast_root(bn2, bn, binv);
+    if (k < n) {
+      double* qn = Qc(k);
+      for (int i = t; i < n; i += NTHREADS) {
+        const double q = ws[i] * binv;
+        qn[i] = q;
+        qs[i] = q;
+      }
+    }
+    if (t == 0) {
+      const double aj = al[j], bj = j > 0 ? be[j] : 0.0;
+      znorm = fmax(znorm, fabs(aj) + bn + fabs(bj));
+      be[k] = bn;
+      const bool bad = field == 0x7ff || (__double2hiint(aj) & 0x7ff00000) == 0x7ff00000;
+      sh.state = bad ? 2 : !(bn > 4.0 * 2.220446049250313e-16 * znorm) ? 1 : 0;
+    }
+    __syncthreads();
+    if (sh.state == 2) {
+      theta = nan("");
+      break;
+    }
+    const bool exhausted = k == n || sh.state == 1;
+    if (exhausted || (k >= 4 && (k & 3) == 0)) {
+      const int e = tridiag_scale(k, al, be, sa, sb, saf, sbf, sh.tri);
+      const float th32 = tridiag_min32(k, saf, sbf, sh.tri);  // in units of 2^e
+      const float here = ldexpf(th32, e);
+      if (exhausted) {
+        theta = tridiag_min64(k, sa, sb, th32, e, sh.tri);
+        break;
+      }
+      if (fabsf(here - theta32_prev) <= 3e-6f * ldexpf(1.0f, e)) {
+        theta = tridiag_min64(k, sa, sb, th32, e, sh.tri);
+        if (!have_prev) {
+          const double th = theta;
+          __syncthreads();
+          theta_prev = tridiag_min64(k - 4, sa, sb, ldexpf(theta32_prev, -e), e, sh.tri);
+          theta = th;
+        }
+        if (t == 0) sh.stop = fabs(theta - theta_prev) <= 64.0 * 2.220446049250313e-16 * fmax(1.0, fabs(theta));
+        __syncthreads();
+        if (sh.stop) break;
+        theta_prev = theta;
+        have_prev = true;
+      } else {
+        have_prev = false;
+      }
+      theta32_prev = here;
+    }
+  }
+  __syncthreads();
   *steps = k;
   return theta;
 }
