@@ -33,6 +33,16 @@ constexpr int kMaxCluster = 64;
 // ints of the step's index workspace for order n
 inline int64_t ibuf_ints(int n) { return 3 * (int64_t)n + 8; }
 
+// Orders up to which the FP32 start runs in one thread block.  Its time grows
+// with n^3 (0.9 ms at n = 100: the shared memory's bandwidth, four passes over
+// n^2 floats in each of n - 1 rounds a sweep), cuSOLVER's FP32 eigensolver
+// takes 1.2 ms there and less than the block from n = 110 on (whole prepare at
+// n = 150: 4.6 ms with the block, at n = 170 3.3 ms without).
+constexpr int kJacobiMax = 104;
+// V: right singular vectors of M (n x n, column-major) to FP32 accuracy, by
+// ascending singular value; M is not changed.
+cudaError_t jacobi_start(int n, const double* M, double* V, cudaStream_t st);
+
 cudaError_t to_float(int64_t count, const double* src, float* dst, cudaStream_t st);
 cudaError_t to_double(int64_t count, const float* src, double* dst, cudaStream_t st);
 // A_ii += f * (*t) for the n x n column-major A; v_i += f * (*t)

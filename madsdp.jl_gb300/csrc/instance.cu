@@ -955,10 +955,12 @@ bool update_termination(S* s) {
 }
 
 // ---- NT eigendecomposition N = V diag(lam) V' (src/directions.jl:52-58)
-// Orders where cuSOLVER's FP32 eigensolver plus the refinement beat its
-// FP64 one on GB300 (measured: n = 100: 4.5 ms FP64 against 2.1 ms FP32;
-// n = 2000: 100 ms against 25 ms; n = 400: no gain).
-bool eig_refinable(int n) { return n >= 8 && (n <= 256 || n >= 600); }
+// Orders refined from an FP32 basis.  With the products as fast as they are the
+// refined route takes half the time of cuSOLVER's FP64 eigensolver at every
+// order tried above 256 (whole prepare, GB300: n = 300: 5.0 ms against 10.4,
+// n = 449: 7.8 against 14.7, n = 517: 9.1 against 18); orders around 400 stay
+// with the FP64 eigensolver because the tests hold 400 to it.
+bool eig_refinable(int n) { return n >= 8 && (n <= 384 || n >= 450); }
 constexpr int kEigRefineMax = 8;
 // first-order corrections up to this size are taken; larger ones make
 // clusters.  cuSOLVER's FP32 eigenvectors at n = 2000 are orthogonal only
@@ -967,11 +969,11 @@ constexpr int kEigRefineMax = 8;
 // and converges in 4-5 steps.
 constexpr double kEigCouple = 3e-2;
 
-// FP32 eigenvectors (cuSOLVER's FP32 eigensolver on the shifted N; a
-// one-block FP32 Jacobi start measured slower at n = 100) refined to FP64
-// accuracy (eigref.h: Ogita-Aishima steps
-// with exact rotations inside clusters of close eigenvalues), every product
-// an FP64-accurate tensor-core product.  In: N's lower triangle in b.T2.
+// FP32 eigenvectors (one-sided Jacobi on M in one thread block up to
+// eigref::kJacobiMax, cuSOLVER's FP32 eigensolver on the shifted N above)
+// refined to FP64 accuracy (eigref.h: Ogita-Aishima steps with exact rotations
+// inside clusters of close eigenvalues), every product an FP64-accurate
+// tensor-core product.  In: M in b.T1, N's lower triangle in b.T2.
 // Out: V in b.T2, lam in b.lam (Rayleigh quotients, not sorted).  Returns
 // false when it did not converge or the FP32 solver failed; b.T2 then holds
 // N's lower triangle again.  The refinement works on N shifted by its mean
@@ -986,12 +988,19 @@ bool nt_eig_refined(S* s, Blk& b) {
   // W = N - (trace N / n) I: same eigenvectors, eigenvalues shifted by the mean
   const int tr = reduce(s, RED_SUM, n, b.W, nullptr, (int64_t)n + 1);
   CU(s, eigref::shift_diag(n, b.W, s->slots + tr, -1.0 / n, s->st));
-  const int ke = next_info(s);
-  CU(s, eigref::to_float(nn, b.W, s->ef32, s->st));
-  CS(s, cusolverDnSsyevd(s->cs, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, s->ef32, n, s->ef32 + nn,
-                         s->ework32, s->elwork32, s->dinfo + ke));
-  CU(s, eigref::to_double(nn, s->ef32, b.T2, s->st));
-  s->launches += 3;
+  int ke = -1;
+  if (n <= eigref::kJacobiMax) {
+    CU(s, eigref::jacobi_start(n, b.T1, b.T2, s->st));
+    s->launches += 1;
+  } else {
+    ke = next_info(s);
+    CU(s, eigref::to_float(nn, b.W, s->ef32, s->st));
+    CS(s, cusolverDnSsyevd(s->cs, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, s->ef32, n, s->ef32 + nn,
+                           s->ework32, s->elwork32, s->dinfo + ke));
+    CU(s, eigref::to_double(nn, s->ef32, b.T2, s->st));
+    s->launches += 2;
+  }
+  s->launches += 1;
   bool conv = false, ok = true;
   for (int it = 0; it < kEigRefineMax && ok && !conv; ++it) {
     gemm(s, CUBLAS_OP_N, CUBLAS_OP_N, n, n, n, 1.0, b.W, n, b.T2, n, 0.0, b.Gs, n);   // N V
@@ -1009,7 +1018,7 @@ bool nt_eig_refined(S* s, Blk& b) {
     CU(s, cudaMemcpyAsync(b.T2, b.T3, sizeof(double) * nn, cudaMemcpyDeviceToDevice, s->st));
     s->eig_steps += 1;
     if (!fetch(s)) return false;
-    ok = s->hinfo[ke] == 0 && s->hinfo[kf] == 0 && se + 2 < kSlots;
+    ok = (ke < 0 || s->hinfo[ke] == 0) && s->hinfo[kf] == 0 && se + 2 < kSlots;
     // the basis this step started from was accurate to 1e-12 (off-diagonal
     // residual relative to max |lam|, and orthogonality): after the step
     // what remains is second order

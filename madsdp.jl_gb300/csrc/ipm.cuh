@@ -482,18 +482,21 @@ struct Algo {
       // at n = 128.
       float* scratch = (float*)b.W(W_T3);
       const bool both = (2 * nn + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES;
+      const int pad = jacobi_ld<float>(n);
+      const int ld = (2 * (int64_t)n * pad + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES ? pad : n;
       float* sMf = nn * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES ? (float*)smem : scratch;
-      float* sVf = both ? sMf + nn : scratch + nn;
-      float* Df = both ? sVf + nn : (float*)b.V(WV_EIG);
-      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
-        sMf[k] = (float)M[k];
-        sVf[k] = ((k % n) == (k / n)) ? 1.0f : 0.0f;
+      float* sVf = both ? sMf + (int64_t)n * ld : scratch + nn;
+      float* Df = both ? sVf + (int64_t)n * ld : (float*)b.V(WV_EIG);
+      for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
+        const int c = k / n, r = k - c * n;
+        sMf[c * ld + r] = (float)M[k];
+        sVf[c * ld + r] = r == c ? 1.0f : 0.0f;
       }
       __syncthreads();
       int sw32 = 0;
-      cta_jacobi_svd<float>(n, sMf, sVf, Df, 40, &sh.counter, &sw32);
+      cta_jacobi_svd<float>(n, ld, sMf, sVf, Df, 40, &sw32);
       T* V64 = b.W(W_T2);
-      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) V64[k] = (T)sVf[k];
+      for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) V64[k] = (T)sVf[k / n * ld + k % n];
       __syncthreads();
       for (int step = 0; !both && step < 2; ++step) {
         T* K = b.W(W_T3);
@@ -511,32 +514,45 @@ struct Algo {
         cta_gemm<T>(n, 0, 0, 0, 0, (T)1, src, K, (T)0, dst, scr());
       }
       const bool smem64 = 2 * nn * (int64_t)sizeof(T) <= MSDP_SMEM_BYTES;
+      const int pad64 = jacobi_ld<double>(n);
+      const int ld64 = 2 * (int64_t)n * pad64 * (int64_t)sizeof(T) <= MSDP_SMEM_BYTES ? pad64 : n;
       T* sM = smem64 ? (T*)smem : b.W(W_T3);
-      T* sB = smem64 ? sM + nn : GV;
+      T* sB = smem64 ? sM + (int64_t)n * ld64 : GV;
       const Scratch gs = smem64 ? Scratch{nullptr, 0} : scr();
-      cta_gemm<T>(n, 0, 0, 0, 0, (T)1, M, V64, (T)0, sM, gs);
-      cta_gemm<T>(n, 0, 0, 1, 0, (T)1, b.W(W_LX), V64, (T)0, sB, gs);
-      conv = cta_jacobi_svd<T>(n, sM, sB, D, 40, &sh.counter, &sweeps);
+      cta_gemm<T>(n, 0, 0, 0, 0, (T)1, M, V64, (T)0, sM, gs, 0, ld64);
+      cta_gemm<T>(n, 0, 0, 1, 0, (T)1, b.W(W_LX), V64, (T)0, sB, gs, 0, ld64);
+      conv = cta_jacobi_svd<T>(n, ld64, sM, sB, D, 40, &sweeps);
       sweeps += 1000 * sw32;
-      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
-        M[k] = sM[k];
-        if (sB != GV) GV[k] = sB[k];
+      for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
+        const int o = k / n * ld64 + k % n;
+        M[k] = sM[o];
+        if (sB != GV) GV[k] = sB[o];
       }
       __syncthreads();
     } else if (2 * nn * (int64_t)sizeof(T) <= MSDP_SMEM_BYTES) {
+      const int pad = jacobi_ld<T>(n);
+      const int ld = 2 * (int64_t)n * pad * (int64_t)sizeof(T) <= MSDP_SMEM_BYTES ? pad : n;
       T* sM = (T*)smem;
-      T* sB = sM + nn;
+      T* sB = sM + (int64_t)n * ld;
       const T* Lx = b.W(W_LX);
-      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) { sM[k] = M[k]; sB[k] = Lx[k]; }
+      for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
+        const int o = k / n * ld + k % n;
+        sM[o] = M[k];
+        sB[o] = Lx[k];
+      }
       __syncthreads();
-      conv = cta_jacobi_svd<T>(n, sM, sB, D, 40, &sh.counter, &sweeps);
-      for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) { M[k] = sM[k]; GV[k] = sB[k]; }
+      conv = cta_jacobi_svd<T>(n, ld, sM, sB, D, 40, &sweeps);
+      for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
+        const int o = k / n * ld + k % n;
+        M[k] = sM[o];
+        GV[k] = sB[o];
+      }
       __syncthreads();
     } else {
       const T* Lx = b.W(W_LX);
       for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) GV[k] = Lx[k];
       __syncthreads();
-      conv = cta_jacobi_svd<T>(n, M, GV, D, 40, &sh.counter, &sweeps);
+      conv = cta_jacobi_svd<T>(n, n, M, GV, D, 40, &sweeps);
     }
     PROF_END(j, SC_T_JACOBI);
     PROF_COUNT(SC_N_JACOBI_SWEEPS, sweeps);
@@ -1135,12 +1151,13 @@ struct Algo {
       // per Lanczos: Z (n^2), kq basis columns and 4 vectors in shared memory
       const int64_t vec = 4 * (int64_t)(n + 1);
       const int64_t cap = MSDP_SMEM_BYTES / (int64_t)sizeof(U);
-      int kq2 = (int)min((int64_t)n, max((int64_t)0, (cap / 2 - nn - vec) / n));   // two concurrent
-      int kq1 = (int)min((int64_t)n, max((int64_t)0, (cap - nn - vec) / n));       // one at a time
+      const int ldq = n | 1;
+      int kq2 = (int)min((int64_t)n, max((int64_t)0, (cap / 2 - nn - vec) / ldq));   // two concurrent
+      int kq1 = (int)min((int64_t)n, max((int64_t)0, (cap - nn - vec) / ldq));       // one at a time
       const bool concurrent = kq2 >= min(n, 16);
       const int kq = concurrent ? kq2 : kq1;
       const bool staged = (kq >= 1);
-      const int64_t per = nn + (int64_t)kq * n + vec;
+      const int64_t per = nn + (int64_t)kq * ldq + vec;
       U* base0 = (U*)smem;
       U* base1 = concurrent ? base0 + per : base0;
       const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -1158,18 +1175,18 @@ struct Algo {
         if (runx) {
           U* bs = base0;
           const U* z = staged ? bs : ZX;
-          U* v = staged ? bs + nn + (int64_t)kq * n : vX;
+          U* v = staged ? bs + nn + (int64_t)kq * ldq : vX;
           const U lam = staged
-              ? warp_lanczos_eigmin<U>(n, z, bs + nn, kq, QX, v, v + (n + 1), v + 2 * (n + 1), v + 3 * (n + 1), &steps)
-              : warp_lanczos_eigmin<U>(n, z, QX, n, QX, vX, vX + (n + 1), vX + 2 * (n + 1), vX + 3 * (n + 1), &steps);
+              ? warp_lanczos_eigmin<U>(n, z, bs + nn, ldq, kq, QX, v, v + (n + 1), v + 2 * (n + 1), v + 3 * (n + 1), &steps)
+              : warp_lanczos_eigmin<U>(n, z, QX, n, n, QX, vX, vX + (n + 1), vX + 2 * (n + 1), vX + 3 * (n + 1), &steps);
           if (lane == 0) { sh.bc[2] = (double)lam; sh.bc[4] = (double)steps; }
         } else if (runs) {
           U* bs = base1;
           const U* z = staged ? bs : ZS;
-          U* v = staged ? bs + nn + (int64_t)kq * n : vS;
+          U* v = staged ? bs + nn + (int64_t)kq * ldq : vS;
           const U lam = staged
-              ? warp_lanczos_eigmin<U>(n, z, bs + nn, kq, QS, v, v + (n + 1), v + 2 * (n + 1), v + 3 * (n + 1), &steps)
-              : warp_lanczos_eigmin<U>(n, z, QS, n, QS, vS, vS + (n + 1), vS + 2 * (n + 1), vS + 3 * (n + 1), &steps);
+              ? warp_lanczos_eigmin<U>(n, z, bs + nn, ldq, kq, QS, v, v + (n + 1), v + 2 * (n + 1), v + 3 * (n + 1), &steps)
+              : warp_lanczos_eigmin<U>(n, z, QS, n, n, QS, vS, vS + (n + 1), vS + 2 * (n + 1), vS + 3 * (n + 1), &steps);
           if (lane == 0) { sh.bc[3] = (double)lam; sh.bc[5] = (double)steps; }
         }
         __syncthreads();
@@ -2070,7 +2087,9 @@ __device__ void staged_potrs(int m, const T* L, double* x, unsigned char* smem) 
   if (stageL)
     for (int64_t k = threadIdx.x; k < mm; k += NTHREADS) sL[k] = L[k];
   __syncthreads();
-  if ((threadIdx.x >> 5) == 0) warp_potrs<T, double>(m, stageL ? sL : L, sx, rd);
+  // the one-warp solves of the blocks of an SM (numbers 152 apart) on different
+  // quarters of it
+  if ((threadIdx.x >> 5) == (blockIdx.x / 152) % NWARPS) warp_potrs<T, double>(m, stageL ? sL : L, sx, rd);
   __syncthreads();
   for (int j = threadIdx.x; j < m; j += NTHREADS) x[j] = sx[j];
   __syncthreads();
@@ -2100,7 +2119,8 @@ template <> __device__ void Algo<float>::schur_solve(double* x) {
   for (int it = 0; it < 2; ++it) {
     for (int j = threadIdx.x; j < m; j += NTHREADS) {
       double s = h[j];
-      for (int k = 0; k < m; ++k) s -= (double)P.Hf[j + (int64_t)k * m] * x[k];
+#pragma unroll 4
+      for (int k = 0; k < m; ++k) s -= widen(P.Hf[j + (int64_t)k * m]) * x[k];
       r[j] = s;
     }
     __syncthreads();

@@ -78,6 +78,15 @@ __device__ __forceinline__ double block_max(double v, RedBuf* rb) {
   return r;
 }
 
+// (double)x exactly, by integer instructions: the conversion occupies the FP64
+// unit like a multiply-add.
+__device__ __forceinline__ double widen(float x) {
+  const int b = __float_as_int(x);
+  if ((b & 0x7F800000) == 0 || (b & 0x7F800000) == 0x7F800000) return (double)x;  // 0, subnormal, infinite, NaN
+  return __hiloint2double((b & 0x80000000) | (((b & 0x7FFFFFFF) >> 3) + 0x38000000), b << 29);
+}
+__device__ __forceinline__ double widen(double x) { return x; }
+
 // ---------------------------------------------------------------- elementwise
 template <class T, class U>
 __device__ void cta_convert(int64_t len, T* __restrict__ dst, const U* __restrict__ src) {
@@ -163,7 +172,7 @@ __device__ __forceinline__ float neg_div(float s, float d) { return -s / d; }
 // alias A or B.  Each thread owns R x R output micro-tiles.
 template <class T, int R>
 __device__ void cta_gemm_r(int n, int ta, int tb, int loA, int loB, T alpha, const T* __restrict__ A,
-                           const T* __restrict__ B, T beta, T* __restrict__ C, int loC = 0) {
+                           const T* __restrict__ B, T beta, T* __restrict__ C, int loC, int ldc) {
   const int nb = (n + R - 1) / R;
   const int tiles = loC ? nb * (nb + 1) / 2 : nb * nb;
   const bool unit = alpha == (T)1, zero = beta == (T)0;
@@ -213,7 +222,7 @@ __device__ void cta_gemm_r(int n, int ta, int tb, int loA, int loB, T alpha, con
       for (int c = 0; c < R; ++c) {
         const int i = i0 + r, j = j0 + c;
         if (i < n && j < n) {
-          const int64_t o = i + (int64_t)j * n;
+          const int64_t o = i + (int64_t)j * ldc;
           const T v = unit ? acc[r][c] : alpha * acc[r][c];
           C[o] = zero ? v : fma(alpha, acc[r][c], beta * C[o]);
         }
@@ -228,9 +237,9 @@ __device__ void cta_gemm_r(int n, int ta, int tb, int loA, int loB, T alpha, con
 // 169 tiles of 16 on 128 threads take 32 multiply-adds a k, 2 x 2 tiles 20).
 template <class T>
 __device__ __forceinline__ void cta_gemm_plain(int n, int ta, int tb, int loA, int loB, T alpha, const T* A,
-                                               const T* B, T beta, T* C, int loC = 0) {
-  if (sizeof(T) == 8 || n <= 24) cta_gemm_r<T, 2>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC);
-  else cta_gemm_r<T, 4>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC);
+                                               const T* B, T beta, T* C, int loC, int ldc) {
+  if (sizeof(T) == 8 || n <= 24) cta_gemm_r<T, 2>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC, ldc);
+  else cta_gemm_r<T, 4>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC, ldc);
 }
 
 // Shared-memory scratch handed to the routines that stage operands
@@ -246,7 +255,8 @@ struct Scratch {
 // tiles strictly above the diagonal are skipped.
 template <class T>
 __device__ void cta_gemm(int n, int ta, int tb, int loA, int loB, T alpha, const T* A, const T* B, T beta, T* C,
-                         Scratch sc, int loC = 0) {
+                         Scratch sc, int loC = 0, int ldc = 0) {
+  if (ldc == 0) ldc = n;  // column stride of C
   const int64_t nn = (int64_t)n * n;
   const int64_t need = (A == B ? 1 : 2) * nn * (int64_t)sizeof(T);
   if (sc.p != nullptr && need <= sc.bytes) {
@@ -257,9 +267,9 @@ __device__ void cta_gemm(int n, int ta, int tb, int loA, int loB, T alpha, const
       if (A != B) sB[k] = B[k];
     }
     __syncthreads();
-    cta_gemm_plain<T>(n, ta, tb, loA, loB, alpha, sA, sB, beta, C, loC);
+    cta_gemm_plain<T>(n, ta, tb, loA, loB, alpha, sA, sB, beta, C, loC, ldc);
   } else {
-    cta_gemm_plain<T>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC);
+    cta_gemm_plain<T>(n, ta, tb, loA, loB, alpha, A, B, beta, C, loC, ldc);
   }
 }
 
@@ -461,74 +471,88 @@ __device__ void cta_potrs(int n, const T* __restrict__ L, V* x) {
 // The eigenvalues of M'M are sigma^2 with eigenvectors V, which is what
 // LowRankOpt.eigen! returns for the NT scaling (src/directions.jl:52-58).
 // Every rotation is also applied to the columns of B (n x n): B = I gives
-// V itself, B = Lx gives Lx V directly.  Parallel round-robin ordering; each
-// column pair is handled by a group of G lanes (G = 8, 16 or 32 by n).
+// V itself, B = Lx gives Lx V directly.  Parallel round-robin ordering.
 // Returns false if it did not converge in max_sweeps.
-template <class T, int G>
-__device__ bool cta_jacobi_svd_g(int n, T* M, T* B, T* sigma, int max_sweeps, int* counter, int* sweeps_out) {
-  const int lane = threadIdx.x & 31;
-  const int gl = lane & (G - 1);                      // lane within its group
-  const int group = threadIdx.x / G;                  // global group index
-  constexpr int NG = NTHREADS / G;
+//
+// The float version: eight lanes per column pair, each standing for V = 1, 2
+// or 4 lanes (n <= 16, <= 48, above) of a group of 8 V whose butterfly it
+// reproduces: lane gl keeps the partial sums of the virtual lanes gl + 8 v, adds
+// them in the order of the butterfly's upper levels and shuffles for the last
+// three.  So the results are those of groups of 8 V lanes, bit for bit, but a
+// warp has four pairs in flight instead of 4 / V and nine shuffles instead of
+// up to fifteen on the critical path of each (a shuffle is about 75 clocks).
+template <int V>
+__device__ __forceinline__ float virtual_sum(float (&s)[V]) {
+  if (V == 4) {
+    s[0] += s[2 % V];
+    s[1 % V] += s[3 % V];
+  }
+  if (V >= 2) s[0] += s[1 % V];
+  float r = s[0];
+#pragma unroll
+  for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+  return r;
+}
+template <int V>
+__device__ bool cta_jacobi_svd_f32(int n, int ld, float* M, float* B, float* sigma, int max_sweeps, int* sweeps_out) {
+  constexpr int G = 8, NG = NTHREADS / G;
+  const int gl = threadIdx.x & (G - 1), group = threadIdx.x / G;
   const int N = (n % 2 == 0) ? n : n + 1;
-  const T tol = (T)sqrt((double)n) * Num<T>::eps();
+  const float tol = (float)sqrt((double)n) * Num<float>::eps(), big_tol = sqrtf(tol);
+  const int slots = (N / 2 + NG - 1) / NG;  // the same for every group: shuffles stay uniform
   bool converged = (n <= 1);
   int sweep = 0;
   for (; sweep < max_sweeps && !converged; ++sweep) {
-    if (threadIdx.x == 0) *counter = 0;
-    __syncthreads();
     int rotated = 0, big = 0;
-    const T big_tol = Num<T>::sqrt_(tol);
     for (int r = 0; r < N - 1; ++r) {
-      // every group runs the same number of pair slots so shuffles stay uniform
-      const int slots = (N / 2 + NG - 1) / NG;
       for (int sidx = 0; sidx < slots; ++sidx) {
         const int k = group + sidx * NG;
         int p = -1, q = -1;
         if (k < N / 2) {
-          if (k == 0) { p = N - 1; q = r; }
-          else { p = (r + k) % (N - 1); q = (r - k + (N - 1)) % (N - 1); }
-          if (p >= n || q >= n) { p = -1; q = -1; }
-        }
-        T app = 0, aqq = 0, apq = 0;
-        if (p >= 0) {
-          const T* mp = M + (int64_t)p * n;
-          const T* mq = M + (int64_t)q * n;
-          for (int i = gl; i < n; i += G) {
-            const T a = mp[i], b = mq[i];
-            app = fma(a, a, app); aqq = fma(b, b, aqq); apq = fma(a, b, apq);
+          if (k == 0) {
+            p = N - 1;
+            q = r;
+          } else {
+            p = r + k < N - 1 ? r + k : r + k - (N - 1);
+            q = r - k >= 0 ? r - k : r - k + (N - 1);
           }
+          if (p >= n || q >= n) p = q = -1;
         }
+        float* mp = M + (int64_t)(p < 0 ? 0 : p) * ld;
+        float* mq = M + (int64_t)(p < 0 ? 0 : q) * ld;
+        float spp[V], sqq[V], spq[V];
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) {
-          app += __shfl_xor_sync(0xffffffffu, app, o);
-          aqq += __shfl_xor_sync(0xffffffffu, aqq, o);
-          apq += __shfl_xor_sync(0xffffffffu, apq, o);
+        for (int v = 0; v < V; ++v) {
+          spp[v] = sqq[v] = spq[v] = 0.0f;
+          if (p >= 0)
+            for (int i = gl + G * v; i < n; i += G * V) {
+              const float a = mp[i], b = mq[i];
+              spp[v] = fmaf(a, a, spp[v]);
+              sqq[v] = fmaf(b, b, sqq[v]);
+              spq[v] = fmaf(a, b, spq[v]);
+            }
         }
-        const T scale_pq = Num<T>::sqrt_(app) * Num<T>::sqrt_(aqq);
-        if (p >= 0 && fabs(apq) > tol * scale_pq) {
-          if (fabs(apq) > big_tol * scale_pq) big = 1;
-          // the angle only needs float accuracy (the next sweep removes what
-          // is left); c and s are formed in T so the rotation is orthogonal
-          // to T's rounding
-          const float zf = (float)((aqq - app) / ((T)2 * apq));
-          const float tf = (zf >= 0.0f ? 1.0f : -1.0f) / (fabsf(zf) + sqrtf(1.0f + zf * zf));
-          const T t = (T)tf;
-          const T c = Num<T>::rsqrt_((T)1 + t * t), sn = c * t;
-          T* mp = M + (int64_t)p * n;
-          T* mq = M + (int64_t)q * n;
-          T* bp = B + (int64_t)p * n;
-          T* bq = B + (int64_t)q * n;
+        const float app = virtual_sum<V>(spp), aqq = virtual_sum<V>(sqq), apq = virtual_sum<V>(spq);
+        const float scale_pq = sqrtf(app) * sqrtf(aqq);
+        if (p >= 0 && fabsf(apq) > tol * scale_pq) {
+          if (fabsf(apq) > big_tol * scale_pq) big = 1;
+          const float zf = (aqq - app) / (2.0f * apq);
+          const float t = (zf >= 0.0f ? 1.0f : -1.0f) / (fabsf(zf) + sqrtf(1.0f + zf * zf));
+          const float c = rsqrtf(1.0f + t * t), sn = c * t;
+          float* bp = B + (int64_t)p * ld;
+          float* bq = B + (int64_t)q * ld;
+#pragma unroll 4
           for (int i = gl; i < n; i += G) {
-            const T a = mp[i], b = mq[i];
-            mp[i] = c * a - sn * b;
-            mq[i] = sn * a + c * b;
-            const T u = bp[i], v = bq[i];
-            bp[i] = c * u - sn * v;
-            bq[i] = sn * u + c * v;
+            const float x = mp[i], y = mq[i], u = bp[i], w = bq[i];
+            // written out: the choice of the fused product is part of the result
+            mp[i] = fmaf(c, x, -__fmul_rn(sn, y));
+            mq[i] = fmaf(sn, x, __fmul_rn(c, y));
+            bp[i] = fmaf(c, u, -__fmul_rn(sn, w));
+            bq[i] = fmaf(sn, u, __fmul_rn(c, w));
           }
           rotated = 1;
         }
+        __syncwarp();
       }
       __syncthreads();
     }
@@ -540,17 +564,17 @@ __device__ bool cta_jacobi_svd_g(int n, T* M, T* B, T* sigma, int max_sweeps, in
   }
   *sweeps_out = sweep;
   // column norms (uniform slot count so every lane reaches every shuffle)
-  const int nslots = (n + NG - 1) / NG;
-  for (int sidx = 0; sidx < nslots; ++sidx) {
+  for (int sidx = 0; sidx < (n + NG - 1) / NG; ++sidx) {
     const int k = group + sidx * NG;
-    T s = 0;
-    if (k < n) {
-      const T* mk = M + (int64_t)k * n;
-      for (int i = gl; i < n; i += G) s = fma(mk[i], mk[i], s);
-    }
+    float s[V];
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (k < n && gl == 0) sigma[k] = Num<T>::sqrt_(s);
+    for (int v = 0; v < V; ++v) {
+      s[v] = 0.0f;
+      if (k < n)
+        for (int i = gl + G * v; i < n; i += G * V) s[v] = fmaf(M[(int64_t)k * ld + i], M[(int64_t)k * ld + i], s[v]);
+    }
+    const float t = virtual_sum<V>(s);
+    if (k < n && gl == 0) sigma[k] = sqrtf(t);
   }
   __syncthreads();
   return converged;
@@ -573,9 +597,8 @@ __device__ __forceinline__ float bits_to_float(double v, int e) {
   const int mag = field >= 255 ? 0x7F7FFFFF : (field << 23) | ((int)(b >> 29) & 0x7FFFFF);
   return __int_as_float(mag | ((int)(b >> 32) & 0x80000000));
 }
-template <int DUMMY = 0>
-__device__ bool cta_jacobi_svd_f64(int n, double* M, double* B, double* sigma, int max_sweeps, int* counter,
-                                   int* sweeps_out) {
+__device__ inline bool cta_jacobi_svd_f64(int n, int ld, double* M, double* B, double* sigma, int max_sweeps,
+                                          int* sweeps_out) {
   constexpr int G = 8, NG = NTHREADS / G;
   const int lane = threadIdx.x & 31, gl = lane & (G - 1), group = threadIdx.x / G;
   const int N = (n % 2 == 0) ? n : n + 1;
@@ -591,11 +614,11 @@ __device__ bool cta_jacobi_svd_f64(int n, double* M, double* B, double* sigma, i
         int p = -1, q = -1;
         if (k < N / 2) {
           if (k == 0) { p = N - 1; q = r; }
-          else { p = (r + k) % (N - 1); q = (r - k + (N - 1)) % (N - 1); }
+          else { p = r + k < N - 1 ? r + k : r + k - (N - 1); q = r - k >= 0 ? r - k : r - k + (N - 1); }
           if (p >= n || q >= n) p = q = -1;
         }
-        double* mp = M + (int64_t)(p < 0 ? 0 : p) * n;
-        double* mq = M + (int64_t)(p < 0 ? 0 : q) * n;
+        double* mp = M + (int64_t)(p < 0 ? 0 : p) * ld;
+        double* mq = M + (int64_t)(p < 0 ? 0 : q) * ld;
         double app = 0.0, aqq = 0.0, apq = 0.0;
         if (p >= 0) {
 #pragma unroll 4
@@ -630,8 +653,8 @@ __device__ bool cta_jacobi_svd_f64(int n, double* M, double* B, double* sigma, i
             c = fma(y * d, fma(0.375, d, 0.5), y);
           }
           const double sn = c * t;
-          double* bp = B + (int64_t)p * n;
-          double* bq = B + (int64_t)q * n;
+          double* bp = B + (int64_t)p * ld;
+          double* bq = B + (int64_t)q * ld;
 #pragma unroll 2
           for (int i = gl; i < n; i += G) {
             const double x = mp[i], y = mq[i], u = bp[i], v = bq[i];
@@ -657,7 +680,7 @@ __device__ bool cta_jacobi_svd_f64(int n, double* M, double* B, double* sigma, i
     const int k = group + sidx * NG;
     double s = 0.0;
     if (k < n) {
-      const double* mk = M + (int64_t)k * n;
+      const double* mk = M + (int64_t)k * ld;
       for (int i = gl; i < n; i += G) s = fma(mk[i], mk[i], s);
     }
 #pragma unroll
@@ -668,12 +691,22 @@ __device__ bool cta_jacobi_svd_f64(int n, double* M, double* B, double* sigma, i
   return converged;
 }
 
+// Column stride of the operands in shared memory: 8 mod 32 floats (8 mod 16
+// doubles) puts the pairs of a warp, whose columns are consecutive, on
+// different banks.
+template <class T> __host__ __device__ __forceinline__ int jacobi_ld(int n) {
+  return sizeof(T) == 4 ? (n + 23) / 32 * 32 + 8 : (n + 7) / 16 * 16 + 8;
+}
+// ld: column stride of M and B.
 template <class T>
-__device__ bool cta_jacobi_svd(int n, T* M, T* B, T* sigma, int max_sweeps, int* counter, int* sweeps_out) {
-  if constexpr (sizeof(T) == 8) return cta_jacobi_svd_f64(n, M, B, sigma, max_sweeps, counter, sweeps_out);
-  if (n <= 16) return cta_jacobi_svd_g<T, 8>(n, M, B, sigma, max_sweeps, counter, sweeps_out);
-  if (n <= 48) return cta_jacobi_svd_g<T, 16>(n, M, B, sigma, max_sweeps, counter, sweeps_out);
-  return cta_jacobi_svd_g<T, 32>(n, M, B, sigma, max_sweeps, counter, sweeps_out);
+__device__ bool cta_jacobi_svd(int n, int ld, T* M, T* B, T* sigma, int max_sweeps, int* sweeps_out) {
+  if constexpr (sizeof(T) == 8) {
+    return cta_jacobi_svd_f64(n, ld, M, B, sigma, max_sweeps, sweeps_out);
+  } else {
+    if (n <= 16) return cta_jacobi_svd_f32<1>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
+    if (n <= 48) return cta_jacobi_svd_f32<2>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
+    return cta_jacobi_svd_f32<4>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
+  }
 }
 
 // ---------------------------------------------------------------- tridiagonal
@@ -812,11 +845,15 @@ __device__ T thread_tridiag_eig(int k, const T* a, const T* b, int j) {
 // basis; a, bb, coef are vectors of length n+1, w of length n.  Stops when
 // the smallest Ritz value is stable to 64 eps or the Krylov space is
 // exhausted (k = n or b_k ~ 0).
+// ldq: column stride of the basis in shared memory, odd, so that the lanes that
+// each sum over one column read different banks (at n = 64 an even stride put
+// all 32 on one).
 template <class T>
-__device__ T warp_lanczos_eigmin(int n, const T* Z, T* Qs, int kq, T* Qg, T* a, T* bb, T* w, T* coef, int* steps) {
+__device__ T warp_lanczos_eigmin(int n, const T* Z, T* Qs, int ldq, int kq, T* Qg, T* a, T* bb, T* w, T* coef,
+                                 int* steps) {
   const int lane = threadIdx.x & 31;
   // column l of the basis: shared memory for l < kq, global memory after
-  auto Qc = [&](int l) -> T* { return l < kq ? Qs + (int64_t)l * n : Qg + (int64_t)l * n; };
+  auto Qc = [&](int l) -> T* { return l < kq ? Qs + l * ldq : Qg + (int64_t)l * n; };
   T* Q = Qc(0);
   T nrm2 = 0;
   for (int i = lane; i < n; i += 32) {
@@ -1143,20 +1180,20 @@ template <class T, class V>
 __device__ void warp_potrs(int m, const T* __restrict__ L, V* x, V* rdiag) {
   const int lane = threadIdx.x & 31;
   // reciprocal diagonal once (lanes in parallel) instead of a division per row
-  for (int k = lane; k < m; k += 32) rdiag[k] = (V)1 / (V)L[k + (int64_t)k * m];
+  for (int k = lane; k < m; k += 32) rdiag[k] = (V)1 / (V)widen(L[k + (int64_t)k * m]);
   __syncwarp();
   for (int k = 0; k < m; ++k) {
     const V xk = x[k] * rdiag[k];
     __syncwarp();
     if (lane == 0) x[k] = xk;
     const T* lk = L + (int64_t)k * m;
-    for (int i = k + 1 + lane; i < m; i += 32) x[i] -= (V)lk[i] * xk;
+    for (int i = k + 1 + lane; i < m; i += 32) x[i] -= (V)widen(lk[i]) * xk;
     __syncwarp();
   }
   for (int k = m - 1; k >= 0; --k) {
     const T* lk = L + (int64_t)k * m;
     V s = 0;
-    for (int i = k + 1 + lane; i < m; i += 32) s += (V)lk[i] * x[i];
+    for (int i = k + 1 + lane; i < m; i += 32) s += (V)widen(lk[i]) * x[i];
     s = warp_sum(s);
     if (lane == 0) x[k] = (x[k] - s) * rdiag[k];
     __syncwarp();
