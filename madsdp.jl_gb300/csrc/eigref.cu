@@ -270,8 +270,8 @@ __global__ void __launch_bounds__(kClusterThreads) k_cluster_solve(int n, const 
 // (consecutive) pairs of a warp on different banks; the pair's columns of M
 // stay in registers between the sums and the rotation.  Bound by the shared
 // memory's bandwidth (M and V read and written once a round, n - 1 rounds a
-// sweep): 0.9 ms at n = 100 where cuSOLVER's FP32 eigensolver takes about a
-// hundred launches and 1.2 ms.
+// sweep).  cuSOLVER's FP32 eigensolver takes about a hundred launches, 1.2 ms
+// of device time at n = 100; kJacobiMax has the figures of both.
 __host__ __device__ inline int jacobi_ld(int n) { return (n + 23) / 32 * 32 + 8; }
 template <int R>
 __global__ void __launch_bounds__(416) k_jacobi32(int n, const double* __restrict__ M, double* __restrict__ V) {

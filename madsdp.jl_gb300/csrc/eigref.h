@@ -34,10 +34,11 @@ constexpr int kMaxCluster = 64;
 inline int64_t ibuf_ints(int n) { return 3 * (int64_t)n + 8; }
 
 // Orders up to which the FP32 start runs in one thread block.  Its time grows
-// with n^3 (0.9 ms at n = 100: the shared memory's bandwidth, four passes over
-// n^2 floats in each of n - 1 rounds a sweep), cuSOLVER's FP32 eigensolver
-// takes 1.2 ms there and less than the block from n = 110 on (whole prepare at
-// n = 150: 4.6 ms with the block, at n = 170 3.3 ms without).
+// with n^3 (the shared memory's bandwidth: four passes over n^2 floats in each
+// of n - 1 rounds a sweep), cuSOLVER's with its hundred launches.  Whole
+// prepare with the block and with cuSOLVER's start (GB300): 0.44 and 0.56 ms at
+// n = 16, 0.86 and 1.39 at 64, 1.44 and 1.94 at 96, 1.86 and 2.18 at 104; at
+// 150 the block took 4.6 ms, cuSOLVER's start 2.85.
 constexpr int kJacobiMax = 104;
 // V: right singular vectors of M (n x n, column-major) to FP32 accuracy, by
 // ascending singular value; M is not changed.

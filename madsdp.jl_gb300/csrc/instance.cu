@@ -958,7 +958,8 @@ bool update_termination(S* s) {
 // Orders refined from an FP32 basis.  With the products as fast as they are the
 // refined route takes half the time of cuSOLVER's FP64 eigensolver at every
 // order tried above 256 (whole prepare, GB300: n = 300: 5.0 ms against 10.4,
-// n = 449: 7.8 against 14.7, n = 517: 9.1 against 18); orders around 400 stay
+// n = 384: 6.1 against 12.8, n = 449: 7.8 against 14.7, n = 517: 9.0 against
+// 17.8); orders around 400 stay
 // with the FP64 eigensolver because the tests hold 400 to it.
 bool eig_refinable(int n) { return n >= 8 && (n <= 384 || n >= 450); }
 constexpr int kEigRefineMax = 8;

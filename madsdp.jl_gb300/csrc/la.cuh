@@ -287,7 +287,10 @@ __device__ void cta_gemm(int n, int ta, int tb, int loA, int loB, T alpha, const
 // the reciprocal pivot).  Three barriers per eight columns instead of 24, and
 // no index divisions over the whole square: the double Schur factorizations
 // of a three-iteration slice took 11 million clocks at m = 127, now 2.7.
-template <class T> __device__ __forceinline__ void chol_pivot(T d, T& root, T& inv);
+template <class T> __device__ __forceinline__ void chol_pivot(T d, T& root, T& inv) {
+  root = Num<T>::sqrt_(d);
+  inv = (T)1 / root;
+}
 template <> __device__ __forceinline__ void chol_pivot<float>(float d, float& root, float& inv) {
   root = sqrtf(d);
   inv = 1.0f / root;
@@ -312,6 +315,21 @@ __device__ __forceinline__ bool pivot_ok(float d) {
   return b > 0 && b < 0x7F800000;
 }
 template <class T>
+__device__ __forceinline__ bool pivot_ok(T d) {
+  return d > (T)0 && Num<T>::finite(d);
+}
+// x of lane `src`, for any T of whole 32-bit words
+template <class T>
+__device__ __forceinline__ T lane_value(T x, int src) {
+  static_assert(sizeof(T) % 4 == 0, "whole words");
+  unsigned w[sizeof(T) / 4];
+  memcpy(w, &x, sizeof(T));
+#pragma unroll
+  for (int k = 0; k < (int)(sizeof(T) / 4); ++k) w[k] = __shfl_sync(0xffffffffu, w[k], src);
+  memcpy(&x, w, sizeof(T));
+  return x;
+}
+template <class T>
 __device__ bool cta_potrf(int n, T* a, int lda, int* flag) {
   constexpr int KB = 8, R = sizeof(T) == 8 ? 2 : 4;
   __shared__ T L11[KB][KB], rinv[KB];  // L11[k][c] = L(c, k)
@@ -328,7 +346,7 @@ __device__ bool cta_potrf(int n, T* a, int lda, int* flag) {
       bool bad = false;
 #pragma unroll
       for (int k = 0; k < KB; ++k) {
-        T d = __shfl_sync(0xffffffffu, x[k], k);
+        T d = lane_value(x[k], k);
         if (!pivot_ok(d)) {
           bad = true;
           d = (T)1;
@@ -340,7 +358,7 @@ __device__ bool cta_potrf(int n, T* a, int lda, int* flag) {
         if (r < KB) L11[k][r] = l;
         if (r == k) rinv[k] = inv;
 #pragma unroll
-        for (int c = k + 1; c < KB; ++c) x[c] = fma(-l, __shfl_sync(0xffffffffu, l, c), x[c]);
+        for (int c = k + 1; c < KB; ++c) x[c] = fma(-l, lane_value(l, c), x[c]);
       }
       if (bad) *flag = 1;
 #pragma unroll
