@@ -366,6 +366,8 @@ int msdp_solver_step_eig(msdp_solver* solver, int32_t block, const double* L, co
  *                         host-assembled H (m x m column-major, lower
  *                         triangle read, Hermitian(H, :L)); *success =
  *                         issuccess
+ *   msdp_schur_factorize_rows  the same of an H stored by rows (turned on
+ *                         the device); its lower triangle is read too
  *   msdp_schur_solve      schur_solve!(ws, rhs) (src/schur_solvers.jl:21):
  *                         rhs (m, host) is overwritten by the solution
  * MSDP_MIXED: FP32-class factor, each solve refined against H in FP64 until
@@ -377,6 +379,7 @@ typedef struct msdp_schur msdp_schur;
 int msdp_schur_create(msdp_context* ctx, int32_t m, int32_t precision, msdp_schur** ws);
 int msdp_schur_destroy(msdp_schur* ws);
 int msdp_schur_factorize(msdp_schur* ws, const double* H, int32_t* success);
+int msdp_schur_factorize_rows(msdp_schur* ws, const double* H, int32_t* success);
 int msdp_schur_solve(msdp_schur* ws, double* rhs);
 int msdp_schur_fp64_active(const msdp_schur* ws);
 

@@ -127,6 +127,7 @@ SIGNATURES = [
     ("msdp_schur_create", i32, [C.c_void_p, i32, i32, P(C.c_void_p)]),
     ("msdp_schur_destroy", i32, [C.c_void_p]),
     ("msdp_schur_factorize", i32, [C.c_void_p, P(f64), P(i32)]),
+    ("msdp_schur_factorize_rows", i32, [C.c_void_p, P(f64), P(i32)]),
     ("msdp_schur_solve", i32, [C.c_void_p, P(f64)]),
     ("msdp_schur_fp64_active", i32, [C.c_void_p]),
     ("msdp_dense_cholesky", i32, [i32, i32, C.c_void_p, i64, P(i32), C.c_void_p]),

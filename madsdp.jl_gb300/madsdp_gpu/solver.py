@@ -665,11 +665,15 @@ class SchurWorkspace:
         self.ctx.adopt(self)
 
     def factorize(self, H) -> bool:
-        Hf = np.asfortranarray(H, dtype=np.float64)
+        # an array stored by rows goes to the GPU as it is and is turned there
+        H = np.asarray(H)
+        rows = H.dtype == np.float64 and H.flags.c_contiguous and H.flags.aligned
+        Hf = H if rows else np.asfortranarray(H, dtype=np.float64)
         if Hf.shape != (self.m, self.m):
             raise ValueError("H must be m x m")
         ok = C.c_int32()
-        rc = self.lib.msdp_schur_factorize(self.h, _ptr(Hf), C.byref(ok))
+        call = self.lib.msdp_schur_factorize_rows if rows else self.lib.msdp_schur_factorize
+        rc = call(self.h, _ptr(Hf), C.byref(ok))
         if rc != 0:
             raise GPUError(f"msdp_schur_factorize: {_lib.ERRORS.get(rc, rc)}")
         return bool(ok.value)

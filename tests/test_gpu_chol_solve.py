@@ -43,3 +43,23 @@ def test_mixed_solve_refines_to_float64(gpu_ctx, m):
     # the refinement stops at 1e-11 |b| or below
     assert np.abs(b - H @ x).max() <= 1.1e-11 * np.abs(b).max() + 8 * m * EPS * np.abs(H).sum(axis=1).max() * np.abs(x).max()
     ws.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("m", [1, 2, 31, 32, 33, 65, 257, 517])
+def test_factorize_takes_any_layout(gpu_ctx, m, precision):
+    # the lower triangle is read whatever the memory order: the same factor,
+    # so the same bits of the solution, and nothing of the upper triangle
+    H, b = _system(m, m + 2)
+    low = np.where(np.tri(m, dtype=bool), H, np.nan)
+    wide = np.full((2 * m, 3 * m), np.nan)
+    wide[::2, ::3] = low
+    ws = M.SchurWorkspace(m, precision=precision)
+    got = []
+    for A in (np.ascontiguousarray(low), np.asfortranarray(low), wide[::2, ::3], low.tolist()):
+        assert ws.factorize(A)
+        got.append(ws.solve(b))
+    assert all(np.array_equal(got[0], x) for x in got[1:])
+    bound = 8 * m * EPS * np.abs(H).sum(axis=1).max() * np.abs(got[0]).max()
+    assert np.abs(b - H @ got[0]).max() <= bound + (1.1e-11 * np.abs(b).max() if precision == "mixed" else 0.0)
+    ws.close()
