@@ -263,23 +263,27 @@ __global__ void __launch_bounds__(kClusterThreads) k_cluster_solve(int n, const 
 }
 
 // ---------------------------------------------------------------- FP32 start
-// Right singular vectors of M (n x n, n <= kJacobiMax) by FP32 one-sided
-// Jacobi in one thread block: eigenvectors of N = M'M.  Eight lanes per column
-// pair, so that all n/2 pairs of a round-robin round run at once; M and V in
-// shared memory with a column stride of 8 mod 32, which puts the four
-// (consecutive) pairs of a warp on different banks; the pair's columns of M
-// stay in registers between the sums and the rotation.  Bound by the shared
-// memory's bandwidth (M and V read and written once a round, n - 1 rounds a
-// sweep).  cuSOLVER's FP32 eigensolver takes about a hundred launches, 1.2 ms
-// of device time at n = 100; kJacobiMax has the figures of both.
-__host__ __device__ inline int jacobi_ld(int n) { return (n + 23) / 32 * 32 + 8; }
+// Right singular vectors of M (n x n, n <= kJacobiMax), which are eigenvectors
+// of N = M'M, by FP32 one-sided Jacobi in one thread block on the columns of
+// M': once they are orthogonal, M' W = V diag(sigma), so the normalized
+// columns are V and no rotation is accumulated.  Eight lanes per column pair,
+// so that all n/2 pairs of a round-robin round run at once; columns padded
+// with zeros to a multiple of 32 floats, which the eight lanes read as whole
+// 128-byte rows (16 bytes each); a pair's columns stay in registers between
+// the sum and the rotation.  The squared norms are fresh at the start of a
+// sweep and carried through its rotations: one sum a pair.  Bound by the
+// shared memory's bandwidth and the latency of a round (n - 1 rounds a sweep).
+// With accumulated rotations and single floats a lane it took 0.83 ms at
+// n = 100, and a solve of that order 38.8 ms where it now takes 35.0;
+// kJacobiMax has the figures beside cuSOLVER's.
+__host__ __device__ inline int jacobi_ld(int n) { return (n + 31) / 32 * 32; }
 template <int R>
-__global__ void __launch_bounds__(416) k_jacobi32(int n, const double* __restrict__ M, double* __restrict__ V) {
+__global__ void __launch_bounds__(512) k_jacobi32(int n, const double* __restrict__ M, double* __restrict__ V) {
   extern __shared__ double sm_[];
   float* A = (float*)sm_;
-  const int ld = jacobi_ld(n);
-  float* B = A + n * ld;
-  __shared__ float red[20];
+  constexpr int ld = 32 * R;
+  __shared__ float red[16], nrm[kJacobiMax];
+  __shared__ int rank[kJacobiMax];
   const int t = threadIdx.x, gl = t & 7, group = t >> 3, lane = t & 31, warp = t >> 5, nw = blockDim.x >> 5;
   // scaled by the largest entry's power of two: sums of squares stay in range
   float mx = 0.0f;
@@ -292,14 +296,27 @@ __global__ void __launch_bounds__(416) k_jacobi32(int n, const double* __restric
   for (int w = 1; w < nw; ++w) mx = fmaxf(mx, red[w]);
   const int e = min(max((__float_as_int(mx) >> 23) - 127, -126), 126);
   const float f = __int_as_float((127 - e) << 23);
-  for (int idx = t; idx < n * n; idx += blockDim.x) {
-    const int c = idx / n, r = idx - c * n;
-    A[c * ld + r] = (float)M[idx] * f;
-    B[c * ld + r] = r == c ? 1.0f : 0.0f;
+  // column c of M' holds row c of M: 4 rows x 8 columns of M a warp, which is
+  // whole sectors of global memory and 4 lanes a bank
+  for (int tile = warp; tile < (n + 3) / 4 * (ld / 8); tile += nw) {
+    const int c = tile / (ld / 8) * 4 + (lane & 3), r = tile % (ld / 8) * 8 + (lane >> 2);
+    if (c < n) A[c * ld + r] = r < n ? (float)M[c + (int64_t)r * n] * f : 0.0f;
   }
   __syncthreads();
   const int N = n + (n & 1);
   const float tol = sqrtf((float)n) * 1.1920929e-7f, big_tol = sqrtf(tol);
+  auto norms = [&]() {  // one warp a column
+    for (int c = warp; c < n; c += nw) {
+      float s = 0.0f;
+#pragma unroll
+      for (int u = 0; u < R; ++u) s = fmaf(A[c * ld + lane + 32 * u], A[c * ld + lane + 32 * u], s);
+#pragma unroll
+      for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) nrm[c] = s;
+    }
+    __syncthreads();
+  };
+  norms();
   for (int sweep = 0; sweep < 30; ++sweep) {
     int rotated = 0, big = 0;
     for (int r = 0; r < N - 1; ++r) {
@@ -314,25 +331,23 @@ __global__ void __launch_bounds__(416) k_jacobi32(int n, const double* __restric
         }
         if (p >= n || q >= n) p = q = -1;
       }
-      float* ap = A + (p < 0 ? 0 : p) * ld;
-      float* aq = A + (p < 0 ? 0 : q) * ld;
-      float x[R], y[R];
-      float spp = 0.0f, sqq = 0.0f, spq = 0.0f;
+      float4* ap = (float4*)(A + (p < 0 ? 0 : p) * ld) + gl;
+      float4* aq = (float4*)(A + (p < 0 ? 0 : q) * ld) + gl;
+      float4 x[R], y[R];
+      const float spp = p >= 0 ? nrm[p] : 0.0f, sqq = p >= 0 ? nrm[q] : 0.0f;
+      float s0 = 0.0f, s1 = 0.0f;
 #pragma unroll
       for (int u = 0; u < R; ++u) {
-        const int i = gl + 8 * u;
-        x[u] = p >= 0 && i < n ? ap[i] : 0.0f;
-        y[u] = p >= 0 && i < n ? aq[i] : 0.0f;
-        spp = fmaf(x[u], x[u], spp);
-        sqq = fmaf(y[u], y[u], sqq);
-        spq = fmaf(x[u], y[u], spq);
+        x[u] = ap[8 * u];
+        y[u] = aq[8 * u];
+        s0 = fmaf(x[u].x, y[u].x, s0);
+        s1 = fmaf(x[u].y, y[u].y, s1);
+        s0 = fmaf(x[u].z, y[u].z, s0);
+        s1 = fmaf(x[u].w, y[u].w, s1);
       }
+      float spq = s0 + s1;
 #pragma unroll
-      for (int o = 4; o; o >>= 1) {
-        spp += __shfl_xor_sync(0xffffffffu, spp, o);
-        sqq += __shfl_xor_sync(0xffffffffu, sqq, o);
-        spq += __shfl_xor_sync(0xffffffffu, spq, o);
-      }
+      for (int o = 4; o; o >>= 1) spq += __shfl_xor_sync(0xffffffffu, spq, o);
       const float scale = sqrtf(spp) * sqrtf(sqq);
       if (p >= 0 && fabsf(spq) > tol * scale) {
         rotated = 1;
@@ -340,46 +355,36 @@ __global__ void __launch_bounds__(416) k_jacobi32(int n, const double* __restric
         const float z = (sqq - spp) / (2.0f * spq);
         const float tn = (z >= 0.0f ? 1.0f : -1.0f) / (fabsf(z) + sqrtf(1.0f + z * z));
         const float c = rsqrtf(1.0f + tn * tn), s = c * tn;
-        float* vp = B + p * ld;
-        float* vq = B + q * ld;
+        if (gl == 0) {
+          nrm[p] = fabsf(fmaf(-tn, spq, spp));
+          nrm[q] = fabsf(fmaf(tn, spq, sqq));
+        }
 #pragma unroll
         for (int u = 0; u < R; ++u) {
-          const int i = gl + 8 * u;
-          if (i < n) {
-            const float a = vp[i], b = vq[i];
-            ap[i] = c * x[u] - s * y[u];
-            aq[i] = s * x[u] + c * y[u];
-            vp[i] = c * a - s * b;
-            vq[i] = s * a + c * b;
-          }
+          const float4 a = x[u], b = y[u];
+          ap[8 * u] = make_float4(c * a.x - s * b.x, c * a.y - s * b.y, c * a.z - s * b.z, c * a.w - s * b.w);
+          aq[8 * u] = make_float4(s * a.x + c * b.x, s * a.y + c * b.y, s * a.z + c * b.z, s * a.w + c * b.w);
         }
       }
       __syncthreads();
     }
     rotated = __syncthreads_or(rotated);
     big = __syncthreads_or(big);
+    norms();
     // quadratic convergence: after a sweep whose rotations were all below
     // sqrt(tol) what is left is below tol
     if (!rotated || !big) break;
   }
-  // columns by ascending singular value: norms, then the rank of each
-  __shared__ float sig[kJacobiMax];
-  __shared__ int rank[kJacobiMax];
-  for (int c = t; c < n; c += blockDim.x) {
-    float s = 0.0f;
-    for (int i = 0; i < n; ++i) s = fmaf(A[c * ld + i], A[c * ld + i], s);
-    sig[c] = s;
-  }
-  __syncthreads();
+  // columns by ascending singular value, normalized
   for (int c = t; c < n; c += blockDim.x) {
     int k = 0;
-    for (int i = 0; i < n; ++i) k += sig[i] < sig[c] || (sig[i] == sig[c] && i < c);
+    for (int i = 0; i < n; ++i) k += nrm[i] < nrm[c] || (nrm[i] == nrm[c] && i < c);
     rank[c] = k;
   }
   __syncthreads();
   for (int idx = t; idx < n * n; idx += blockDim.x) {
     const int c = idx / n, r = idx - c * n;
-    V[r + (int64_t)rank[c] * n] = (double)B[c * ld + r];
+    V[r + (int64_t)rank[c] * n] = (double)(A[c * ld + r] * rsqrtf(nrm[c]));
   }
 }
 
@@ -404,14 +409,15 @@ cudaError_t jacobi_start(int n, const double* M, double* V, cudaStream_t st) {
   static std::once_flag once;
   static cudaError_t attr = cudaSuccess;
   std::call_once(once, [] {
-    const int most = 2 * kJacobiMax * jacobi_ld(kJacobiMax) * (int)sizeof(float);
-    attr = cudaFuncSetAttribute(k_jacobi32<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
-    if (attr == cudaSuccess) attr = cudaFuncSetAttribute(k_jacobi32<13>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
+    const int most = kJacobiMax * jacobi_ld(kJacobiMax) * (int)sizeof(float);
+    attr = cudaFuncSetAttribute(k_jacobi32<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, most);
   });
   if (attr != cudaSuccess) return attr;
-  const int threads = ((n + 1) / 2 * 8 + 31) / 32 * 32, smem = 2 * n * jacobi_ld(n) * (int)sizeof(float);
-  if (n <= 64) k_jacobi32<8><<<1, threads, smem, st>>>(n, M, V);
-  else k_jacobi32<13><<<1, threads, smem, st>>>(n, M, V);
+  const int threads = ((n + 1) / 2 * 8 + 31) / 32 * 32, smem = n * jacobi_ld(n) * (int)sizeof(float);
+  if (n <= 32) k_jacobi32<1><<<1, threads, smem, st>>>(n, M, V);
+  else if (n <= 64) k_jacobi32<2><<<1, threads, smem, st>>>(n, M, V);
+  else if (n <= 96) k_jacobi32<3><<<1, threads, smem, st>>>(n, M, V);
+  else k_jacobi32<4><<<1, threads, smem, st>>>(n, M, V);
   return cudaGetLastError();
 }
 

@@ -34,12 +34,12 @@ constexpr int kMaxCluster = 64;
 inline int64_t ibuf_ints(int n) { return 3 * (int64_t)n + 8; }
 
 // Orders up to which the FP32 start runs in one thread block.  Its time grows
-// with n^3 (the shared memory's bandwidth: four passes over n^2 floats in each
-// of n - 1 rounds a sweep), cuSOLVER's with its hundred launches.  Whole
-// prepare with the block and with cuSOLVER's start (GB300): 0.44 and 0.56 ms at
-// n = 16, 0.86 and 1.39 at 64, 1.44 and 1.94 at 96, 1.86 and 2.18 at 104; at
-// 150 the block took 4.6 ms, cuSOLVER's start 2.85.
-constexpr int kJacobiMax = 104;
+// with n^3 (the shared memory's bandwidth, n - 1 rounds of the whole matrix a
+// sweep), cuSOLVER's with its hundred launches.  Whole prepare with the block
+// and with cuSOLVER's start (GB300): 0.43 and 0.55 ms at n = 16, 0.76 and 1.38
+// at 64, 1.16 and 1.96 at 96, 1.83 and 2.66 at 128; with 20 warps and five
+// columns of registers it turns round: 3.0 and 2.8 at 130, 3.4 and 2.9 at 160.
+constexpr int kJacobiMax = 128;
 // V: right singular vectors of M (n x n, column-major) to FP32 accuracy, by
 // ascending singular value; M is not changed.
 cudaError_t jacobi_start(int n, const double* M, double* V, cudaStream_t st);

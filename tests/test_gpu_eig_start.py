@@ -1,7 +1,7 @@
 """The NT eigendecomposition at the orders where its route changes: 8 (first
 refined one), the column groups of the one-block FP32 start (8 lanes a pair,
-8 columns a step: 9, 31, 33, 64, 65, 103, 104), cuSOLVER's FP32 start (105,
-257, 384) and the FP64 eigensolver (7, 385).  Objectives and trajectories
+8 columns a step: 9, 31, 33, 64, 65, 96, 97, 127, 128), cuSOLVER's FP32
+start (129, 257, 384) and the FP64 eigensolver (7, 385).  Objectives and trajectories
 against the oracle with the tolerances of the instance tests (1e-7 of the sum
 of the objectives; per iteration 1e-6 while the gap is above 1e-5); the
 counters show which route ran."""
@@ -14,7 +14,7 @@ from problems import compare_trajectories
 
 pytestmark = pytest.mark.gpu
 
-ORDERS = [7, 8, 9, 31, 33, 64, 65, 103, 104, 105, 257, 384, 385]
+ORDERS = [7, 8, 9, 31, 33, 64, 65, 96, 97, 127, 128, 129, 257, 384, 385]
 
 
 @pytest.mark.parametrize("n", ORDERS)
