@@ -475,28 +475,46 @@ struct Algo {
       // path): eigenvectors by FP32 Jacobi, then M V and Lx V in FP64 and
       // FP64 polishing sweeps to float64 convergence (quadratic from the
       // FP32 basis).  FP32 operands live in shared memory when both fit (up to
-      // n = 95), else the vectors (and from n = 136 on M too) in the FP64
-      // scratch, and the basis is made orthonormal to FP64 by two Newton-Schulz
-      // steps V (3 I - V'V) / 2 (the defect of 1e-6 is squared twice).  FP64
-      // sweeps from the identity at these sizes took 130 million clocks a call
-      // at n = 128.
+      // n = 95).  Above, the columns of M' are made orthogonal instead: they
+      // are V diag(sigma), so no rotation is accumulated and the one matrix
+      // fits up to n = 135 (then in the FP64 scratch).  That basis is made
+      // orthonormal to FP64 by two Newton-Schulz steps V (3 I - V'V) / 2 (the
+      // defect of 1e-6 is squared twice).  FP64 sweeps from the identity at
+      // these sizes took 130 million clocks a call at n = 128.
       float* scratch = (float*)b.W(W_T3);
       const bool both = (2 * nn + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES;
       const int pad = jacobi_ld<float>(n);
-      const int ld = (2 * (int64_t)n * pad + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES ? pad : n;
-      float* sMf = nn * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES ? (float*)smem : scratch;
-      float* sVf = both ? sMf + (int64_t)n * ld : scratch + nn;
+      const int64_t cols = both ? 2 : 1;
+      const int ld = (cols * n * pad + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES ? pad : n;
+      float* sMf = (nn + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES ? (float*)smem : scratch;
+      float* sVf = sMf + (int64_t)n * ld;  // both only
       float* Df = both ? sVf + (int64_t)n * ld : (float*)b.V(WV_EIG);
-      for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
-        const int c = k / n, r = k - c * n;
-        sMf[c * ld + r] = (float)M[k];
-        sVf[c * ld + r] = r == c ? 1.0f : 0.0f;
-      }
-      __syncthreads();
-      int sw32 = 0;
-      cta_jacobi_svd<float>(n, ld, sMf, sVf, Df, 40, &sw32);
       T* V64 = b.W(W_T2);
-      for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) V64[k] = (T)sVf[k / n * ld + k % n];
+      int sw32 = 0;
+      if (both) {
+        for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
+          const int c = k / n, r = k - c * n;
+          sMf[c * ld + r] = (float)M[k];
+          sVf[c * ld + r] = r == c ? 1.0f : 0.0f;
+        }
+        __syncthreads();
+        cta_jacobi_svd<float>(n, ld, sMf, sVf, Df, 40, &sw32);
+        for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) V64[k] = (T)sVf[k / n * ld + k % n];
+      } else {
+        for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
+          const int c = k / n, r = k - c * n;
+          sMf[r * ld + c] = (float)M[k];
+        }
+        __syncthreads();
+        cta_jacobi_svd_f32<4, false>(n, ld, sMf, (float*)nullptr, Df, 40, &sw32);
+        int bad = 0;
+        for (int k = threadIdx.x; k < n; k += NTHREADS) bad |= !(Df[k] > 0.0f && Df[k] < INFINITY);
+        bad = __syncthreads_or(bad);  // out of FP32's range: polished from the identity
+        for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
+          const int c = k / n, r = k - c * n;
+          V64[k] = bad ? (T)(r == c) : (T)(sMf[c * ld + r] / Df[c]);
+        }
+      }
       __syncthreads();
       for (int step = 0; !both && step < 2; ++step) {
         T* K = b.W(W_T3);
@@ -521,7 +539,8 @@ struct Algo {
       const Scratch gs = smem64 ? Scratch{nullptr, 0} : scr();
       cta_gemm<T>(n, 0, 0, 0, 0, (T)1, M, V64, (T)0, sM, gs, 0, ld64);
       cta_gemm<T>(n, 0, 0, 1, 0, (T)1, b.W(W_LX), V64, (T)0, sB, gs, 0, ld64);
-      conv = cta_jacobi_svd<T>(n, ld64, sM, sB, D, 40, &sweeps);
+      conv = both ? cta_jacobi_svd<T>(n, ld64, sM, sB, D, 40, &sweeps)
+                  : cta_jacobi_polish(n, ld64, (double*)sM, (double*)sB, (double*)D, 40, &sweeps);
       sweeps += 1000 * sw32;
       for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
         const int o = k / n * ld64 + k % n;

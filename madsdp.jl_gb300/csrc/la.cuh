@@ -511,7 +511,7 @@ __device__ __forceinline__ float virtual_sum(float (&s)[V]) {
   for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
   return r;
 }
-template <int V>
+template <int V, bool VECS = true>
 __device__ bool cta_jacobi_svd_f32(int n, int ld, float* M, float* B, float* sigma, int max_sweeps, int* sweeps_out) {
   constexpr int G = 8, NG = NTHREADS / G;
   const int gl = threadIdx.x & (G - 1), group = threadIdx.x / G;
@@ -557,16 +557,36 @@ __device__ bool cta_jacobi_svd_f32(int n, int ld, float* M, float* B, float* sig
           const float zf = (aqq - app) / (2.0f * apq);
           const float t = (zf >= 0.0f ? 1.0f : -1.0f) / (fabsf(zf) + sqrtf(1.0f + zf * zf));
           const float c = rsqrtf(1.0f + t * t), sn = c * t;
-          float* bp = B + (int64_t)p * ld;
-          float* bq = B + (int64_t)q * ld;
+          if constexpr (VECS) {
+            float* bp = B + (int64_t)p * ld;
+            float* bq = B + (int64_t)q * ld;
 #pragma unroll 4
-          for (int i = gl; i < n; i += G) {
-            const float x = mp[i], y = mq[i], u = bp[i], w = bq[i];
-            // written out: the choice of the fused product is part of the result
-            mp[i] = fmaf(c, x, -__fmul_rn(sn, y));
-            mq[i] = fmaf(sn, x, __fmul_rn(c, y));
-            bp[i] = fmaf(c, u, -__fmul_rn(sn, w));
-            bq[i] = fmaf(sn, u, __fmul_rn(c, w));
+            for (int i = gl; i < n; i += G) {
+              const float x = mp[i], y = mq[i], u = bp[i], w = bq[i];
+              // written out: the choice of the fused product is part of the result
+              mp[i] = fmaf(c, x, -__fmul_rn(sn, y));
+              mq[i] = fmaf(sn, x, __fmul_rn(c, y));
+              bp[i] = fmaf(c, u, -__fmul_rn(sn, w));
+              bq[i] = fmaf(sn, u, __fmul_rn(c, w));
+            }
+          } else {
+            constexpr int U = 4;  // rows a lane loads before the first store
+            for (int i0 = gl; i0 < n; i0 += G * U) {
+              float x[U], y[U];
+#pragma unroll
+              for (int k4 = 0; k4 < U; ++k4) {
+                const int i = min(i0 + G * k4, n - 1);
+                x[k4] = mp[i];
+                y[k4] = mq[i];
+              }
+#pragma unroll
+              for (int k4 = 0; k4 < U; ++k4) {
+                const int i = i0 + G * k4;
+                if (i >= n) break;
+                mp[i] = fmaf(c, x[k4], -__fmul_rn(sn, y[k4]));
+                mq[i] = fmaf(sn, x[k4], __fmul_rn(c, y[k4]));
+              }
+            }
           }
           rotated = 1;
         }
@@ -705,6 +725,148 @@ __device__ inline bool cta_jacobi_svd_f64(int n, int ld, double* M, double* B, d
     for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
     if (k < n && gl == 0) sigma[k] = sqrt(s);
   }
+  __syncthreads();
+  return converged;
+}
+
+// The same where the incoming basis is orthonormal to FP64 (above order 95).
+// The squared norms of M's columns are fresh at the start of a sweep and
+// carried through its rotations (they only enter the test and the angle, which
+// are float accurate; a sweep whose rotations are small changes them by their
+// squares, one with large rotations is followed by another), and a rotation is
+// three shears: 7 FP64 operations a row and pair, 5 in a sweep of tiny
+// rotations, instead of 11.  The operands are in global memory at these
+// orders: four rows are loaded before the first store, or every row waits for
+// the cache (max-cut slice of 64 problems, n = 50 to 128: 176 ms, now 126).
+// Below, a basis with FP32's defect passes it on to the scaling (1e-6), and
+// the sums and rotations keep their roundings: a different one is enough to
+// move an FP32 entry of a later iteration's start, and with it the iterates by
+// that 1e-6.
+__device__ inline bool cta_jacobi_polish(int n, int ld, double* M, double* B, double* sigma, int max_sweeps,
+                                         int* sweeps_out) {
+  constexpr int G = 8, NG = NTHREADS / G;
+  constexpr int U = 4;  // rows a lane loads before the first store (the compiler cannot move loads past them)
+  const int lane = threadIdx.x & 31, gl = lane & (G - 1), group = threadIdx.x / G;
+  const int N = (n % 2 == 0) ? n : n + 1;
+  const float tol = sqrtf((float)n) * 2.220446e-16f, big_tol = sqrtf(tol);
+  double* nrm = sigma;
+  const int nslots = (n + NG - 1) / NG;
+  auto norms = [&]() {
+    for (int sidx = 0; sidx < nslots; ++sidx) {
+      const int k = group + sidx * NG;
+      double s = 0.0;
+      if (k < n) {
+        const double* mk = M + (int64_t)k * ld;
+        for (int i = gl; i < n; i += G) s = fma(mk[i], mk[i], s);
+      }
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (k < n && gl == 0) nrm[k] = s;
+    }
+    __syncthreads();
+  };
+  norms();
+  bool converged = (n <= 1);
+  int sweep = 0;
+  for (; sweep < max_sweeps && !converged; ++sweep) {
+    int rotated = 0, big = 0;
+    const int slots = (N / 2 + NG - 1) / NG;  // the same for every group: shuffles stay uniform
+    for (int r = 0; r < N - 1; ++r) {
+      for (int sidx = 0; sidx < slots; ++sidx) {
+        const int k = group + sidx * NG;
+        int p = -1, q = -1;
+        if (k < N / 2) {
+          if (k == 0) { p = N - 1; q = r; }
+          else { p = r + k < N - 1 ? r + k : r + k - (N - 1); q = r - k >= 0 ? r - k : r - k + (N - 1); }
+          if (p >= n || q >= n) p = q = -1;
+        }
+        double* mp = M + (int64_t)(p < 0 ? 0 : p) * ld;
+        double* mq = M + (int64_t)(p < 0 ? 0 : q) * ld;
+        double app = 0.0, aqq = 0.0, apq = 0.0;
+        if (p >= 0) {
+          app = nrm[p];
+          aqq = nrm[q];
+#pragma unroll 8
+          for (int i = gl; i < n; i += G) apq = fma(mp[i], mq[i], apq);
+        }
+#pragma unroll
+        for (int o = G / 2; o > 0; o >>= 1) apq += __shfl_xor_sync(0xffffffffu, apq, o);
+        // scaled by the larger of the two norms' exponents
+        const int e = max((__double2hiint(app) >> 20) & 0x7FF, (__double2hiint(aqq) >> 20) & 0x7FF) - 1023;
+        const float fp = bits_to_float(app, e), fq = bits_to_float(aqq, e), fpq = bits_to_float(apq, e);
+        const float scale = sqrtf(fp) * sqrtf(fq);
+        if (p >= 0 && e < 1024 && fabsf(fpq) > tol * scale) {  // e = 1024: infinite or NaN
+          if (fabsf(fpq) > big_tol * scale) big = 1;
+          // the angle only needs float accuracy (the next sweep removes what
+          // is left)
+          const float zf = bits_to_float(aqq - app, e) / (2.0f * fpq);
+          const float tf = (zf >= 0.0f ? 1.0f : -1.0f) / (fabsf(zf) + sqrtf(1.0f + zf * zf));
+          const double t = widen(tf);
+          double* bp = B + (int64_t)p * ld;
+          double* bq = B + (int64_t)q * ld;
+          // three shears: h = tan(angle / 2), sn = 2 h / (1 + h^2), orthogonal to
+          // the rounding of sn.  tiny: the cosine is 1 - 5e-19, below the
+          // rounding of a whole sweep
+          const bool tiny = fabsf(tf) < 1e-9f;
+          double h = 0.0, sn = t;
+          if (gl == 0) {
+            nrm[p] = fabs(fma(-t, apq, app));
+            nrm[q] = fabs(fma(t, apq, aqq));
+          }
+          if (!tiny) {
+            const float hf = tf / (1.0f + sqrtf(1.0f + tf * tf));
+            h = widen(hf);
+            const double h2 = h * h, hh = h + h;
+            if (fabsf(hf) < 1e-4f) {
+              sn = fma(hh, fma(h2, h2, -h2), hh);
+            } else {
+              const double a = 1.0 + h2, y = widen(1.0f / fmaf(hf, hf, 1.0f)), d = fma(-a, y, 1.0);
+              sn = hh * fma(y, fma(d, d, d), y);
+            }
+          }
+          for (int i0 = gl; i0 < n; i0 += G * U) {
+            double x[U], y[U], u[U], v[U];
+#pragma unroll
+            for (int k4 = 0; k4 < U; ++k4) {
+              const int i = min(i0 + G * k4, n - 1);
+              x[k4] = mp[i];
+              y[k4] = mq[i];
+              u[k4] = bp[i];
+              v[k4] = bq[i];
+            }
+#pragma unroll
+            for (int k4 = 0; k4 < U; ++k4) {
+              const int i = i0 + G * k4;
+              if (i >= n) break;
+              if (tiny) {
+                mp[i] = fma(-sn, y[k4], x[k4]);
+                mq[i] = fma(sn, x[k4], y[k4]);
+                bp[i] = fma(-sn, v[k4], u[k4]);
+                bq[i] = fma(sn, u[k4], v[k4]);
+              } else {
+                const double x1 = fma(-h, y[k4], x[k4]), u1 = fma(-h, v[k4], u[k4]);
+                const double y1 = fma(sn, x1, y[k4]), v1 = fma(sn, u1, v[k4]);
+                mp[i] = fma(-h, y1, x1);
+                mq[i] = y1;
+                bp[i] = fma(-h, v1, u1);
+                bq[i] = v1;
+              }
+            }
+          }
+          rotated = 1;
+        }
+        __syncwarp();
+      }
+      __syncthreads();
+    }
+    rotated = __syncthreads_or(rotated);
+    big = __syncthreads_or(big);
+    // quadratic convergence
+    converged = !rotated || !big;
+    norms();
+  }
+  *sweeps_out = sweep;
+  for (int k = threadIdx.x; k < n; k += NTHREADS) sigma[k] = sqrt(nrm[k]);
   __syncthreads();
   return converged;
 }
