@@ -1,10 +1,12 @@
 // Whole-GPU solver for one large SDP (blocks of hundreds to thousands, m in
 // the thousands): every step of the interior-point iteration is a sequence
-// of device-wide operations on one stream.  Dense products, Cholesky
-// factorizations and symmetric eigendecompositions go to cuBLAS/cuSOLVER;
-// the Schur-complement assembly of sparse constraints, A(X), A*(y), the
-// residuals, the NT scaling arithmetic, the Mehrotra correction and every
-// reduction are kernels of this file.  The iteration restates
+// of device-wide operations on one stream (the two sides of a large step
+// length on two).  Dense products run on the tensor cores (tcgemm.h),
+// Cholesky factorizations and solves in chol.h, eigendecompositions in
+// eigref.h from an FP32 basis, step lengths in lanczos.h; cuSOLVER supplies
+// larger FP32 bases and the dense fallback.  The Schur-complement assembly of
+// sparse constraints, A(X), A*(y), the residuals, the NT scaling arithmetic,
+// the Mehrotra correction and every reduction are kernels of this file.  The iteration restates
 // src/primal_dual.jl, src/step.jl, src/directions.jl, src/blocks.jl and
 // src/solver.jl (file:line at each step) with exact eigenvalues for the
 // step lengths.
