@@ -583,25 +583,22 @@ struct Algo {
     if (__syncthreads_or(bad)) return false;
     T* G = GV;
     T* t2 = b.W(W_T2);
-    // double: the columns' factors once, in shared memory (a root and two
-    // divisions per entry took most of this phase)
-    T* f = (T*)smem;  // D^-1/2, D^-3/2, D^-1
+    // double: the columns' roots once, in shared memory.  Quotients, not products
+    // with reciprocals: the roundings matter (cta_jacobi_svd_f64)
+    T* f = (T*)smem;  // D^1/2, D^3/2
     if constexpr (sizeof(T) == 8) {
       for (int k = threadIdx.x; k < n; k += NTHREADS) {
-        double root, inv;
-        chol_pivot<double>(D[k], root, inv);
-        const double rec = fast_recip(D[k]);
-        f[k] = inv;
-        f[n + k] = inv * rec;
-        f[2 * n + k] = rec;
+        const T sq = Num<T>::sqrt_(D[k]);
+        f[k] = sq;
+        f[n + k] = D[k] * sq;
       }
       __syncthreads();
       for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
         const int j = (int)k / n;
-        const T g = G[k] * f[j];
+        const T g = G[k] / f[j];
         G[k] = g;                         // G = Lx V D^-1/2
-        M[k] *= f[n + j];                 // (M V) D^-3/2
-        t2[k] = g * f[2 * n + j];         // G D^-1
+        M[k] /= f[n + j];                 // (M V) D^-3/2
+        t2[k] = g / D[j];                 // G D^-1
       }
     } else {
       for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
@@ -1128,7 +1125,7 @@ struct Algo {
         cta_gemm<T>(n, 0, 0, 0, 0, (T)1, t2, b.W(W_G), (T)0, t3, scr());
         for (int64_t k = threadIdx.x; k < b.nn; k += NTHREADS) {
           const int p = (int)(k % n), q = (int)(k / n);
-          RNT[k] = neg_div(t3[k] + t3[q + (int64_t)p * n], D[p] + D[q]);
+          RNT[k] = -(t3[k] + t3[q + (int64_t)p * n]) / (D[p] + D[q]);
         }
         __syncthreads();
         // G RNT G' with RNT symmetric: lower triangle only
@@ -1229,11 +1226,7 @@ struct Algo {
       const T* D = b.V(WV_D);
       if constexpr (sizeof(T) == 8) {
         T* f = (T*)smem;  // D^-1/2, one root per column instead of two per entry
-        for (int k = threadIdx.x; k < n; k += NTHREADS) {
-          double root, inv;
-          chol_pivot<double>(D[k], root, inv);
-          f[k] = inv;
-        }
+        for (int k = threadIdx.x; k < n; k += NTHREADS) f[k] = Num<T>::rsqrt_(D[k]);
         __syncthreads();
         for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
           const T sc = f[(int)k % n] * f[(int)k / n];
@@ -1276,12 +1269,10 @@ struct Algo {
     if (f32) {
     } else if (n <= 256) {
       if constexpr (sizeof(T) == 8) {
-        int s1 = 0, s2 = 0;
-        const double lx = cta_lanczos_min(n, ZX, b.W(W_Q), smem, MSDP_SMEM_BYTES, sh.lz, &s1);
-        const double ls = cta_lanczos_min(n, ZS, b.W(W_RNT), smem, MSDP_SMEM_BYTES, sh.lz, &s2);
-        if (threadIdx.x == 0) { sh.bc[2] = lx; sh.bc[3] = ls; }
+        pair_lanczos_min(n, ZX, ZS, b.W(W_Q), b.W(W_RNT), smem, MSDP_SMEM_BYTES, sh.lz);
+        if (threadIdx.x == 0) { sh.bc[2] = sh.lz.theta[0]; sh.bc[3] = sh.lz.theta[1]; }
         __syncthreads();
-        steps = s1 + s2;
+        steps = sh.lz.steps[0] + sh.lz.steps[1];
       } else {
         lanczos_pair<T>(n, ZX, ZS, b.W(W_Q), b.W(W_RNT), b.V(WV_LA), b.V(WV_LA2), steps);
       }

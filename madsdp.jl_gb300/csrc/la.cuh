@@ -145,26 +145,6 @@ __device__ __forceinline__ void tri_index(int64_t idx, int& j, int& k) {
   k = (int)(idx - (int64_t)r * (r + 1) / 2);
 }
 
-// 1/d of a normal d by an FP32 reciprocal of the mantissa and one third-order
-// correction (four dependent FP64 instructions, against about 700 clocks for a
-// division); within an ulp.
-__device__ __forceinline__ double fast_recip(double d) {
-  const long long b = __double_as_longlong(d);
-  const int field = (int)(b >> 52) & 0x7FF;
-  if (field < 2 || field > 2044) return 1.0 / d;
-  const double m = __longlong_as_double((b & 0x800FFFFFFFFFFFFFll) | 0x3FF0000000000000ll);  // +-[1, 2)
-  const float f = __frcp_rn(__int_as_float(0x3F800000 | (int)((b >> 29) & 0x7FFFFF)));       // (0.5, 1]
-  const int fb = __float_as_int(f);
-  const double y = __hiloint2double((((fb >> 3) & 0x0FFFFFFF) + 0x38000000) | ((int)(b >> 32) & 0x80000000), fb << 29);
-  const double e = fma(-m, y, 1.0);
-  const double z = fma(y, fma(e, e, e), y);
-  return __longlong_as_double(__double_as_longlong(z) - ((long long)(field - 1023) << 52));
-}
-
-// -s / d; in double by the reciprocal above (within two ulps)
-__device__ __forceinline__ double neg_div(double s, double d) { return -s * fast_recip(d); }
-__device__ __forceinline__ float neg_div(float s, float d) { return -s / d; }
-
 // ---------------------------------------------------------------- GEMM
 // C = alpha * op(A) * op(B) + beta * C for n x n matrices.  ta/tb: 0 = as
 // stored, 1 = transposed.  loA/loB: the stored operand is lower triangular
@@ -296,15 +276,17 @@ template <> __device__ __forceinline__ void chol_pivot<float>(float d, float& ro
   inv = 1.0f / root;
 }
 template <> __device__ __forceinline__ void chol_pivot<double>(double d, double& root, double& inv) {
-  if (__double2hiint(d) < 0x00100000) {  // subnormal
+  if (__double2hiint(d) < 0x06400000) {  // below 2^-923 the residuals fall out of range
     root = sqrt(d);
     inv = 1.0 / root;
     return;
   }
   // root and reciprocal as sqrt and a division round them, by one residual
-  // correction each (Markstein 1990): about 700 clocks instead of 1500
+  // correction each (Markstein 1990): about 700 clocks instead of 1500.  His
+  // reciprocal misses where the root's mantissa is all ones
   fast_root(d, root, inv);
-  inv = fma(fma(-root, inv, 1.0), inv, inv);
+  const long long b = __double_as_longlong(root);
+  inv = (b & 0xFFFFFFFFFFFFFll) == 0xFFFFFFFFFFFFFll ? 1.0 / root : fma(fma(-root, inv, 1.0), inv, inv);
 }
 __device__ __forceinline__ bool pivot_ok(double d) {
   const long long b = __double_as_longlong(d);
@@ -499,14 +481,14 @@ __device__ void cta_potrs(int n, const T* __restrict__ L, V* x) {
 // three.  So the results are those of groups of 8 V lanes, bit for bit, but a
 // warp has four pairs in flight instead of 4 / V and nine shuffles instead of
 // up to fifteen on the critical path of each (a shuffle is about 75 clocks).
-template <int V>
-__device__ __forceinline__ float virtual_sum(float (&s)[V]) {
+template <int V, class T>
+__device__ __forceinline__ T virtual_sum(T (&s)[V]) {
   if (V == 4) {
     s[0] += s[2 % V];
     s[1 % V] += s[3 % V];
   }
   if (V >= 2) s[0] += s[1 % V];
-  float r = s[0];
+  T r = s[0];
 #pragma unroll
   for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
   return r;
@@ -618,88 +600,134 @@ __device__ bool cta_jacobi_svd_f32(int n, int ld, float* M, float* B, float* sig
   return converged;
 }
 
-// The double version: eight lanes per column pair at every order, and only
-// what needs FP64 in FP64.  A FP64 instruction holds its quarter of the SM for
-// 64 clocks whatever the lanes do, so four pairs share a warp's instructions;
-// the rotation test and the angle are formed in FP32 (from the FP64 sums, by
-// their bits), and c comes from the angle by a series (|t| < 1e-4, where the
-// polishing sweeps are) or a corrected FP32 reciprocal root.  About 26 FP64
-// instructions a pair at n = 64 where the generic version has 90, among them
-// two square roots, two divisions and a reciprocal root: 48 million clocks of
-// a three-iteration slice before (FP32 start included), 24 now.
-// Rounds to FP32 by truncation, scaled by 2^-e.
+// The leading 24 bits of v 2^-e (zero when that is below FP32's normal range,
+// the largest float above it), by integer instructions.
 __device__ __forceinline__ float bits_to_float(double v, int e) {
   const long long b = __double_as_longlong(v);
-  const int field = ((int)(b >> 52) & 0x7FF) - 1023 - e + 127;
-  if (field <= 0) return 0.0f;
+  const int raw = (int)(b >> 52) & 0x7FF, field = raw - 1023 - e + 127;
+  if (raw == 0 || field <= 0) return 0.0f;
   const int mag = field >= 255 ? 0x7F7FFFFF : (field << 23) | ((int)(b >> 29) & 0x7FFFFF);
   return __int_as_float(mag | ((int)(b >> 32) & 0x80000000));
 }
-__device__ inline bool cta_jacobi_svd_f64(int n, int ld, double* M, double* B, double* sigma, int max_sweeps,
-                                          int* sweeps_out) {
+
+// |apq| > tol sqrt(app) sqrt(aqq), and the same with big_tol, as the FP64
+// expressions decide it.  FP32 settles it unless the two sides are within 1e-5
+// of each other (the truncations and roots are off by 4e-7) or the norms are
+// out of range: then the FP64 roots (773 clocks each) are taken.
+__device__ __forceinline__ bool rotates(double app, double aqq, double apq, double tol, double big_tol, bool& big) {
+  const int ep = (__double2hiint(app) >> 20) & 0x7FF, eq = (__double2hiint(aqq) >> 20) & 0x7FF;
+  const int e = max(ep, eq);
+  if (min(ep, eq) > 0 && e < 0x7FF && e - min(ep, eq) <= 100) {
+    const float scale = sqrtf(bits_to_float(app, e - 1023)) * sqrtf(bits_to_float(aqq, e - 1023));
+    const float x = fabsf(bits_to_float(apq, e - 1023)), a = (float)tol * scale, b = (float)big_tol * scale;
+    const bool sure = fabsf(x - a) > 1e-5f * a && fabsf(x - b) > 1e-5f * b;
+    if (sure) {
+      big = x > b;
+      return x > a;
+    }
+  }
+  const double scale = sqrt(app) * sqrt(aqq);
+  big = fabs(apq) > big_tol * scale;
+  return fabs(apq) > tol * scale;
+}
+
+// The double version, with the roundings of groups of 8 V lanes in the same
+// way: below order 96 the FP32 basis that comes in is orthonormal to FP32 only,
+// its defect stays in the scaling matrices, and a different rounding anywhere
+// before the next basis is enough to move that basis and with it the iterates
+// by 1e-6.  A FP64 instruction holds its quarter of the SM for 64 clocks
+// whatever the lanes do, so four pairs share a warp's instructions, the
+// rotation test is settled in FP32, and rotations by less than 2^-27, whose
+// cosine rounds to 1, leave out the products with it.  With 8 V lanes a pair, two
+// roots in every test and one warp a matrix in the step lengths
+// (pair_lanczos_min) three iterations of 512 problems of order 6 to 64 took
+// 72.1 ms, now 41.8; free in its roundings this part allowed 39.6.
+template <int V>
+__device__ __noinline__ bool cta_jacobi_svd_f64(int n, int ld, double* M, double* B, double* sigma, int max_sweeps,
+                                                int* sweeps_out) {
   constexpr int G = 8, NG = NTHREADS / G;
-  const int lane = threadIdx.x & 31, gl = lane & (G - 1), group = threadIdx.x / G;
+  constexpr int U = 4;  // rows a lane loads before the first store (the compiler cannot move loads past them)
+  const int gl = threadIdx.x & (G - 1), group = threadIdx.x / G;
   const int N = (n % 2 == 0) ? n : n + 1;
-  const float tol = sqrtf((float)n) * 2.220446e-16f, big_tol = sqrtf(tol);
+  const double tol = sqrt((double)n) * Num<double>::eps(), big_tol = sqrt(tol);
+  const int slots = (N / 2 + NG - 1) / NG;  // the same for every group: shuffles stay uniform
   bool converged = (n <= 1);
   int sweep = 0;
   for (; sweep < max_sweeps && !converged; ++sweep) {
     int rotated = 0, big = 0;
-    const int slots = (N / 2 + NG - 1) / NG;  // the same for every group: shuffles stay uniform
     for (int r = 0; r < N - 1; ++r) {
       for (int sidx = 0; sidx < slots; ++sidx) {
         const int k = group + sidx * NG;
         int p = -1, q = -1;
         if (k < N / 2) {
-          if (k == 0) { p = N - 1; q = r; }
-          else { p = r + k < N - 1 ? r + k : r + k - (N - 1); q = r - k >= 0 ? r - k : r - k + (N - 1); }
+          if (k == 0) {
+            p = N - 1;
+            q = r;
+          } else {
+            p = r + k < N - 1 ? r + k : r + k - (N - 1);
+            q = r - k >= 0 ? r - k : r - k + (N - 1);
+          }
           if (p >= n || q >= n) p = q = -1;
         }
         double* mp = M + (int64_t)(p < 0 ? 0 : p) * ld;
         double* mq = M + (int64_t)(p < 0 ? 0 : q) * ld;
-        double app = 0.0, aqq = 0.0, apq = 0.0;
-        if (p >= 0) {
-#pragma unroll 4
-          for (int i = gl; i < n; i += G) {
-            const double x = mp[i], y = mq[i];
-            app = fma(x, x, app); aqq = fma(y, y, aqq); apq = fma(x, y, apq);
-          }
-        }
+        double spp[V], sqq[V], spq[V];
 #pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) {
-          app += __shfl_xor_sync(0xffffffffu, app, o);
-          aqq += __shfl_xor_sync(0xffffffffu, aqq, o);
-          apq += __shfl_xor_sync(0xffffffffu, apq, o);
-        }
-        // scaled by the larger of the two norms' exponents
-        const int e = max((__double2hiint(app) >> 20) & 0x7FF, (__double2hiint(aqq) >> 20) & 0x7FF) - 1023;
-        const float fp = bits_to_float(app, e), fq = bits_to_float(aqq, e), fpq = bits_to_float(apq, e);
-        const float scale = sqrtf(fp) * sqrtf(fq);
-        if (p >= 0 && e < 1024 && fabsf(fpq) > tol * scale) {  // e = 1024: infinite or NaN
-          if (fabsf(fpq) > big_tol * scale) big = 1;
+        for (int v = 0; v < V; ++v) spp[v] = sqq[v] = spq[v] = 0.0;
+        if (p >= 0)
+          for (int i0 = gl; i0 < n; i0 += G * V) {
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+              const int i = i0 + G * v;
+              if (i < n) {
+                const double x = mp[i], y = mq[i];
+                spp[v] = fma(x, x, spp[v]);
+                sqq[v] = fma(y, y, sqq[v]);
+                spq[v] = fma(x, y, spq[v]);
+              }
+            }
+          }
+        const double app = virtual_sum<V>(spp), aqq = virtual_sum<V>(sqq), apq = virtual_sum<V>(spq);
+        bool large = false;
+        if (p >= 0 && rotates(app, aqq, apq, tol, big_tol, large)) {
+          if (large) big = 1;
           // the angle only needs float accuracy (the next sweep removes what
           // is left); c and s are formed in FP64 so the rotation is orthogonal
           // to its rounding
-          const float zf = bits_to_float(aqq - app, e) / (2.0f * fpq);
+          const float zf = (float)((aqq - app) / (2.0 * apq));
           const float tf = (zf >= 0.0f ? 1.0f : -1.0f) / (fabsf(zf) + sqrtf(1.0f + zf * zf));
-          const double t = (double)tf, t2 = t * t;
-          double c;
-          if (fabsf(tf) < 1e-4f) {
-            c = fma(t2, fma(t2, 0.375, -0.5), 1.0);
-          } else {
-            const double x = 1.0 + t2, y = (double)rsqrtf((float)x), d = fma(-x * y, y, 1.0);
-            c = fma(y * d, fma(0.375, d, 0.5), y);
-          }
-          const double sn = c * t;
+          const double t = widen(tf);
+          const bool tiny = fabsf(tf) < 7.4505806e-9f;  // 2^-27: 1 + t^2 rounds to 1
+          const double c = tiny ? 1.0 : rsqrt(fma(t, t, 1.0)), sn = tiny ? t : __dmul_rn(c, t);
           double* bp = B + (int64_t)p * ld;
           double* bq = B + (int64_t)q * ld;
-#pragma unroll 2
-          for (int i = gl; i < n; i += G) {
-            const double x = mp[i], y = mq[i], u = bp[i], v = bq[i];
-            mp[i] = fma(c, x, -(sn * y));
-            mq[i] = fma(sn, x, c * y);
-            bp[i] = fma(c, u, -(sn * v));
-            bq[i] = fma(sn, u, c * v);
+          for (int i0 = gl; i0 < n; i0 += G * U) {
+            double x[U], y[U], u[U], w[U];
+#pragma unroll
+            for (int k4 = 0; k4 < U; ++k4) {
+              const int i = min(i0 + G * k4, n - 1);
+              x[k4] = mp[i];
+              y[k4] = mq[i];
+              u[k4] = bp[i];
+              w[k4] = bq[i];
+            }
+#pragma unroll
+            for (int k4 = 0; k4 < U; ++k4) {
+              const int i = i0 + G * k4;
+              if (i >= n) break;
+              // written out: the choice of the fused product is part of the result
+              if (tiny) {
+                mp[i] = __dadd_rn(x[k4], -__dmul_rn(sn, y[k4]));
+                mq[i] = fma(sn, x[k4], y[k4]);
+                bp[i] = __dadd_rn(u[k4], -__dmul_rn(sn, w[k4]));
+                bq[i] = fma(sn, u[k4], w[k4]);
+              } else {
+                mp[i] = fma(c, x[k4], -__dmul_rn(sn, y[k4]));
+                mq[i] = fma(sn, x[k4], __dmul_rn(c, y[k4]));
+                bp[i] = fma(c, u[k4], -__dmul_rn(sn, w[k4]));
+                bq[i] = fma(sn, u[k4], __dmul_rn(c, w[k4]));
+              }
+            }
           }
           rotated = 1;
         }
@@ -709,21 +737,21 @@ __device__ inline bool cta_jacobi_svd_f64(int n, int ld, double* M, double* B, d
     }
     rotated = __syncthreads_or(rotated);
     big = __syncthreads_or(big);
-    // quadratic convergence, as in the generic version
+    // quadratic convergence, as in the float version
     converged = !rotated || !big;
   }
   *sweeps_out = sweep;
-  const int nslots = (n + NG - 1) / NG;
-  for (int sidx = 0; sidx < nslots; ++sidx) {
+  for (int sidx = 0; sidx < (n + NG - 1) / NG; ++sidx) {
     const int k = group + sidx * NG;
-    double s = 0.0;
-    if (k < n) {
-      const double* mk = M + (int64_t)k * ld;
-      for (int i = gl; i < n; i += G) s = fma(mk[i], mk[i], s);
-    }
+    double s[V];
 #pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (k < n && gl == 0) sigma[k] = sqrt(s);
+    for (int v = 0; v < V; ++v) {
+      s[v] = 0.0;
+      if (k < n)
+        for (int i = gl + G * v; i < n; i += G * V) s[v] = fma(M[(int64_t)k * ld + i], M[(int64_t)k * ld + i], s[v]);
+    }
+    const double t = virtual_sum<V>(s);
+    if (k < n && gl == 0) sigma[k] = sqrt(t);
   }
   __syncthreads();
   return converged;
@@ -881,7 +909,9 @@ template <class T> __host__ __device__ __forceinline__ int jacobi_ld(int n) {
 template <class T>
 __device__ bool cta_jacobi_svd(int n, int ld, T* M, T* B, T* sigma, int max_sweeps, int* sweeps_out) {
   if constexpr (sizeof(T) == 8) {
-    return cta_jacobi_svd_f64(n, ld, M, B, sigma, max_sweeps, sweeps_out);
+    if (n <= 16) return cta_jacobi_svd_f64<1>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
+    if (n <= 48) return cta_jacobi_svd_f64<2>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
+    return cta_jacobi_svd_f64<4>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
   } else {
     if (n <= 16) return cta_jacobi_svd_f32<1>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
     if (n <= 48) return cta_jacobi_svd_f32<2>(n, ld, M, B, sigma, max_sweeps, sweeps_out);
@@ -1144,214 +1174,341 @@ __device__ T warp_lanczos_eigmin(int n, const T* Z, T* Qs, int ldq, int kq, T* Q
   return theta;
 }
 
-// Shared state of cta_lanczos_min.
-struct LanczosShared {
-  TridiagShared tri;
-  double red[NWARPS];
-  int state, stop;
+// x lies above the smallest eigenvalue of the tridiagonal (a, b2), by the
+// count of sturm_count (the first negative pivot decides): the same values,
+// with the squares of b formed once.
+__device__ __forceinline__ bool sturm_below(int k, const double* a, const double* b2, double x, double pivmin) {
+  double d = a[0] - x;
+  if (fabs(d) < pivmin) d = -pivmin;
+  bool neg = d < 0.0;
+  for (int i = 1; i < k; ++i) {
+    d = (a[i] - x) - b2[i] / d;
+    if (fabs(d) < pivmin) d = -pivmin;
+    neg = neg || d < 0.0;
+  }
+  return neg;
+}
+
+// Work vectors of tridiag_eigmin_as for k rows: squares of b, the scaled
+// tridiagonal of the division-free counts, and the FP32 one.
+struct TridiagWork {
+  double *b2, *sa, *sb;
+  float *af, *bf;
 };
 
-// Smallest eigenvalue of the symmetric Z (n x n, n <= 256) in float64 by
-// Lanczos with full reorthogonalization, run by the whole CTA: the iteration
-// of warp_lanczos_eigmin (start vector, two passes against the whole basis,
-// Ritz value every 4 steps until it moves by at most 64 eps) with the sums
-// split over all threads as (output, part) pairs, the norm taken from the
-// second pass's w'w, and the Ritz value looked at in FP32 before the FP64 one
-// is formed (tridiag.cuh).  Z, the basis and the vectors live in shared memory
-// as far as they fit (all of it up to n = 64); the rest of the basis in Qg.
-// One warp per matrix kept one quarter of the SM busy and spent a division per
-// row of every Sturm count: 34 million clocks of a three-iteration slice at
-// n = 64 (three CTAs an SM), 8 million with this.
-__device__ inline double cta_lanczos_min(int n, const double* Zg, double* Qg, unsigned char* smem, int64_t smem_bytes,
-                                         LanczosShared& sh, int* steps) {
-  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  double* qs = (double*)smem;      // [n]
-  double* ws = qs + n;             // [n]
-  double* part = ws + n;           // [NTHREADS]
-  double* coef = part + NTHREADS;  // [n + 2] each
-  double* al = coef + n + 2;
-  double* be = al + n + 2;
-  double* sa = be + n + 2;
-  double* sb = sa + n + 2;
-  float* saf = (float*)(sb + n + 2);
-  float* sbf = saf + n + 2;
-  double* rest = (double*)(sbf + n + 2);
-  int64_t room = smem_bytes / 8 - (rest - qs);
-  const double* Z = Zg;
-  if ((int64_t)n * n <= room) {
-    for (int k = t; k < n * n; k += NTHREADS) rest[k] = Zg[k];
-    Z = rest;
-    rest += (int64_t)n * n;
-    room -= (int64_t)n * n;
-  }
-  const int kq = (int)(room > 0 ? room / n : 0);
-  auto Qc = [&](int l) -> double* { return l < kq ? rest + (int64_t)l * n : Qg + (int64_t)l * n; };
-  // start vector
-  double nrm2 = 0.0;
-  for (int i = t; i < n; i += NTHREADS) {
-    uint32_t h = (uint32_t)(i + 1) * 2654435761u;
-    h ^= h >> 15; h *= 2246822519u; h ^= h >> 13;
-    const double v = (double)(h & 0xffffff) / 16777216.0 - 0.5 + 0.01;
-    qs[i] = v;
-    nrm2 = fma(v, v, nrm2);
-  }
-  nrm2 = warp_sum(nrm2);
-  if (lane == 0) sh.red[warp] = nrm2;
-  if (t == 0) be[0] = 0.0;
-  __syncthreads();
-  {
-    double s = 0.0;
+// The value of warp_tridiag_eigmin<double>, bit for bit, at about half of its
+// FP64 instructions: one warp, `th32` gets the FP32 bracket's middle.
+// The 32 points of a multisection round are compared with an eigenvalue known
+// to 1e-14 of the norm from division-free counts (tridiag.cuh); only points
+// within 2e-14 of that get the count with divisions (900 clocks a row).  Both
+// kinds of count are exact for a matrix within a few eps of this one, so
+// beyond 90 eps they agree.  want = false: the FP32 part alone.
+__device__ __noinline__ inline double tridiag_eigmin_as(int k, const double* a, const double* b, const TridiagWork& W, bool want,
+                                           double* scale_out, float* th32) {
+  const int lane = threadIdx.x & 31;
+  double scale = 0.0;
+  for (int i = lane; i < k; i += 32)
+    scale = fmax(scale, fabs(a[i]) + (i > 0 ? fabs(b[i]) : 0.0) + (i + 1 < k ? fabs(b[i + 1]) : 0.0));
 #pragma unroll
-    for (int w = 0; w < NWARPS; ++w) s += sh.red[w];
-    double root, inv;
-    fast_root(s, root, inv);
-    for (int i = t; i < n; i += NTHREADS) {
-      const double v = qs[i] * inv;
-      qs[i] = v;
-      Qc(0)[i] = v;
+  for (int o = 16; o; o >>= 1) scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
+  *scale_out = scale;
+  *th32 = 0.0f;
+  if (!(scale > 1e-30 && scale < 1e30))  // the general form takes any scale
+    return want ? warp_tridiag_eigmin<double>(k, a, b) : 0.0;
+  const float inv = (float)(1.0 / scale);
+  const int e = ((__double2hiint(scale) >> 20) & 0x7FF) - 1022;  // scale < 2^e
+  const double f = __longlong_as_double((long long)(1023 - e) << 52);
+  for (int i = lane; i < k; i += 32) {
+    const float bi = i > 0 ? (float)b[i] * inv : 0.0f;
+    W.af[i] = (float)a[i];
+    W.bf[i] = __fmul_rn(bi, bi);
+    if (want) {
+      const double y = i > 0 ? b[i] : 0.0;
+      W.b2[i] = __dmul_rn(y, y);
+      W.sa[i] = a[i] * f;
+      W.sb[i] = (y * f) * (y * f);
     }
   }
-  __syncthreads();
-  const int U = n <= 32 ? 4 : n <= 64 ? 2 : 1;  // parts of a row's sum
-  double theta = 0.0, theta_prev = INFINITY, znorm = 0.0;
-  float theta32_prev = INFINITY;
-  bool have_prev = false;
-  int k = 0;
+  __syncwarp();
+  float lo = -1.0f, hi = 1.0f;
+  const float pivf = 1e-30f;
+  for (int it = 0; it < 5; ++it) {
+    const float x = lo + (hi - lo) * (float)(lane + 1) / 33.0f;
+    // the first row's product was rounded there, the others' were fused
+    float d = __fsub_rn(__fmul_rn(W.af[0], inv), x);
+    if (fabsf(d) < pivf) d = -pivf;
+    bool neg = d < 0.0f;
+    for (int i = 1; i < k; ++i) {
+      d = __fadd_rn(fmaf(W.af[i], inv, -x), -(W.bf[i] / d));
+      if (fabsf(d) < pivf) d = -pivf;
+      neg = neg || d < 0.0f;
+    }
+    const unsigned ball = __ballot_sync(0xffffffffu, neg);
+    if (ball == 0) { lo = lo + (hi - lo) * 32.0f / 33.0f; continue; }
+    const int first = __ffs(ball) - 1;
+    const float nhi = lo + (hi - lo) * (float)(first + 1) / 33.0f;
+    const float nlo = first == 0 ? lo : lo + (hi - lo) * (float)first / 33.0f;
+    lo = nlo; hi = nhi;
+  }
+  *th32 = 0.5f * (lo + hi);
+  if (!want) return 0.0;
+  const double w = 4e-6 * fmax(1.0, fabs((double)lo) + fabs((double)hi));
+  double dlo = ((double)lo - w) * scale, dhi = ((double)hi + w) * scale;
+  const double pivmin = 4.93e-32 * fmax(scale, 1e-30);
+  // the eigenvalue to 1e-14 of the norm, [tl, tu] in units of 2^e
+  double tl = dlo * f, tu = dhi * f;
+  bool tested_l = false, tested_u = false;
+  for (int it = 0; it < 8 && tu - tl > 1e-14; ++it) {
+    const double h = (tu - tl) * (1.0 / 33.0);
+    const unsigned above = __ballot_sync(0xffffffffu, sturm_above(k, W.sa, W.sb, fma(h, (double)(lane + 1), tl)));
+    const int first = above == 0xffffffffu ? 32 : __ffs(~above) - 1;
+    const double l = tl;
+    tl = fma(h, (double)first, l);
+    tested_l = tested_l || first > 0;
+    if (first < 32) {
+      tu = fma(h, (double)(first + 1), l);
+      tested_u = true;
+    }
+  }
+  // the FP32 bracket is 4e-6 to both sides: an end that never moved was not
+  // tested, and the general form sees to it
+  if (!tested_l || !tested_u) return warp_tridiag_eigmin<double>(k, a, b);
+  const double g = __longlong_as_double((long long)(1023 + e) << 52);
+  const double near_lo = (tl - 2e-14) * g, near_hi = (tu + 2e-14) * g;
+  for (int it = 0; it < 16; ++it) {
+    if (dhi - dlo <= 2.0 * 2.220446049250313e-16 * fmax(fabs(dlo), fabs(dhi)) + pivmin) break;
+    const double x = dlo + (dhi - dlo) * (double)(lane + 1) / 33.0;
+    bool neg = x > near_hi;
+    const bool close = x >= near_lo && x <= near_hi;
+    if (__any_sync(0xffffffffu, close)) {
+      const bool c = sturm_below(k, a, W.b2, x, pivmin);
+      if (close) neg = c;
+    }
+    const unsigned ball = __ballot_sync(0xffffffffu, neg);
+    if (ball == 0) { dlo = dlo + (dhi - dlo) * 32.0 / 33.0; continue; }
+    const int first = __ffs(ball) - 1;
+    const double nhi = dlo + (dhi - dlo) * (double)(first + 1) / 33.0;
+    const double nlo = first == 0 ? dlo : dlo + (dhi - dlo) * (double)first / 33.0;
+    dlo = nlo; dhi = nhi;
+  }
+  return (dlo + dhi) / 2;
+}
+
+// Shared state of pair_lanczos_min, one entry a matrix.
+struct LanczosShared {
+  double alpha[2], inv[2], theta[2];
+  int steps[2], stop[2];
+};
+
+// Smallest eigenvalues of two symmetric matrices (n x n, n <= 256) in float64,
+// the iteration of warp_lanczos_eigmin with its roundings, two warps a matrix:
+// a row of the vectors per lane, a coefficient per lane, the sums over the rows
+// (alpha, the norm) and the tridiagonal on one warp of the two, as there.  Z,
+// the first columns of the basis and the vectors live in shared memory as far
+// as they fit.
+// The roundings matter: the step length enters every entry of the next iterate
+// (see cta_jacobi_svd_f64).  The FP64 Ritz value is formed only where the
+// iteration can stop: while the FP32 one (good to 1e-6 of the norm) still moves
+// by more than 2e-5 of the norm in four steps, the FP64 one moves by more than
+// 64 eps max(1, |theta|).
+// Bound by the FP64 units: a multiply-add of one warp holds a quarter of the SM
+// for 64 clocks.  With one warp a matrix, all columns on one shared-memory bank
+// at even orders and nine counts with divisions for each Ritz value it took
+// about half of the iteration of a block of 64.
+template <int R>  // rows a lane, n <= 64 R
+__device__ __noinline__ void pair_lanczos_min_r(int n, const double* ZX, const double* ZS, double* QX, double* QS,
+                                                unsigned char* smem, int64_t smem_bytes, LanczosShared& sh) {
+  static_assert(NTHREADS == 128, "two warps a matrix");
+  const double eps = 2.220446049250313e-16;
+  const int side = threadIdx.x >> 6, gt = threadIdx.x & 63, gw = gt >> 5, lane = gt & 31;
+  // the blocks of an SM (numbers 152 apart) take their one-warp parts on
+  // different quarters of it
+  const bool lead = gw == ((int)(blockIdx.x / 152) & 1);
+  const int cl = lead ? lane + 32 : lane;  // coefficients 0-31 on the other warp
+  const int64_t nn = (int64_t)n * n;
+  const int ldq = n | 1;
+  const int64_t vec = 8 * (int64_t)(n + 1), cap = smem_bytes / 16;  // doubles of one matrix
+  const bool zs = cap - nn - vec >= (int64_t)ldq * min(n, 16);
+  const int kq = (int)min((int64_t)n, max((int64_t)0, (cap - vec - (zs ? nn : 0)) / ldq));
+  double* base = (double*)smem + (side ? cap : 0);
+  double* a = base;
+  double* bb = a + (n + 1);
+  double* w = bb + (n + 1);
+  double* coef = w + (n + 1);
+  TridiagWork tw;
+  tw.b2 = coef + (n + 1);
+  tw.sa = tw.b2 + (n + 1);
+  tw.sb = tw.sa + (n + 1);
+  tw.af = (float*)(tw.sb + (n + 1));
+  tw.bf = tw.af + (n + 1);
+  double* Qs = base + vec;
+  double* Zs = Qs + (int64_t)kq * ldq;
+  const double* Zg = side ? ZS : ZX;
+  double* Qg = side ? QS : QX;
+  auto Qc = [&](int l) -> double* { return l < kq ? Qs + l * ldq : Qg + (int64_t)l * n; };
+  auto bar = [&] { asm volatile("bar.sync %0, 64;" ::"r"(1 + side) : "memory"); };
+  // sum over the rows i = lane, lane + 32, ... of p_i q_i, then over the lanes
+  auto dot = [&](const double* p, const double* q) {
+    double s = 0.0;
+#pragma unroll 4
+    for (int i = lane; i < n; i += 32) s = fma(p[i], q[i], s);
+    return warp_sum(s);
+  };
+  if (zs)
+    for (int k = gt; k < (int)nn; k += 64) Zs[k] = Zg[k];
+  const double* Z = zs ? Zs : Zg;
+  if (lead) {
+    double* Q = Qc(0);
+    double nrm2 = 0.0;
+    for (int i = lane; i < n; i += 32) {
+      uint32_t h = (uint32_t)(i + 1) * 2654435761u;
+      h ^= h >> 15; h *= 2246822519u; h ^= h >> 13;
+      const double v = ((double)(h & 0xffffff) / 16777216.0 - 0.5) + 0.01;
+      Q[i] = v;
+      nrm2 = fma(v, v, nrm2);
+    }
+    const double inv = 1.0 / sqrt(warp_sum(nrm2));
+    for (int i = lane; i < n; i += 32) Q[i] *= inv;
+  }
+  bar();
+  double theta = 0.0, theta_prev = INFINITY, znorm = 0.0;  // the lead warp's
+  float here = 0.0f, here_prev = INFINITY;
+  bool have_prev = true;
   for (int j = 0; j < n; ++j) {
-    // ---- w = Z q
-    if (U > 1) {
-      const int i = t % n, u = t / n;
-      if (u < U) {
-        double s = 0.0;
-#pragma unroll 4
-        for (int r = u * n / U; r < (u + 1) * n / U; ++r) s = fma(Z[(int64_t)r * n + i], qs[r], s);
-        part[t] = s;
-      }
-      __syncthreads();
-      if (t < n) {
-        double s = part[t];
-        for (int v = 1; v < U; ++v) s += part[v * n + t];
-        ws[t] = s;
-      }
-    } else {
-      for (int i = t; i < n; i += NTHREADS) {
-        double s = 0.0;
-#pragma unroll 8
-        for (int r = 0; r < n; ++r) s = fma(Z[(int64_t)r * n + i], qs[r], s);
-        ws[i] = s;
+    const double* qj = Qc(j);
+    const double* qp = j > 0 ? Qc(j - 1) : qj;
+    double wl[R];
+#pragma unroll
+    for (int t = 0; t < R; ++t) wl[t] = 0.0;
+    // w = Z q_j; the next columns are loaded while these are summed
+    constexpr int P = R <= 2 ? 4 : 2;
+    double z[P][R];
+    auto load = [&](int r) {
+#pragma unroll
+      for (int u = 0; u < P; ++u)
+#pragma unroll
+        for (int t = 0; t < R; ++t) z[u][t] = Z[(int64_t)min(r + u, n - 1) * n + min(gt + 64 * t, n - 1)];
+    };
+    load(0);
+    for (int r = 0; r < n; r += P) {
+      double y[P][R];
+#pragma unroll
+      for (int u = 0; u < P; ++u)
+#pragma unroll
+        for (int t = 0; t < R; ++t) y[u][t] = z[u][t];
+      if (r + P < n) load(r + P);
+#pragma unroll
+      for (int u = 0; u < P; ++u)
+        if (r + u < n) {
+          const double qr = qj[r + u];
+#pragma unroll
+          for (int t = 0; t < R; ++t)
+            if (gt + 64 * t < n) wl[t] = fma(y[u][t], qr, wl[t]);
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < R; ++t)
+      if (gt + 64 * t < n) w[gt + 64 * t] = wl[t];
+    bar();
+    if (lead) {
+      const double aj = dot(qj, w);
+      if (lane == 0) {
+        a[j] = aj;
+        sh.alpha[side] = aj;
       }
     }
-    __syncthreads();
-    // ---- two passes against q_0 .. q_j; the second one's last output is w'w
-    const int L = j + 1;
-    bool large = false;
+    bar();
+    {
+      const double aj = sh.alpha[side], bj = j > 0 ? bb[j] : 0.0;
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        const int i = gt + 64 * t;
+        if (i < n) {
+          double v = fma(-aj, qj[i], wl[t]);
+          if (j > 0) v = fma(-bj, qp[i], v);
+          wl[t] = v;
+          w[i] = v;
+        }
+      }
+    }
+    bar();
+    // full reorthogonalization, twice: coef_l = Q_l . w (one lane per l)
     for (int pass = 0; pass < 2; ++pass) {
-      const int LL = L + pass;
-      int C = 16;  // neighbouring lanes of one coefficient
-      while (C > 1 && C * LL > NTHREADS) C >>= 1;
-      for (int l0 = 0; l0 < LL; l0 += NTHREADS / C) {
-        const int l = l0 + t / C, c = t & (C - 1);
+      for (int l = cl; l <= j; l += 64) {
+        const double* ql = Qc(l);
         double s = 0.0;
-        if (l < LL) {
-          const double* q = l < L ? Qc(l) : ws;
 #pragma unroll 4
-          for (int i = c; i < n; i += C) s = fma(q[i], ws[i], s);
-        }
-        for (int o = C >> 1; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (c == 0 && l < LL) coef[l] = s;
+        for (int i = 0; i < n; ++i) s = fma(ql[i], w[i], s);
+        coef[l] = s;
       }
-      __syncthreads();
-      if (pass == 0 && t == 0) al[j] = coef[j];
-      if (U > 1) {
-        const int i = t % n, u = t / n;
-        if (u < U) {
-          double s = 0.0;
+      bar();
+#pragma unroll
+      for (int t = 0; t < R; ++t) {
+        const int i = gt + 64 * t;
+        if (i < n) {
+          double v = wl[t];
 #pragma unroll 4
-          for (int l = u * L / U; l < (u + 1) * L / U; ++l) s = fma(-coef[l], Qc(l)[i], s);
-          part[t] = s;
-        }
-        __syncthreads();
-        if (t < n) {
-          double s = part[t];
-          for (int v = 1; v < U; ++v) s += part[v * n + t];
-          ws[t] += s;
-        }
-      } else {
-        for (int i = t; i < n; i += NTHREADS) {
-          double s = ws[i];
-#pragma unroll 4
-          for (int l = 0; l < L; ++l) s = fma(-coef[l], Qc(l)[i], s);
-          ws[i] = s;
+          for (int l = 0; l <= j; ++l) v = fma(-coef[l], Qc(l)[i], v);
+          wl[t] = v;
+          w[i] = v;
         }
       }
-      if (pass == 1) {
-        // a coefficient above 2^-30 |w'| changes the norm
-        const int en = (__double2hiint(coef[L]) >> 20) - 1023;
-        int ec = -2000;
-        for (int l = t; l < L; l += NTHREADS) ec = max(ec, ((__double2hiint(coef[l]) >> 20) & 0x7ff) - 1023);
-        large = __syncthreads_or(2 * ec > en - 60);
-      } else {
-        __syncthreads();
-      }
+      bar();
     }
-    k = L;
-    double bn2 = coef[L];
-    if (large)
-      for (int l = 0; l < L; ++l) bn2 = fma(-coef[l], coef[l], bn2);
-    const int field = __double2hiint(bn2) >> 20;  // 0x7ff: infinite or NaN; below 27: 1e-300 or negative
-    double bn = 0.0, binv = 0.0;
-    if (field > 27 && field < 0x7ff) fast_root(bn2, bn, binv);
-    if (k < n) {
-      double* qn = Qc(k);
-      for (int i = t; i < n; i += NTHREADS) {
-        const double q = ws[i] * binv;
-        qn[i] = q;
-        qs[i] = q;
-      }
-    }
-    if (t == 0) {
-      const double aj = al[j], bj = j > 0 ? be[j] : 0.0;
+    const int k = j + 1;
+    if (lead) {
+      const double aj = sh.alpha[side], bj = j > 0 ? bb[j] : 0.0;
+      const double bn = sqrt(dot(w, w));
       znorm = fmax(znorm, fabs(aj) + bn + fabs(bj));
-      be[k] = bn;
-      const bool bad = field == 0x7ff || (__double2hiint(aj) & 0x7ff00000) == 0x7ff00000;
-      sh.state = bad ? 2 : !(bn > 4.0 * 2.220446049250313e-16 * znorm) ? 1 : 0;
-    }
-    __syncthreads();
-    if (sh.state == 2) {
-      theta = nan("");
-      break;
-    }
-    const bool exhausted = k == n || sh.state == 1;
-    if (exhausted || (k >= 4 && (k & 3) == 0)) {
-      const int e = tridiag_scale(k, al, be, sa, sb, saf, sbf, sh.tri);
-      const float th32 = tridiag_min32(k, saf, sbf, sh.tri);  // in units of 2^e
-      const float here = ldexpf(th32, e);
-      if (exhausted) {
-        theta = tridiag_min64(k, sa, sb, th32, e, sh.tri);
-        break;
-      }
-      if (fabsf(here - theta32_prev) <= 3e-6f * ldexpf(1.0f, e)) {
-        theta = tridiag_min64(k, sa, sb, th32, e, sh.tri);
-        if (!have_prev) {
-          const double th = theta;
-          __syncthreads();
-          theta_prev = tridiag_min64(k - 4, sa, sb, ldexpf(theta32_prev, -e), e, sh.tri);
-          theta = th;
+      if (lane == 0) bb[k] = bn;
+      __syncwarp();
+      const bool exhausted = (k == n) || !(bn > eps * znorm * 4.0);
+      bool stop = exhausted;
+      if (exhausted || (k >= 4 && (k % 4) == 0)) {
+        double scale;
+        float th;
+        tridiag_eigmin_as(k, a, bb, tw, false, &scale, &th);
+        here = th * (float)scale;
+        const bool moves = scale > 1e-8 && scale < 1e30 && fabsf(here - here_prev) > 2e-5f * (float)scale;
+        if (exhausted || !moves) {
+          if (!exhausted && !have_prev) theta_prev = tridiag_eigmin_as(k - 4, a, bb, tw, true, &scale, &th);
+          theta = tridiag_eigmin_as(k, a, bb, tw, true, &scale, &th);
+          const double tolr = eps * 64.0 * fmax(1.0, fabs(theta));
+          stop = exhausted || fabs(theta - theta_prev) <= tolr;
+          theta_prev = theta;
+          have_prev = true;
+        } else {
+          have_prev = false;
         }
-        if (t == 0) sh.stop = fabs(theta - theta_prev) <= 64.0 * 2.220446049250313e-16 * fmax(1.0, fabs(theta));
-        __syncthreads();
-        if (sh.stop) break;
-        theta_prev = theta;
-        have_prev = true;
-      } else {
-        have_prev = false;
+        here_prev = here;
       }
-      theta32_prev = here;
+      if (lane == 0) {
+        sh.stop[side] = stop;
+        sh.inv[side] = 1.0 / bn;
+        if (stop) {
+          sh.theta[side] = theta;
+          sh.steps[side] = k;
+        }
+      }
     }
+    bar();
+    if (sh.stop[side]) break;
+    {
+      double* qn = Qc(k);
+      const double inv = sh.inv[side];
+#pragma unroll
+      for (int t = 0; t < R; ++t)
+        if (gt + 64 * t < n) qn[gt + 64 * t] = wl[t] * inv;
+    }
+    bar();
   }
   __syncthreads();
-  *steps = k;
-  return theta;
+}
+__device__ inline void pair_lanczos_min(int n, const double* ZX, const double* ZS, double* QX, double* QS,
+                                        unsigned char* smem, int64_t smem_bytes, LanczosShared& sh) {
+  if (n <= 64) pair_lanczos_min_r<1>(n, ZX, ZS, QX, QS, smem, smem_bytes, sh);
+  else if (n <= 128) pair_lanczos_min_r<2>(n, ZX, ZS, QX, QS, smem, smem_bytes, sh);
+  else pair_lanczos_min_r<4>(n, ZX, ZS, QX, QS, smem, smem_bytes, sh);
 }
 
 // Solve L L' x = b in place (L lower, ld m) by ONE warp; x (and L, when
