@@ -323,7 +323,10 @@ __global__ void __launch_bounds__(kThreads, 1)
     const int c0 = (warp >> 2) * HALF;
     const int64_t row = (int64_t)tm * BM + (warp & 3) * 32 + lane;
     const bool row_ok = row < a.M;
-    const float scaleU = __int_as_float((127 + a.U) << 23);
+    // the last orders' sum, below 2^-7, is taken in units of 2^-38, which fit 32
+    // bits, and what is below that (U > 38, K up to 256) by its remainder
+    const int up = max(a.U - 38, 0);
+    const float scale_hi = __int_as_float((127 + a.U - up) << 23), scale_lo = __int_as_float((127 + up) << 23);
     const uint32_t tw = tbase + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)c0;
     long long acc[HALF];
 #pragma unroll
@@ -358,13 +361,18 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int j = 0; j < 8; ++j) {
           if constexpr (NG == 5) {
             // orders 0-3: integers below 2^24 times 2^-8g, gathered in units
-            // of 2^-24 by wide multiply-adds; the rest below 2^-7 in units of
-            // 2^-U, U <= 38
+            // of 2^-24 by wide multiply-adds; the rest as one 64-bit rounding
+            // of v 2^U would give it: v has 24 bits, so the remainder of the
+            // first conversion is exact
             long long tsum = (long long)__float2int_rn(__uint_as_float(v[0][j])) * (1 << 24);
             tsum += (long long)__float2int_rn(__uint_as_float(v[1][j]) * 0x1p8f) * (1 << 16);
             tsum += (long long)__float2int_rn(__uint_as_float(v[2][j]) * 0x1p16f) * (1 << 8);
             tsum += (long long)__float2int_rn(__uint_as_float(v[3][j]) * 0x1p24f);
-            acc[sg * 8 + j] += (tsum << (a.U - 24)) + (long long)__float2int_rn(__uint_as_float(v[4][j]) * scaleU);
+            const float x = __uint_as_float(v[4][j]) * scale_hi;
+            const int h = __float2int_rn(x);
+            long long rest = h;
+            if (up) rest = rest * (1ll << up) + __float2int_rn((x - __int2float_rn(h)) * scale_lo);
+            acc[sg * 8 + j] += (tsum << (a.U - 24)) + rest;
           } else {
             // an exact integer and a remainder below 2^18
             acc[sg * 8 + j] += (long long)__float2int_rn(__uint_as_float(v[0][j])) << a.U;
@@ -698,7 +706,7 @@ cudaError_t gemm(const Sliced& A, const Sliced& B, Mode mode, const Out& o, cuda
   a.block_kb = (nchunks + pl.splits - 1) / pl.splits * a.chunk_kb;
   int lg = 0;
   while (((int64_t)1 << lg) < std::max<int64_t>(A.K, 2)) ++lg;
-  a.U = std::max(24, std::min(mode == kMixed ? 46 : 38, 47 - lg));
+  a.U = std::max(24, std::min(46, 47 - lg));  // K is below 2^22 (grid of the slicing), so 47 - lg is at least 25
   a.exa = A.ex;
   a.exb = B.ex;
   a.C = o.C;
