@@ -28,7 +28,6 @@ namespace {
 struct SharedState {
   RedBuf rb;
   int flag;
-  int counter;
   int prob;
   int stop;
   int erd64;     // FP32 phase: E(Rd) in float64 formed for this iteration
@@ -477,10 +476,13 @@ struct Algo {
       // FP32 basis).  FP32 operands live in shared memory when both fit (up to
       // n = 95).  Above, the columns of M' are made orthogonal instead: they
       // are V diag(sigma), so no rotation is accumulated and the one matrix
-      // fits up to n = 135 (then in the FP64 scratch).  That basis is made
-      // orthonormal to FP64 by two Newton-Schulz steps V (3 I - V'V) / 2 (the
-      // defect of 1e-6 is squared twice).  FP64 sweeps from the identity at
-      // these sizes took 130 million clocks a call at n = 128.
+      // fits up to n = 135 (then in the FP64 scratch), scaled by a power of two
+      // so that their squares stay in FP32's range.  That basis is made
+      // orthonormal to FP64 by Newton-Schulz steps V (3 I - V'V) / 2, which square
+      // the defect: two from 1e-5, more where the last FP32 sweep left more.  A
+      // defect above 0.2 or not a number (a basis that did not converge, entries
+      // beyond FP32) is given up: the sweeps then start from the identity, as all
+      // did at these sizes before (130 million clocks a call at n = 128).
       float* scratch = (float*)b.W(W_T3);
       const bool both = (2 * nn + n) * (int64_t)sizeof(float) <= MSDP_SMEM_BYTES;
       const int pad = jacobi_ld<float>(n);
@@ -501,35 +503,53 @@ struct Algo {
         cta_jacobi_svd<float>(n, ld, sMf, sVf, Df, 40, &sw32);
         for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) V64[k] = (T)sVf[k / n * ld + k % n];
       } else {
+        if (threadIdx.x == 0) sh.flag = 0;
+        __syncthreads();
+        int top = 0;  // exponent of the largest entry
+        for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) top = max(top, exponent_field((double)M[k]));
+        top = __reduce_max_sync(0xffffffffu, top);
+        if ((threadIdx.x & 31) == 0) atomicMax(&sh.flag, top);
+        __syncthreads();
+        const double unit = __longlong_as_double((long long)(2046 - min(max(sh.flag, 1), 2045)) << 52);
         for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
           const int c = k / n, r = k - c * n;
-          sMf[r * ld + c] = (float)M[k];
+          sMf[r * ld + c] = (float)((double)M[k] * unit);
         }
         __syncthreads();
         cta_jacobi_svd_f32<4, false>(n, ld, sMf, (float*)nullptr, Df, 40, &sw32);
-        int bad = 0;
-        for (int k = threadIdx.x; k < n; k += NTHREADS) bad |= !(Df[k] > 0.0f && Df[k] < INFINITY);
-        bad = __syncthreads_or(bad);  // out of FP32's range: polished from the identity
         for (int k = threadIdx.x; k < (int)nn; k += NTHREADS) {
           const int c = k / n, r = k - c * n;
-          V64[k] = bad ? (T)(r == c) : (T)(sMf[c * ld + r] / Df[c]);
+          V64[k] = (T)(sMf[c * ld + r] / Df[c]);
         }
       }
       __syncthreads();
-      for (int step = 0; !both && step < 2; ++step) {
+      for (int step = 0; !both; ++step) {
         T* K = b.W(W_T3);
-        T* src = step ? GV : V64;
-        T* dst = step ? V64 : GV;
+        T* src = (step & 1) ? GV : V64;
+        T* dst = (step & 1) ? V64 : GV;
         cta_gemm<T>(n, 1, 0, 0, 0, (T)1, src, src, (T)0, K, scr(), 1);
+        double defect = 0.0;  // |I - V'V|^2 / 4 of the lower triangle
         for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) {
           const int r = (int)k % n, c = (int)k / n;
           if (r < c) continue;
           const T v = r == c ? (T)1.5 - (T)0.5 * K[k] : (T)-0.5 * K[k];
+          const double d = (double)(r == c ? v - (T)1 : v);
+          defect = fma(d, d, defect);
           K[k] = v;
           K[c + (int64_t)r * n] = v;
         }
-        __syncthreads();
+        defect = block_sum(defect, &sh.rb);
+        if (step == 6 || !(defect <= 1e-2)) {  // or not a number
+          cta_set_identity<T>(n, V64, (T)1);
+          break;
+        }
         cta_gemm<T>(n, 0, 0, 0, 0, (T)1, src, K, (T)0, dst, scr());
+        if (defect > 1e-17) continue;  // squared below: 0.75 (9e-9)^2 = 6e-17
+        if (dst != V64) {
+          for (int64_t k = threadIdx.x; k < nn; k += NTHREADS) V64[k] = dst[k];
+          __syncthreads();
+        }
+        break;
       }
       const bool smem64 = 2 * nn * (int64_t)sizeof(T) <= MSDP_SMEM_BYTES;
       const int pad64 = jacobi_ld<double>(n);

@@ -610,13 +610,16 @@ __device__ __forceinline__ float bits_to_float(double v, int e) {
   return __int_as_float(mag | ((int)(b >> 32) & 0x80000000));
 }
 
+// Biased binary exponent: 0 for zero and subnormal numbers, 2047 for infinities
+// and NaN.
+__device__ __forceinline__ int exponent_field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
+
 // |apq| > tol sqrt(app) sqrt(aqq), and the same with big_tol, as the FP64
 // expressions decide it.  FP32 settles it unless the two sides are within 1e-5
 // of each other (the truncations and roots are off by 4e-7) or the norms are
 // out of range: then the FP64 roots (773 clocks each) are taken.
 __device__ __forceinline__ bool rotates(double app, double aqq, double apq, double tol, double big_tol, bool& big) {
-  const int ep = (__double2hiint(app) >> 20) & 0x7FF, eq = (__double2hiint(aqq) >> 20) & 0x7FF;
-  const int e = max(ep, eq);
+  const int ep = exponent_field(app), eq = exponent_field(aqq), e = max(ep, eq);
   if (min(ep, eq) > 0 && e < 0x7FF && e - min(ep, eq) <= 100) {
     const float scale = sqrtf(bits_to_float(app, e - 1023)) * sqrtf(bits_to_float(aqq, e - 1023));
     const float x = fabsf(bits_to_float(apq, e - 1023)), a = (float)tol * scale, b = (float)big_tol * scale;
