@@ -29,6 +29,12 @@ __device__ __forceinline__ void store_remote(const double* p, int rank, double v
   asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
 }
 
+__device__ __forceinline__ void store_remote_int(const int* p, int rank, int v) {
+  uint32_t a;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(p)), "r"(rank));
+  asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+
 // Every block of the cluster holds a slice of the rows of Z and of the basis
 // in shared memory for the whole iteration.  Per step: w = Z q on the slice;
 // two passes of classical Gram-Schmidt against the whole basis (the first
@@ -77,17 +83,24 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
   double* xch = (double*)(sbf + n + 2);         // [2][cs][n + 2], clusters of more than one block
   __shared__ TridiagShared tsh;
   __shared__ double red[8];
-  __shared__ int state, stop;
+  __shared__ int state, stop, top_s, tops[8];
 
   auto cluster_sync = [&] {
     if (cs == 1) __syncthreads();
     else
       asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
   };
+  if (t == 0) top_s = 0;
+  __syncthreads();
+  int top = 0;  // exponent of the largest entry
   for (int idx = t; idx < n * nr; idx += kThreads) {
     const int r = idx / nr, i = idx - r * nr;
-    Zs[idx] = J.Z[r0 + i + (int64_t)r * n];
+    const double z = J.Z[r0 + i + (int64_t)r * n];
+    Zs[idx] = z;
+    top = max(top, (__double2hiint(z) >> 20) & 0x7FF);
   }
+  top = __reduce_max_sync(0xffffffffu, top);
+  if (lane == 0) atomicMax(&top_s, top);
   // the start vector, whole on every block
   double v = 0.0;
   if (t < n) {
@@ -112,6 +125,23 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
   }
   if (t == 0) be[0] = 0.0;
   cluster_sync();
+  // Entries outside 2^-100 to 2^100 are scaled to 1: squares and the FP32 norm
+  // of the tridiagonal stay in range.  (Infinities and NaN are left to `state`.)
+  if (cs > 1) {
+    if (t < cs) store_remote_int(tops + rank, t, top_s);
+    cluster_sync();
+    top = 0;
+    for (int r = 0; r < cs; ++r) top = max(top, tops[r]);
+  } else {
+    top = top_s;
+  }
+  const bool scaled = top < 0x7FF && (top < 923 || top > 1123);
+  const int up = scaled ? min(max(1023 - top, -1022), 1022) : 0;
+  const double unit = __longlong_as_double((long long)(1023 + up) << 52);  // 1 of Z's units
+  if (scaled) {
+    for (int idx = t; idx < n * nr; idx += kThreads) Zs[idx] *= unit;
+    __syncthreads();
+  }
 
   const int U = nr > 64 ? 1 : nr > 32 ? 2 : 4;  // parts of an update: four warps in all
   // parts of a sum split over threads: a power of two, at most 16
@@ -262,7 +292,7 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
           theta_prev = tridiag_min64(k - 4, sa, sb, ldexpf(theta32_prev, -e), e, tsh);
           theta = th;
         }
-        if (t == 0) stop = fabs(theta - theta_prev) <= 64.0 * kEps * fmax(1.0, fabs(theta));
+        if (t == 0) stop = fabs(theta - theta_prev) <= 64.0 * kEps * fmax(unit, fabs(theta));
         __syncthreads();
         if (stop) break;
         theta_prev = theta;
@@ -273,7 +303,7 @@ __global__ void __launch_bounds__(kThreads) k_lanczos(const Job* __restrict__ jo
       theta32_prev = here;
     }
   }
-  if (rank == 0 && t == 0) *J.out = theta;
+  if (rank == 0 && t == 0) *J.out = scaled ? theta * __longlong_as_double((long long)(1023 - up) << 52) : theta;
   // no block leaves while another may still reach its shared memory
   if (cs > 1) cluster_sync();
 }
@@ -394,7 +424,7 @@ __global__ void __launch_bounds__(kThreads) k_orthogonalize(int n, int j, double
       for (int l = 0; l < L; ++l) bn2 = fma(-coef[l], coef[l], bn2);
     const int field = __double2hiint(bn2) >> 20;
     double bn = 0.0, binv = 0.0;
-    if (field > 27 && field < 0x7ff) fast_root(bn2, bn, binv);  // above 1e-300
+    if (field > 0 && field < 0x7ff) fast_root(bn2, bn, binv);
     else bn2 = field == 0x7ff ? bn2 : 0.0;
     for (int i = t; i < nr; i += 128) Q[(int64_t)(j + 1) * n + r0 + i] = ws[i] * binv;
     if (rank == 0 && t == 0) ab[kMaxSteps + j] = bn2;

@@ -86,7 +86,8 @@ struct TridiagShared {
 // ---- block-wide forms: called by every thread of the block (at least 128)
 
 // Scaled copies of the tridiagonal (a, b), b[i] between rows i - 1 and i:
-// sa = a 2^-e, sb = (b 2^-e)^2 with the norm at most 2^e; returns e.
+// sa = a 2^-e, sb = (b 2^-e)^2 with the norm at most 2^e; returns e.  The norm is
+// taken in FP32: the caller sees to it that it is below 2^126.
 __device__ inline int tridiag_scale(int k, const double* a, const double* b, double* sa, double* sb, float* saf,
                                     float* sbf, TridiagShared& sh) {
   const int t = threadIdx.x;
@@ -97,7 +98,7 @@ __device__ inline int tridiag_scale(int k, const double* a, const double* b, dou
 #pragma unroll
     for (int o = 16; o; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
     if (t == 0) {
-      // m 1.001 < 2^e; FP32 covers norms of 1e-38 to 1e38
+      // m 1.001 < 2^e
       const float g = fmaxf(m * 1.001f, 1e-37f);
       sh.e = min((__float_as_int(g) >> 23) - 126, 127);
     }
