@@ -169,8 +169,12 @@ __device__ inline double tridiag_min64(int k, const double* sa, const double* sb
           hi_moved = true;
         }
       }
-      // an end that never moved was not tested
-      if (attempt == 0 && ((!lo_moved && lo0 > -1.0) || (!hi_moved && hi0 < 1.0))) continue;
+      // an end that never moved was not tested: once more over the whole interval,
+      // after every warp has read the last round's entries of `first`
+      if (attempt == 0 && ((!lo_moved && lo0 > -1.0) || (!hi_moved && hi0 < 1.0))) {
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        continue;
+      }
       if (t == 0) sh.theta = exp_add(0.5 * (lo + hi), e);
       break;
     }
