@@ -74,14 +74,17 @@ __device__ __forceinline__ void pivot_root(float d, float& root, float& inv) {
 template <class T, int NS>
 __global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict__ A, int64_t lda,
                                               int* __restrict__ info, __nv_bfloat16* __restrict__ sl,
-                                              int32_t* __restrict__ ex, int64_t Rpad, double* __restrict__ diag) {
+                                              int32_t* __restrict__ ex, int64_t Rpad, double* __restrict__ diag,
+                                              int* __restrict__ err, int polls) {
   __shared__ T colx[NB][NB], coll[NB][NB];  // column j: x and x / d, by row
   __shared__ T yv[NB][ROWS];                // column j of the panel, unscaled
   __shared__ T piv[NB], rinv[NB], root[NB];
   __shared__ double xs[ROWS][NB + 1];
-  __shared__ int bad_s, stuck_s;
+  __shared__ int bad_s, stuck_s, failed_s;
   __shared__ volatile int ready_d[NB], ready_y[NB];  // columns published
-  if (*(volatile int*)info != 0) return;  // an earlier block column failed
+  // one thread looks whether an earlier block column failed: block 0 of this
+  // launch may report a pivot meanwhile, and the block decides as one
+  if (threadIdx.x == 0) failed_s = *(volatile int*)info;
   const int kb = min(NB, n - k0);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, w = warp & 3;
   const bool dg = warp < 4;
@@ -100,16 +103,14 @@ __global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict
   }
   if (threadIdx.x == 0) bad_s = stuck_s = 0;
   if (threadIdx.x < NB) ready_d[threadIdx.x] = ready_y[threadIdx.x] = 0;
-  // a flag of a warp of this block (all are resident); the limit is far above
-  // any wait
+  // a flag of a warp of this block (all are resident); a wait that runs out is
+  // reported at the end, and the warps go on with what is there
   auto wait_for = [&](volatile int* flag) {
-    for (int it = 0; it < (1 << 22); ++it)
-      if (*flag) {
-        __threadfence_block();
-        __syncwarp();
-        return;
-      }
-    stuck_s = 1;
+    int it = 0;
+    while (!*flag && it < polls) ++it;
+    if (it == polls && !*flag) stuck_s = 1;
+    __threadfence_block();
+    __syncwarp();
   };
   auto raise = [&](volatile int* flag) {
     __threadfence_block();
@@ -128,6 +129,7 @@ __global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict
     raise(&ready_d[j]);
   };
   __syncthreads();
+  if (failed_s) return;
   if (dg) {
     if (w == 0) publish(0, x[0]);
 #pragma unroll
@@ -166,8 +168,16 @@ __global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict
     }
   }
   __syncthreads();
-  if (bad_s || stuck_s) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(info, 0, bad_s ? bad_s : k0 + 1);
+  if (stuck_s) {
+    // from any block: its rows and slices are missing
+    if (threadIdx.x == 0) {
+      atomicExch(err, 6);
+      atomicCAS(info, 0, k0 + 1);
+    }
+    return;
+  }
+  if (bad_s) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicCAS(info, 0, bad_s);
     return;
   }
   if (warp == 0) {
@@ -597,9 +607,11 @@ cudaError_t potrf(Work& w, int n, double* A, int64_t lda, int* info, tcg::Mode m
     const int64_t nr = n - k0 - kb;
     const unsigned grid = (unsigned)std::max<int64_t>(1, (nr + ROWS - 1) / ROWS);
     if (mode == tcg::kMixed)
-      k_panel<float, 3><<<grid, 256, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
+      k_panel<float, 3><<<grid, 256, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag,
+                                                 w.err, w.polls);
     else
-      k_panel<double, 7><<<grid, 256, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag);
+      k_panel<double, 7><<<grid, 256, 0, st>>>(n, k0, A, lda, info, w.panel.s, w.panel.ex, w.panel.Rpad, w.diag,
+                                                 w.err, w.polls);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (launches) *launches += 1;

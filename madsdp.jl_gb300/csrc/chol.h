@@ -4,11 +4,11 @@
 // block factorizations (src/blocks.jl:94-113, src/directions.jl:46).
 //
 // One launch per 32-wide block column: every thread block factors the
-// 32 x 32 diagonal block in one warp's registers (redundantly, so no block
-// waits on another) while a second warp solves 32 rows of the panel below
-// against it (L21 = A21 L11^-T), and writes them back together with their
-// bf16 slices;
-// a second launch applies the trailing update A22 -= L21 L21' on the tensor
+// 32 x 32 diagonal block in the registers of four warps (redundantly, so no
+// block waits on another) while four more solve 32 rows of the panel below
+// against it (L21 = A21 L11^-T), a column behind, told by flags in shared
+// memory; they write the rows back together with their bf16 slices.  A second
+// launch applies the trailing update A22 -= L21 L21' on the tensor
 // cores (tcgemm.h, lower triangle only).  kFp64: FP64 diagonal blocks and
 // FP64-accurate updates; kMixed: FP32 diagonal blocks and split-precision
 // updates (an FP32-class factor for iterative refinement).
@@ -28,7 +28,8 @@ struct Work {
   double* dinv = nullptr;  // their inverses (the triangular solves)
   int64_t nmax = 0;
   bool solves = true;    // potrf also forms dinv
-  int* err = nullptr;    // tensor-core error flag (device)
+  int* err = nullptr;    // error flag (device): waits of the products and of these kernels that ran out
+  int polls = 1 << 22;   // looks at a flag before a wait of the panel kernel runs out (far above any wait)
 };
 
 int64_t work_bytes(int64_t nmax);

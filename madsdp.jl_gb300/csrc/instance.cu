@@ -525,7 +525,7 @@ struct msdp_solver {
   int* dinfo = nullptr;
   double *partial = nullptr, *slots = nullptr;
   double* hslots = nullptr;
-  int* hinfo = nullptr;
+  int *hterr = nullptr, *hinfo = nullptr;  // host copies of terr and, after it, dinfo
   int nslot = 0, ninfo = 0;
   double bnorm = 0.0, dnorm = 0.0, cmax = 0.0;
   // user initial point
@@ -645,8 +645,10 @@ int copy_slot(S* s, const double* src) {
 // Bring every slot and info written since the last fetch to the host.
 bool fetch(S* s) {
   if (s->nslot) CU(s, cudaMemcpyAsync(s->hslots, s->slots, sizeof(double) * s->nslot, cudaMemcpyDeviceToHost, s->st));
-  if (s->ninfo) CU(s, cudaMemcpyAsync(s->hinfo, s->dinfo, sizeof(int) * s->ninfo, cudaMemcpyDeviceToHost, s->st));
+  // terr is the int before dinfo[0]
+  if (s->ninfo) CU(s, cudaMemcpyAsync(s->hinfo - 1, s->terr, sizeof(int) * (s->ninfo + 1), cudaMemcpyDeviceToHost, s->st));
   CU(s, cudaStreamSynchronize(s->st));
+  note(s, s->hinfo[-1] == 0, "a wait in a kernel ran out");
   return !s->fail;
 }
 void reset_slots(S* s) { s->nslot = 0; s->ninfo = 0; }
@@ -1837,11 +1839,10 @@ int tc_setup(S* s, bool mixed) {
   }
   s->tfix = (long long*)tcalloc(8 * fixn);
   s->tfix_len = fixn;
-  s->terr = (int*)tcalloc(sizeof(int));
   void* cwm = tcalloc(chol::work_bytes(nmax));
   void* cwh = tcalloc(chol::work_bytes(std::max(m, 1)));
   s->hinfo_dev = (int*)tcalloc(sizeof(int));
-  if (!s->tAm || !s->tBm || !s->tfix || !s->terr || !cwm || !cwh || !s->hinfo_dev) return 1;
+  if (!s->tAm || !s->tBm || !s->tfix || !cwm || !cwh || !s->hinfo_dev) return 1;
   CU(s, chol::init(&s->cw, cwm, nmax, s->terr, s->st, false));
   CU(s, chol::init(&s->cwH, cwh, std::max(m, 1), s->terr, s->st));
   CU(s, cudaMemsetAsync(s->hinfo_dev, 0, sizeof(int), s->st));
@@ -2028,7 +2029,7 @@ void release(S* s) {
   for (void* p : s->allocs) cudaFree(p);
   s->allocs.clear();
   if (s->hslots) cudaFreeHost(s->hslots);
-  if (s->hinfo) cudaFreeHost(s->hinfo);
+  if (s->hterr) cudaFreeHost(s->hterr);
   if (s->cb) cublasDestroy(s->cb);
   if (s->cs) cusolverDnDestroy(s->cs);
 }
@@ -2130,15 +2131,18 @@ int msdp_solver_create(msdp_context* ctx, const msdp_problem_desc* d, const msdp
     }
   }
   s->partial = vec(kRedBlocks); s->slots = vec(kSlots);
-  s->dinfo = dalloc<int>(s, kInfos);
+  s->terr = dalloc<int>(s, kInfos + 1);
+  s->dinfo = s->terr ? s->terr + 1 : nullptr;
   bool okalloc = s->b && s->dlin && s->Clin && s->Cw && s->y && s->dy && s->Rp && s->h && s->acc && s->x && s->z &&
                  s->dx && s->dz && s->Rdlin && s->zinv && s->corrlin && s->vlin && s->ctv && s->wlin && s->H &&
                  s->H0 && s->partial && s->slots && s->dinfo && (!dense_ws || (s->Tb && s->Bb)) && s->ir_r &&
                  s->ir_d && s->ir_h;
   if (!okalloc) return bail(MSDP_ERR_OUT_OF_MEMORY);
   if (cudaMallocHost((void**)&s->hslots, sizeof(double) * kSlots) != cudaSuccess ||
-      cudaMallocHost((void**)&s->hinfo, sizeof(int) * kInfos) != cudaSuccess)
+      cudaMallocHost((void**)&s->hterr, sizeof(int) * (kInfos + 1)) != cudaSuccess)
     return bail(MSDP_ERR_OUT_OF_MEMORY);
+  s->hterr[0] = 0;
+  s->hinfo = s->hterr + 1;
   int lwork = 0;
   for (int i = 0; i < s->nb; ++i) {
     Blk& b = s->B[i];
