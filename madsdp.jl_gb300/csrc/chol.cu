@@ -18,8 +18,7 @@ constexpr int ROWS = 32;  // panel rows per thread block, one per lane
 // because the 32 pivots are one serial chain.
 __device__ __forceinline__ double pivot_inv(double d) {
   const long long b = __double_as_longlong(d);
-  const int field = (int)(b >> 52);
-  if (field < 2 || field > 2044) return 1.0 / d;
+  const int field = (int)(b >> 52);  // 2 to 2044
   const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll);  // [1, 2)
   const float f = __frcp_rn(__int_as_float(0x3F800000 | (int)((b >> 29) & 0x7FFFFF)));    // (0.5, 1]
   const int fb = __float_as_int(f);
@@ -29,6 +28,16 @@ __device__ __forceinline__ double pivot_inv(double d) {
   return __longlong_as_double(__double_as_longlong(z) - ((long long)(field - 1023) << 52));
 }
 __device__ __forceinline__ float pivot_inv(float d) { return 1.0f / d; }
+// x / d for a positive finite pivot; a division where 1 / d leaves the normal
+// range (0 times an infinite reciprocal is no zero)
+__device__ __forceinline__ double pivot_quotient(double x, double d) {
+  const int field = __double2hiint(d) >> 20;
+  return field < 2 || field > 2044 ? x / d : x * pivot_inv(d);
+}
+__device__ __forceinline__ float pivot_quotient(float x, float d) {
+  const int field = __float_as_int(d) >> 23;
+  return field < 2 || field > 252 ? x / d : x * pivot_inv(d);
+}
 // positive and finite
 __device__ __forceinline__ bool pivot_ok(double d) {
   const long long b = __double_as_longlong(d);
@@ -124,7 +133,7 @@ __global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict
       if (lane == 0 && bad_s == 0) bad_s = k0 + j + 1;  // columns come in order
       d = (T)1;  // the factor is not used
     }
-    coll[j][lane] = xj * pivot_inv(d);
+    coll[j][lane] = pivot_quotient(xj, d);
     if (lane == 0) piv[j] = d;
     raise(&ready_d[j]);
   };
