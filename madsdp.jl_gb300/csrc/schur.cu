@@ -27,7 +27,7 @@ struct msdp_schur {
   double* red = nullptr;   // partial maxima of |r| and |b|
   int* info = nullptr;
   int* err = nullptr;
-  double* hmax = nullptr;  // pinned host copy of the partial maxima
+  double* hmax = nullptr;  // pinned host copy of the partial maxima and, after them, of err
   void* wmem = nullptr;
   chol::Work w;
   bool factored = false;
@@ -220,7 +220,7 @@ int msdp_schur_create(msdp_context* ctx, int32_t m, int32_t precision, msdp_schu
   ws->red = q; q += 2 * kRedBlocks;
   ws->info = (int*)q;
   ws->err = ws->info + 1;
-  if (cudaMallocHost((void**)&ws->hmax, sizeof(double) * 2 * kRedBlocks) != cudaSuccess ||
+  if (cudaMallocHost((void**)&ws->hmax, sizeof(double) * (2 * kRedBlocks + 1)) != cudaSuccess ||
       cudaMemsetAsync(ws->info, 0, 2 * sizeof(int), ws->st) != cudaSuccess ||
       chol::init(&ws->w, p, mv, ws->err, ws->st) != cudaSuccess) {
     msdp_schur_destroy(ws);
@@ -280,8 +280,12 @@ int msdp_schur_solve(msdp_schur* ws, double* rhs) {
         return MSDP_ERR_CUDA;
     }
   }
+  // with the solution the error flag: a wait of the triangular solves that ran
+  // out leaves no numbers in it
+  int* herr = (int*)(ws->hmax + 2 * kRedBlocks);
   if (cudaMemcpyAsync(rhs, ws->x, sizeof(double) * m, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-      cudaStreamSynchronize(st) != cudaSuccess)
+      cudaMemcpyAsync(herr, ws->err, sizeof(int), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess || *herr)
     return MSDP_ERR_CUDA;
   return MSDP_OK;
 }
