@@ -12,41 +12,6 @@ namespace {
 constexpr int NB = 32;    // block column width (= K of the trailing update)
 constexpr int ROWS = 32;  // panel rows per thread block, one per lane
 
-// 1/d of a positive finite pivot.  In double: the reciprocal of d's mantissa
-// in FP32 (both conversions by integer instructions) and one third-order
-// correction y (1 + e + e^2), e = 1 - m y: four dependent FP64 instructions,
-// because the 32 pivots are one serial chain.
-__device__ __forceinline__ double pivot_inv(double d) {
-  const long long b = __double_as_longlong(d);
-  const int field = (int)(b >> 52);  // 2 to 2044
-  const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll);  // [1, 2)
-  const float f = __frcp_rn(__int_as_float(0x3F800000 | (int)((b >> 29) & 0x7FFFFF)));    // (0.5, 1]
-  const int fb = __float_as_int(f);
-  const double y = __hiloint2double(((fb >> 3) & 0x0FFFFFFF) + 0x38000000, fb << 29);
-  const double e = fma(-m, y, 1.0);
-  const double z = fma(y, fma(e, e, e), y);
-  return __longlong_as_double(__double_as_longlong(z) - ((long long)(field - 1023) << 52));
-}
-__device__ __forceinline__ float pivot_inv(float d) { return 1.0f / d; }
-// x / d for a positive finite pivot; a division where 1 / d leaves the normal
-// range (0 times an infinite reciprocal is no zero)
-__device__ __forceinline__ double pivot_quotient(double x, double d) {
-  const int field = __double2hiint(d) >> 20;
-  return field < 2 || field > 2044 ? x / d : x * pivot_inv(d);
-}
-__device__ __forceinline__ float pivot_quotient(float x, float d) {
-  const int field = __float_as_int(d) >> 23;
-  return field < 2 || field > 252 ? x / d : x * pivot_inv(d);
-}
-// positive and finite
-__device__ __forceinline__ bool pivot_ok(double d) {
-  const long long b = __double_as_longlong(d);
-  return b > 0 && b < 0x7FF0000000000000ll;
-}
-__device__ __forceinline__ bool pivot_ok(float d) {
-  const int b = __float_as_int(d);
-  return b > 0 && b < 0x7F800000;
-}
 __device__ __forceinline__ void pivot_root(double d, double& root, double& inv) {
   if (__double2hiint(d) < 0x00100000) {  // subnormal
     root = sqrt(d);
@@ -133,7 +98,7 @@ __global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict
       if (lane == 0 && bad_s == 0) bad_s = k0 + j + 1;  // columns come in order
       d = (T)1;  // the factor is not used
     }
-    coll[j][lane] = pivot_quotient(xj, d);
+    coll[j][lane] = fast_quotient(xj, d);
     if (lane == 0) piv[j] = d;
     raise(&ready_d[j]);
   };

@@ -10,6 +10,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "scalar.cuh"
 #include "tridiag.cuh"
 
 #ifndef NTHREADS
@@ -77,15 +78,6 @@ __device__ __forceinline__ double block_max(double v, RedBuf* rb) {
   __syncthreads();
   return r;
 }
-
-// (double)x exactly, by integer instructions: the conversion occupies the FP64
-// unit like a multiply-add.
-__device__ __forceinline__ double widen(float x) {
-  const int b = __float_as_int(x);
-  if ((b & 0x7F800000) == 0 || (b & 0x7F800000) == 0x7F800000) return (double)x;  // 0, subnormal, infinite, NaN
-  return __hiloint2double((b & 0x80000000) | (((b & 0x7FFFFFFF) >> 3) + 0x38000000), b << 29);
-}
-__device__ __forceinline__ double widen(double x) { return x; }
 
 // ---------------------------------------------------------------- elementwise
 template <class T, class U>
@@ -276,25 +268,7 @@ template <> __device__ __forceinline__ void chol_pivot<float>(float d, float& ro
   inv = 1.0f / root;
 }
 template <> __device__ __forceinline__ void chol_pivot<double>(double d, double& root, double& inv) {
-  if (__double2hiint(d) < 0x06400000) {  // below 2^-923 the residuals fall out of range
-    root = sqrt(d);
-    inv = 1.0 / root;
-    return;
-  }
-  // root and reciprocal as sqrt and a division round them, by one residual
-  // correction each (Markstein 1990): about 700 clocks instead of 1500.  His
-  // reciprocal misses where the root's mantissa is all ones
-  fast_root(d, root, inv);
-  const long long b = __double_as_longlong(root);
-  inv = (b & 0xFFFFFFFFFFFFFll) == 0xFFFFFFFFFFFFFll ? 1.0 / root : fma(fma(-root, inv, 1.0), inv, inv);
-}
-__device__ __forceinline__ bool pivot_ok(double d) {
-  const long long b = __double_as_longlong(d);
-  return b > 0 && b < 0x7FF0000000000000ll;
-}
-__device__ __forceinline__ bool pivot_ok(float d) {
-  const int b = __float_as_int(d);
-  return b > 0 && b < 0x7F800000;
+  exact_root(d, root, inv);
 }
 template <class T>
 __device__ __forceinline__ bool pivot_ok(T d) {
@@ -599,20 +573,6 @@ __device__ bool cta_jacobi_svd_f32(int n, int ld, float* M, float* B, float* sig
   __syncthreads();
   return converged;
 }
-
-// The leading 24 bits of v 2^-e (zero when that is below FP32's normal range,
-// the largest float above it), by integer instructions.
-__device__ __forceinline__ float bits_to_float(double v, int e) {
-  const long long b = __double_as_longlong(v);
-  const int raw = (int)(b >> 52) & 0x7FF, field = raw - 1023 - e + 127;
-  if (raw == 0 || field <= 0) return 0.0f;
-  const int mag = field >= 255 ? 0x7F7FFFFF : (field << 23) | ((int)(b >> 29) & 0x7FFFFF);
-  return __int_as_float(mag | ((int)(b >> 32) & 0x80000000));
-}
-
-// Biased binary exponent: 0 for zero and subnormal numbers, 2047 for infinities
-// and NaN.
-__device__ __forceinline__ int exponent_field(double v) { return (__double2hiint(v) >> 20) & 0x7FF; }
 
 // |apq| > tol sqrt(app) sqrt(aqq), and the same with big_tol, as the FP64
 // expressions decide it.  FP32 settles it unless the two sides are within 1e-5

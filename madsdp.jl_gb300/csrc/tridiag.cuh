@@ -1,6 +1,6 @@
 // Device helpers of the Lanczos iterations: the smallest eigenvalue of a
 // symmetric tridiagonal by multisection with the division-free Sturm
-// sequence, and a square root with its reciprocal by a short FP64 chain.
+// sequence.
 //
 // With p_0 = 1, p_1 = a_0 - x, p_i = (a_{i-1} - x) p_{i-1} - b_{i-1}^2 p_{i-2},
 // x lies below the smallest eigenvalue exactly when every p_i is positive.
@@ -13,23 +13,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-// sqrt(d) and 1/sqrt(d) of a positive, normal, finite d: an FP32 reciprocal
-// square root of the mantissa and one third-order correction
-// (y (1 + e/2 + 3/8 e^2), e = 1 - m y^2), then one Newton correction of the
-// root: about 300 clocks of dependent FP64 instructions, where sqrt and a
-// division take about 1500.
-__device__ __forceinline__ void fast_root(double d, double& root, double& inv) {
-  const long long b = __double_as_longlong(d);
-  const int field = (int)(b >> 52);
-  const int k = (field - 1023) >> 1, odd = (field - 1023) & 1;
-  const double m = __longlong_as_double((b & 0xFFFFFFFFFFFFFll) | ((long long)(1023 + odd) << 52));  // [1, 4)
-  const double y = (double)rsqrtf((float)m);
-  const double e = fma(-m * y, y, 1.0);
-  const double z = fma(y * e, fma(0.375, e, 0.5), y);
-  inv = __longlong_as_double(__double_as_longlong(z) - ((long long)k << 52));
-  const double s = d * inv;
-  root = fma(fma(-s, s, d) * 0.5, inv, s);
-}
+#include "scalar.cuh"
 
 // v * 2^e for a normal v whose result is normal, or 0
 __device__ __forceinline__ double exp_add(double v, int e) {
