@@ -794,7 +794,8 @@ def run_gpu(args):
                      "note": "algorithmic flops of the iteration (28n^3 + nnz^2 + m^3/3 + 4m^2 per instance-"
                              "iteration) / iterate-kernel time; the kernel runs on CUDA cores (FP32/FP64), not tcgen05",
                      "limiter": "FP64 pipe (1.25 TFLOP/s nominal on GB300): 26% of active cycles on average, "
-                                "saturated on the busiest SMs (profiles/ipm_kernel_sos_batch.txt)",
+                                "saturated on the busiest SMs, in a profile of an earlier form of this kernel "
+                                "(profiles/ipm_kernel_sos_batch.txt)",
                      "fp64_pipe_frac": achieved * 1e3 / fp64_rate, "fp32_pipe_frac": achieved * 1e3 / fp32_rate,
                      "pipe_peaks_gflops": {"fp64": fp64_rate, "fp32": fp32_rate,
                                            "source": "measured FMA throughput, profiles/gb300_primitives.txt"}},

@@ -44,7 +44,7 @@ __device__ __forceinline__ void pivot_root(float d, float& root, float& inv) {
 // Bound by 32 times that chain and the 300 instructions per quarter: 24 us
 // (in stream order).  With the diagonal block in one warp and a root in every
 // step the kernel took 40 us, with four warps and block barriers 29 us; with
-// block-wide steps, roots and divisions and 64 rows per block 99-123 us (ncu).
+// block-wide steps, roots and divisions and 64 rows per block 99-123 us.
 template <class T, int NS>
 __global__ void __launch_bounds__(256) k_panel(int n, int k0, double* __restrict__ A, int64_t lda,
                                               int* __restrict__ info, __nv_bfloat16* __restrict__ sl,
@@ -277,7 +277,7 @@ __host__ __device__ inline int64_t solve_smem(int nbk, int cs) {
 // read in order; the sum over the lanes is taken when B's turn comes).  Bound
 // by the FP64 pipes of the cluster's SMs (n^2 multiply-adds at 1.6 per clock
 // and SM) and, per block row, by one exchange and two 32 x 32 products:
-// 385 us at n = 2000 and 25 us at n = 100 (ncu).  One block of 1024 threads
+// 385 us at n = 2000 and 25 us at n = 100.  One block of 1024 threads
 // alone took 1706 and 46 us.
 // Every wait is bounded; a wait that runs out sets *err and the block goes on
 // to the closing cluster barrier.

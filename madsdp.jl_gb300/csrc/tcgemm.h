@@ -80,14 +80,15 @@ cudaError_t slice(const Source& src, Sliced* dst, cudaStream_t st);
 struct Out {
   double* C = nullptr;
   int64_t ldc = 0;
-  double alpha = 1.0, beta = 0.0;  // beta 0 or 1 with one K chunk and alpha = +-2^p: written in the epilogue
+  double alpha = 1.0, beta = 0.0;  // any values, with or without a split of K
   bool lower = false;           // only entries with row >= col (tiles below the diagonal)
-  long long* fix = nullptr;     // M x N int64 workspace (split K or general alpha/beta)
+  long long* fix = nullptr;     // M x N int64 workspace (split K only, see needs_fix)
   int64_t ldfix = 0;
   int* err = nullptr;           // device flag: nonzero when a bounded wait ran out
 };
 int64_t fix_bytes(int64_t M, int64_t N);
-// True when this product needs the fixed-point workspace.
+// True when this product needs the fixed-point workspace: its K range is split
+// over several thread blocks.
 bool needs_fix(const Sliced& A, const Sliced& B, Mode mode, const Out& o);
 // C = alpha * A B^T (+ beta C): A and B are K-major slices (rows of A = rows
 // of C, rows of B = columns of C).  `launches` counts the kernels issued.
