@@ -41,7 +41,7 @@ __device__ __forceinline__ void pivot_root(float d, float& root, float& inv) {
 // it and publishes its pivot before the rest of the step's work; the warps
 // wait for columns by flags in shared memory (bounded), not for each other.
 // No FP64 comparisons: they cost as much as a multiply-add.
-// Bound by 32 times that chain and the 300 instructions per quarter: 24 us
+// Bound by 32 times that chain and the 300 instructions per quarter: 21 to 24 us
 // (in stream order).  With the diagonal block in one warp and a root in every
 // step the kernel took 40 us, with four warps and block barriers 29 us; with
 // block-wide steps, roots and divisions and 64 rows per block 99-123 us.

@@ -604,7 +604,7 @@ __device__ __forceinline__ bool rotates(double app, double aqq, double apq, doub
 // cosine rounds to 1, leave out the products with it.  With 8 V lanes a pair, two
 // roots in every test and one warp a matrix in the step lengths
 // (pair_lanczos_min) three iterations of 512 problems of order 6 to 64 took
-// 72.1 ms, now 41.8; free in its roundings this part allowed 39.6.
+// 72 ms, now 41 to 42; free in its roundings this part allowed 39.6.
 template <int V>
 __device__ __noinline__ bool cta_jacobi_svd_f64(int n, int ld, double* M, double* B, double* sigma, int max_sweeps,
                                                 int* sweeps_out) {
